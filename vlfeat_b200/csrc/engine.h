@@ -25,16 +25,20 @@ struct DevModel {
 };
 
 // Derived per-component constants for the exact E-step (vl/gmm.c:741-756):
-// inv = 1/sigma^2, cst = log w - (D/2) log 2pi - (1/2) sum log sigma^2
+// img = the E-step's image of means and 1/sigma^2 (exact_image_elems
+// elements, 16-byte aligned), inv = 1/sigma^2 (either may be null), cst = log w - (D/2) log 2pi - (1/2) sum log sigma^2
 // (-inf when the prior is below 1e-6), sis = sqrt(1/sigma^2) (vl/fisher.c:388).
 template <typename T>
 struct DevDerived {
   T *inv = nullptr;
   double *cst = nullptr;
   T *sis = nullptr;
+  T *img = nullptr;
 };
 
 // ---------------------------------------------------------------- exact path
+template <typename T>
+size_t exact_image_elems(i64 K, i64 D);
 template <typename T>
 void exact_prepare(const DevModel<T> &m, DevDerived<T> &der, cudaStream_t s);
 
@@ -144,8 +148,8 @@ void exact_fisher_batch(const T *X, const i64 *h_offsets, i64 numImages, const D
 // allocation, no host-to-device copies, no event timing).  Every scratch
 // element the kernels read is written earlier in the same call.
 struct ExactFvScratch {
-  float *inv, *sis, *q;
-  double *cst, *llp, *pu, *pv;
+  float *img, *sis, *q;
+  double *cst, *pu, *pv;
   Segment *segs;
   int *segBegin;
   i64 *rows;

@@ -181,7 +181,7 @@ double device_estep(const T *dX, i64 N, const vlb::DevModel<T> &m, T *dq, int pr
   }
   if (!done) {
     vlb::DevDerived<T> der;
-    der.inv = sc.slot[17].get<T>(m.K * m.D);
+    der.img = sc.slot[17].get<T>(vlb::exact_image_elems<T>(m.K, m.D));
     der.sis = sc.slot[18].get<T>(m.K * m.D);
     der.cst = sc.slot[19].get<double>(m.K);
     vlb::exact_prepare(m, der, s);

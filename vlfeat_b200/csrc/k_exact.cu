@@ -37,147 +37,408 @@ __device__ __forceinline__ T warp_sum(T v) {
 __device__ __forceinline__ float dexp(float x) { return expf(x); }
 __device__ __forceinline__ double dexp(double x) { return exp(x); }
 
-// ------------------------------------------------------------ prepare
-// Per-component constants, vl/gmm.c:741-756 and vl/fisher.c:386-390.
+// Asynchronous global -> shared copies (16, 8 or 4 bytes; bytes past srcBytes
+// are zero-filled and nothing is read for them).
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t srcBytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(srcBytes) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src, uint32_t srcBytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(srcBytes) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, uint32_t srcBytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(srcBytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// Elements [0, n) of a row of width w (n <= w) to shared memory, the rest
+// zeros, in pieces of VB bytes; w and the addresses suit VB.
+template <int VB, typename T>
+__device__ __forceinline__ void cp_async_piece(uint32_t dst, const T *src, bool in) {
+  if constexpr (VB == 16) cp_async16(dst, src, in ? 16u : 0u);
+  else if constexpr (VB == 8) cp_async8(dst, src, in ? 8u : 0u);
+  else cp_async4(dst, src, in ? 4u : 0u);
+}
+
+// ------------------------------------------------------------ model image
+// The E-step streams the means and inverse variances through shared memory
+// in chunks of es_dc dimensions.  The image holds them in the order its lanes
+// read: components in blocks of 32 NJ (component 32 j + l of a block belongs
+// to lane l), per block, dimension, pair of components (j, j + 1) and lane
+// [-mu_j, -mu_j+1, 1/s2_j, 1/s2_j+1].  Padded components and dimensions are
+// zeros, which add nothing to a distance.
 template <typename T>
-__global__ void k_prepare(const T *__restrict__ priors, const T *__restrict__ covs, int K, int D,
-                          T halfDimLog2Pi, T *__restrict__ inv, double *__restrict__ cst,
-                          T *__restrict__ sis) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+__host__ __device__ constexpr int es_dc() { return 64 / (int)sizeof(T); }  // dimensions per chunk
+// Pairs of components per lane (NJ / 2) for K components: the smallest block
+// that holds them, up to 256; above that the block size that pads least
+// (the larger one on a tie).
+__host__ __device__ inline int es_half_nj(i64 K) {
+  for (int h = 1; h <= 4; ++h)
+    if (K <= 64 * h) return h;
+  int best = 4;
+  i64 pad = (K + 255) / 256 * 256;
+  for (int h = 3; h >= 2; --h) {
+    const i64 p = (K + 64 * h - 1) / (64 * h) * (64 * h);
+    if (p < pad) {
+      pad = p;
+      best = h;
+    }
+  }
+  return best;
+}
+__host__ __device__ inline i64 es_blocks(i64 K) {
+  const int kb = 64 * es_half_nj(K);
+  return (K + kb - 1) / kb;
+}
+template <typename T>
+__host__ __device__ inline i64 es_dpad(i64 D) { return (D + es_dc<T>() - 1) / es_dc<T>() * es_dc<T>(); }
+
+// ------------------------------------------------------------ prepare
+// Per-component constants, vl/gmm.c:741-756 and vl/fisher.c:386-390, and the
+// E-step's image.  One warp per (padded) component, lanes over dimensions;
+// the sum of the logarithms runs over the dimensions in order (a shuffle per
+// term, the logarithms themselves formed 32 at a time).  Bound by latency: 10 us
+// a launch at K = 256, D = 80, where one thread per component took 39.
+template <typename T>
+__global__ void k_prepare(const T *__restrict__ priors, const T *__restrict__ means, const T *__restrict__ covs,
+                          int K, int D, T halfDimLog2Pi, T *__restrict__ inv, double *__restrict__ cst,
+                          T *__restrict__ sis, T *__restrict__ img) {
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x % 32;
+  const int h = es_half_nj(K), kb = 64 * h;
+  const int Dp = (int)es_dpad<T>(D);
+  if (img) {
+    if (k >= (int)es_blocks(K) * kb) return;
+    const int j = (k % kb) / 32;
+    T *o = img + ((i64)(k / kb) * Dp * h + j / 2) * 128 + (k % 32) * 4 + (j & 1);
+    for (int d = lane; d < Dp; d += 32) {
+      const bool in = k < K && d < D;
+      o[(i64)d * h * 128] = in ? -means[(i64)k * D + d] : (T)0;
+      o[(i64)d * h * 128 + 2] = in ? (T)1 / covs[(i64)k * D + d] : (T)0;
+    }
+  }
   if (k >= K) return;
   T acc = 0;
-  for (int d = 0; d < D; ++d) {
-    T c = covs[(i64)k * D + d];
-    acc += (T)log((double)c);
-    inv[(i64)k * D + d] = (T)1 / c;
-    sis[(i64)k * D + d] = (T)sqrt(1.0 / (double)c);
+  for (int d0 = 0; d0 < D; d0 += 32) {
+    const int d = d0 + lane;
+    T lg = 0;
+    if (d < D) {
+      const T c = covs[(i64)k * D + d];
+      lg = (T)log((double)c);
+      if (inv) inv[(i64)k * D + d] = (T)1 / c;
+      sis[(i64)k * D + d] = (T)sqrt(1.0 / (double)c);
+    }
+    const int n = min(32, D - d0);
+    for (int l = 0; l < n; ++l) acc += __shfl_sync(0xffffffffu, lg, l);
   }
-  T logw = ((double)priors[k] < 1e-6) ? (T)(-INFINITY) : (T)log((double)priors[k]);
-  cst[k] = (double)(T)(logw - halfDimLog2Pi) - 0.5 * (double)acc;
+  if (lane == 0) {
+    const T logw = ((double)priors[k] < 1e-6) ? (T)(-INFINITY) : (T)log((double)priors[k]);
+    cst[k] = (double)(T)(logw - halfDimLog2Pi) - 0.5 * (double)acc;
+  }
 }
 
 // ------------------------------------------------------------ E-step
-// Log-densities of a TM x TK tile of (descriptor, component) pairs.  The
-// dimension is streamed through shared memory in chunks of DC.  Each thread
-// owns a register tile of 8 descriptors x 4 components: per dimension, 16-byte
-// shared loads of its 8 x values, 4 means and 4 inverse variances feed 32
-// updates acc += (x - mu)^2 / sigma^2.  Per (descriptor, component) the sum
-// runs over the dimensions in ascending order.
-template <typename T, int TM, int TK, int DC>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 2) k_logp(const T *__restrict__ X, i64 N, int D, int K,
-                                                  const T *__restrict__ means,
-                                                  const T *__restrict__ inv,
-                                                  const double *__restrict__ cst,
-                                                  T *__restrict__ q) {
-  constexpr int RR = 8, CC = 4, NCG = TK / CC;
-  static_assert(TM * TK == kThreads * RR * CC, "one 8 x 4 register tile per thread");
-  constexpr int XP = TM + 16 / (int)sizeof(T), MP = TK + 16 / (int)sizeof(T);  // padded, 16-byte rows
-  constexpr int VW = 16 / (int)sizeof(T);                                     // elements per vector
-  using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-  __shared__ __align__(16) T sx[DC][XP];
-  __shared__ __align__(16) T smu[DC][MP];
-  __shared__ __align__(16) T siv[DC][MP];
-  const int tid = threadIdx.x;
-  const int tc = tid % NCG, tr = tid / NCG;
-  const i64 i0 = (i64)blockIdx.x * TM;
-  const int k0 = blockIdx.y * TK;
-  T acc[RR][CC];
-#pragma unroll
-  for (int r = 0; r < RR; ++r)
-#pragma unroll
-    for (int c = 0; c < CC; ++c) acc[r][c] = 0;
+// Log-densities c_k - 1/2 sum_d (x - mu)^2 / sigma^2 and, with NORM, the
+// row-wise log-sum-exp normalisation (vl/gmm.c:741-790) and the optional FAST
+// one-hot (vl/fisher.c:398-417: first arg-max wins) in one pass over X, the
+// posteriors written once.
+//
+// A warp owns R rows and the block's NJ * 32 components: lane l holds
+// components l, l + 32, ..., so a row's reductions stay inside the warp and
+// run in the order of a warp striding over the row.  Per (row, component) the
+// sum runs over the dimensions in ascending order: (x - mu), its square, and
+// the fused square * iv + acc, in packed pairs of components for float.
+//
+// Bound: the float version issues 3 lane operations per (row, component,
+// dimension) and the FMA pipes take 128 a clock and SM, packed or not
+// (measured: 123), so R x NJ = 64 accumulators per lane keep the operand loads
+// (NJ / 2 16-byte loads per dimension, R broadcast 8-byte loads per two) at
+// under half of the shared-memory bandwidth.  Model and row chunks are copied
+// asynchronously, three stages ahead; two blocks of 64 rows share an SM, so
+// that one block's exponentials and divisions run beside the other's sums.
+// A packed instruction holds the issue port for two clocks, so the sum of all
+// instructions' issue clocks bounds the kernel: 3 x 80 of about 117 a row and
+// warp for the sums at D = 80, K = 256, the rest the exponentials, divisions
+// and conversions.  1.04 M rows, K = 256, D = 80: 2.86 ms (1.72 at the pipes'
+// rate); two kernels with the logits in memory between them took 2.94 + 0.73.
+// 100,000 rows, K = 64, D = 64: 0.086 ms against 0.070 + 0.054.
+// K above 256 (NORM false): one block per (rows, component block) writes the
+// logits and k_normalize finishes the rows.
+template <typename T, int NJ, int R>
+struct EsLayout {
+  static constexpr int DC = es_dc<T>();
+  static constexpr int kStages = 3;
+  static constexpr int kModel = NJ * 32 * DC * 2;  // elements of a model chunk
+  static constexpr size_t bytes(int warps) {
+    return sizeof(T) * (size_t)kStages * (kModel + (size_t)warps * R * DC);
+  }
+};
 
-  for (int d0 = 0; d0 < D; d0 += DC) {
-    for (int e = tid; e < TM * DC; e += kThreads) {
-      int r = e / DC, dd = e % DC;
-      i64 i = i0 + r;
-      int d = d0 + dd;
-      sx[dd][r] = (i < N && d < D) ? X[i * D + d] : (T)0;
-    }
-    for (int e = tid; e < TK * DC; e += kThreads) {
-      int c = e / DC, dd = e % DC;
-      int k = k0 + c, d = d0 + dd;
-      bool ok = (k < K && d < D);
-      smu[dd][c] = ok ? means[(i64)k * D + d] : (T)0;
-      siv[dd][c] = ok ? inv[(i64)k * D + d] : (T)0;
-    }
-    __syncthreads();
-    const int dl = min(DC, D - d0);
-    for (int dd = 0; dd < dl; ++dd) {
-      T x[RR], m[CC], iv[CC];
-#pragma unroll
-      for (int u = 0; u < RR / VW; ++u) {
-        const V w = *reinterpret_cast<const V *>(&sx[dd][tr * RR + u * VW]);
-        const T *wp = reinterpret_cast<const T *>(&w);
-#pragma unroll
-        for (int e = 0; e < VW; ++e) x[u * VW + e] = wp[e];
+template <typename T, int NJ, int R, bool NORM, int VB>
+__global__ void __launch_bounds__(kThreads, 2) k_estep(const T *__restrict__ X, i64 N, int D, int K,
+                                                       const T *__restrict__ img, const double *__restrict__ cst,
+                                                       T *__restrict__ q, int fast, double *__restrict__ ll_part) {
+  using L = EsLayout<T, NJ, R>;
+  constexpr int DC = L::DC, H = NJ / 2, NST = L::kStages;
+  constexpr int VE = VB / (int)sizeof(T);  // elements per copied piece of a row
+  extern __shared__ __align__(16) unsigned char es_smem[];
+  T *sm = (T *)es_smem;                  // [stage][DC][H][32][4]
+  T *sx = sm + NST * L::kModel;          // [stage][row][DC]
+  const int tid = threadIdx.x, w = tid / 32, lane = tid % 32, nthr = blockDim.x;
+  const int rows = nthr / 32 * R;
+  const i64 i0 = (i64)blockIdx.x * rows;
+  const int nch = (D + DC - 1) / DC;
+  img += (i64)blockIdx.y * nch * L::kModel;
+  const int kbase = blockIdx.y * NJ * 32;
+
+  auto issue = [&](int c) {
+    if (c < nch) {
+      const int st = c % NST;
+      const T *ms = img + (i64)c * L::kModel;
+      T *md = sm + st * L::kModel;
+      for (int e = tid; e < L::kModel * (int)sizeof(T) / 16; e += nthr)
+        cp_async16(tc::smem_u32((char *)md + 16 * e), (const char *)ms + 16 * e, 16u);
+      T *xd = sx + st * rows * DC;
+      const int d0 = c * DC;
+      for (int e = tid; e < rows * (DC / VE); e += nthr) {
+        const int r = e / (DC / VE), v = (e % (DC / VE)) * VE;
+        const i64 i = i0 + r;
+        const bool in = i < N && d0 + v < D;
+        cp_async_piece<VB>(tc::smem_u32(xd + r * DC + v), in ? X + i * D + d0 + v : X, in);
       }
+    }
+    cp_async_commit();
+  };
+  issue(0);
+  issue(1);
+
+  unsigned long long acc[R][sizeof(T) == 4 ? H : NJ];  // float: packed pairs; double: values
 #pragma unroll
-      for (int u = 0; u < CC / VW; ++u) {
-        const V a = *reinterpret_cast<const V *>(&smu[dd][tc * CC + u * VW]);
-        const V b = *reinterpret_cast<const V *>(&siv[dd][tc * CC + u * VW]);
-        const T *ap = reinterpret_cast<const T *>(&a);
-        const T *bp = reinterpret_cast<const T *>(&b);
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int e = 0; e < VW; ++e) {
-          m[u * VW + e] = ap[e];
-          iv[u * VW + e] = bp[e];
-        }
-      }
+    for (int j = 0; j < (sizeof(T) == 4 ? H : NJ); ++j) acc[r][j] = 0ull;
+
+  for (int c = 0; c < nch; ++c) {
+    cp_async_wait<1>();
+    __syncthreads();  // chunk c has landed; every warp is done with chunk c - 1's stage
+    issue(c + 2);
+    const T *mc = sm + (c % NST) * L::kModel + lane * 4;
+    const T *xc = sx + (c % NST) * rows * DC + w * R * DC;
+    const int dl = min(DC, D - c * DC);
+#pragma unroll 1
+    for (int dd = 0; dd < dl; dd += 2) {  // an odd last dimension meets a zero one
       if constexpr (sizeof(T) == 4) {
-        // Packed fp32x2 over component pairs: each half is the scalar
-        // x - mu, (x - mu)^2 and the fused (x - mu)^2 iv + acc.
-        constexpr unsigned long long kNeg = 0x8000000080000000ull;
+        float2 x[R];
 #pragma unroll
-        for (int c = 0; c < CC; c += 2) {
-          const unsigned long long mn = tc::f2u(m[c], m[c + 1]) ^ kNeg, ivp = tc::f2u(iv[c], iv[c + 1]);
+        for (int r = 0; r < R; ++r) x[r] = *(const float2 *)(xc + r * DC + dd);
 #pragma unroll
-          for (int r = 0; r < RR; ++r) {
-            const unsigned long long df = tc::add2(tc::f2u(x[r], x[r]), mn);
-            const unsigned long long a = tc::fma2(tc::mul2(df, df), ivp, tc::f2u(acc[r][c], acc[r][c + 1]));
-            acc[r][c] = tc::lo32(a);
-            acc[r][c + 1] = tc::hi32(a);
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int h = 0; h < H; ++h) {
+            const ulonglong2 m = *(const ulonglong2 *)(mc + ((dd + e) * H + h) * 128);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const float xv = e ? x[r].y : x[r].x;
+              const unsigned long long df = tc::add2(tc::f2u(xv, xv), m.x);
+              acc[r][h] = tc::fma2(tc::mul2(df, df), m.y, acc[r][h]);
+            }
           }
-        }
       } else {
+        double2 x[R];
 #pragma unroll
-        for (int r = 0; r < RR; ++r)
+        for (int r = 0; r < R; ++r) x[r] = *(const double2 *)(xc + r * DC + dd);
 #pragma unroll
-          for (int c = 0; c < CC; ++c) {
-            T diff = x[r] - m[c];
-            acc[r][c] += diff * diff * iv[c];
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int h = 0; h < H; ++h) {
+            const double2 mu = *(const double2 *)(mc + ((dd + e) * H + h) * 128);
+            const double2 iv = *(const double2 *)(mc + ((dd + e) * H + h) * 128 + 2);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const double xv = e ? x[r].y : x[r].x;
+              const double d0 = xv + mu.x, d1 = xv + mu.y;
+              acc[r][2 * h] = (unsigned long long)__double_as_longlong(
+                  fma(d0 * d0, iv.x, __longlong_as_double((long long)acc[r][2 * h])));
+              acc[r][2 * h + 1] = (unsigned long long)__double_as_longlong(
+                  fma(d1 * d1, iv.y, __longlong_as_double((long long)acc[r][2 * h + 1])));
+            }
           }
       }
     }
-    __syncthreads();
   }
-  if constexpr (sizeof(T) == 4 && CC == 4) {
-    // The thread's 4 components of a row in one 16-byte store.
-    const int kb = k0 + tc * CC;
-    if ((K & 3) == 0 && kb + CC <= K && ((uintptr_t)q & 15) == 0) {
-      const double c0 = cst[kb], c1 = cst[kb + 1], c2 = cst[kb + 2], c3 = cst[kb + 3];
+  cp_async_wait<0>();
+
+  // ------------------------------------------------------- epilogue
+  double ck[NJ];
 #pragma unroll
-      for (int r = 0; r < RR; ++r) {
-        const i64 i = i0 + tr * RR + r;
-        if (i < N)
-          *reinterpret_cast<float4 *>(q + i * K + kb) =
-              make_float4((float)(c0 - 0.5 * (double)acc[r][0]), (float)(c1 - 0.5 * (double)acc[r][1]),
-                          (float)(c2 - 0.5 * (double)acc[r][2]), (float)(c3 - 0.5 * (double)acc[r][3]));
+  for (int j = 0; j < NJ; ++j) {
+    const int k = kbase + lane + 32 * j;
+    ck[j] = k < K ? cst[k] : -INFINITY;
+  }
+  const i64 row0 = i0 + w * R;
+  constexpr int G = R < 8 ? R : 8;  // rows per log-likelihood partial
+  // The logits take the accumulators' place; each reduction step runs over all
+  // of the warp's rows, so that their shuffles are in flight together.
+  auto get = [&](int r, int j) -> T {
+    if constexpr (sizeof(T) == 4) return j & 1 ? tc::hi32(acc[r][j / 2]) : tc::lo32(acc[r][j / 2]);
+    else return __longlong_as_double((long long)acc[r][j]);
+  };
+  auto put = [&](int r, int j, T v) {
+    if constexpr (sizeof(T) == 4) acc[r][j / 2] = j & 1 ? tc::f2u(tc::lo32(acc[r][j / 2]), v) : tc::f2u(v, tc::hi32(acc[r][j / 2]));
+    else acc[r][j] = (unsigned long long)__double_as_longlong(v);
+  };
+  T mx[R], sum[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    mx[r] = (T)(-INFINITY);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const T v = (T)(ck[j] - 0.5 * (double)get(r, j));
+      put(r, j, v);
+      mx[r] = max(mx[r], v);
+    }
+  }
+  if constexpr (!NORM) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      T *row = q + (row0 + r) * K + kbase;
+      if (row0 + r < N) {
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+          if (kbase + lane + 32 * j < K) row[lane + 32 * j] = get(r, j);
       }
-      return;
+    }
+  } else {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int r = 0; r < R; ++r) mx[r] = max(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], o));
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      sum[r] = 0;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const T e = dexp(get(r, j) - mx[r]);
+        put(r, j, e);
+        sum[r] += e;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int r = 0; r < R; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+    T rsum = 1, rmax = 0;  // lane r: row r's sum of exponentials and maximum
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (lane == r) {
+        rsum = sum[r];
+        rmax = mx[r];
+      }
+      T *row = q + (row0 + r) * K;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) put(r, j, get(r, j) / sum[r]);
+      if (fast) {
+        T bv = (T)(-INFINITY);
+        int bi = 0x7fffffff;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+          if (get(r, j) > bv && lane + 32 * j < K) {
+            bv = get(r, j);
+            bi = lane + 32 * j;
+          }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const T ov = __shfl_xor_sync(0xffffffffu, bv, o);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+        }
+        if (bi == 0x7fffffff) bi = 0;  // all-NaN row: the reference keeps index 0
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) put(r, j, (T)(lane + 32 * j == bi));
+      }
+      if (row0 + r < N) {
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+          if (lane + 32 * j < K) row[lane + 32 * j] = get(r, j);
+      }
+    }
+    if (ll_part) {
+      // Log-likelihood partials of G rows, added in row order.
+      const double lr = (lane < R && row0 + lane < N) ? log((double)rsum) + (double)rmax : 0.0;
+#pragma unroll
+      for (int g = 0; g < R; g += G) {
+        double t = 0;
+#pragma unroll
+        for (int j = 0; j < G; ++j) t += __shfl_sync(0xffffffffu, lr, g + j);
+        if (lane == 0 && row0 + g < N) ll_part[(row0 + g) / G] = t;
+      }
     }
   }
-#pragma unroll
-  for (int c = 0; c < CC; ++c) {
-    const int k = k0 + tc * CC + c;
-    if (k >= K) continue;
-    const double cc = cst[k];
-#pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      const i64 i = i0 + tr * RR + r;
-      if (i < N) q[i * K + k] = (T)(cc - 0.5 * (double)acc[r][c]);
-    }
+}
+
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    VLB_CUDA(cudaGetDevice(&dev));
+    VLB_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+    return v;
+  }();
+  return n;
+}
+
+template <typename T, int NJ, int R, bool NORM>
+void launch_estep_as(const T *X, i64 N, i64 D, i64 K, const T *img, const double *cst, T *q, bool fast,
+                     double *ll_part, int warps, bool vec, cudaStream_t s) {
+  auto kern = vec ? k_estep<T, NJ, R, NORM, 16> : k_estep<T, NJ, R, NORM, (int)sizeof(T)>;
+  const size_t smem = EsLayout<T, NJ, R>::bytes(warps);
+  VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const dim3 g((unsigned)((N + warps * R - 1) / (warps * R)), NORM ? 1u : (unsigned)es_blocks(K));
+  kern<<<g, warps * 32, smem, s>>>(X, N, (int)D, (int)K, img, cst, q, fast ? 1 : 0, ll_part);
+}
+
+// Launches the E-step over N > 0 rows; returns the rows per log-likelihood
+// partial (K <= 256), or 0 when the rows still need k_normalize.
+template <typename T>
+int launch_estep(const T *X, i64 N, i64 D, i64 K, const T *img, const double *cst, T *q, bool fast,
+                 double *ll_part, cudaStream_t s) {
+  constexpr int VE = 16 / (int)sizeof(T);
+  const bool vec = D % VE == 0 && ((uintptr_t)X & 15) == 0;
+  const int h = es_half_nj(K);
+  const bool f4 = sizeof(T) == 4;
+  if (K > 256) {
+    if (h == 2) launch_estep_as<T, 4, 8, false>(X, N, D, K, img, cst, q, fast, ll_part, 8, vec, s);
+    else if (h == 3) launch_estep_as<T, 6, sizeof(T) == 4 ? 8 : 4, false>(X, N, D, K, img, cst, q, fast, ll_part, 8, vec, s);
+    else launch_estep_as<T, 8, sizeof(T) == 4 ? 8 : 4, false>(X, N, D, K, img, cst, q, fast, ll_part, 8, vec, s);
+    return 0;
   }
+  // Float with up to 128 components takes 16 rows per warp when that still
+  // gives every SM its two blocks; otherwise blocks of half the warps spread
+  // the rows over more SMs.
+  const bool wide = f4 && h <= 2 && N >= (i64)sm_count() * 2 * 128;
+  const int warps = N >= (i64)sm_count() * 2 * 64 ? 8 : 4;
+  if (h == 1) {
+    if constexpr (sizeof(T) == 4)
+      if (wide) {
+        launch_estep_as<T, 2, 16, true>(X, N, D, K, img, cst, q, fast, ll_part, 8, vec, s);
+        return 8;
+      }
+    launch_estep_as<T, 2, 8, true>(X, N, D, K, img, cst, q, fast, ll_part, warps, vec, s);
+    return 8;
+  }
+  if (h == 2) {
+    if constexpr (sizeof(T) == 4)
+      if (wide) {
+        launch_estep_as<T, 4, 16, true>(X, N, D, K, img, cst, q, fast, ll_part, 8, vec, s);
+        return 8;
+      }
+    launch_estep_as<T, 4, 8, true>(X, N, D, K, img, cst, q, fast, ll_part, warps, vec, s);
+    return 8;
+  }
+  constexpr int R = sizeof(T) == 4 ? 8 : 4;
+  if (h == 3) launch_estep_as<T, 6, R, true>(X, N, D, K, img, cst, q, fast, ll_part, warps, vec, s);
+  else launch_estep_as<T, 8, R, true>(X, N, D, K, img, cst, q, fast, ll_part, warps, vec, s);
+  return R;
 }
 
 // Row-wise log-sum-exp normalisation (vl/gmm.c:776-790), one warp per row,
@@ -609,20 +870,6 @@ __global__ void __launch_bounds__(kThreads) k_fisher_stats(
   }
 }
 
-// Asynchronous global -> shared copies (16 or 4 bytes; bytes past srcBytes
-// are zero-filled and nothing is read for them).
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t srcBytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(srcBytes) : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, uint32_t srcBytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(srcBytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 // Thresholded statistics visiting only the (row, component) pairs that pass
 // the skip, for float data up to 128 dimensions:
 //  - kSpFisher: k_fisher_stats' statistics (vl/fisher.c:419-449): per segment,
@@ -917,27 +1164,40 @@ inline unsigned grid1(i64 n, int b) { return (unsigned)((n + b - 1) / b); }
 
 // ================================================================ launchers
 
+// Elements of the E-step's model image for K components of dimension D.
+template <typename T>
+size_t exact_image_elems(i64 K, i64 D) {
+  return (size_t)es_blocks(K) * 64 * es_half_nj(K) * 2 * es_dpad<T>(D);
+}
+
+namespace {
+template <typename T>
+unsigned prepare_grid(i64 K) {
+  return (unsigned)((es_blocks(K) * 64 * es_half_nj(K) * 32 + 127) / 128);
+}
+}  // namespace
+
 template <typename T>
 void exact_prepare(const DevModel<T> &m, DevDerived<T> &der, cudaStream_t s) {
   VLB_LAUNCH("exact_prepare", s,
-             k_prepare<T><<<grid1(m.K, 128), 128, 0, s>>>(m.priors, m.covs, (int)m.K, (int)m.D,
-                                                          half_dim_log_2pi<T>(m.D), der.inv,
-                                                          der.cst, der.sis));
+             k_prepare<T><<<prepare_grid<T>(m.K), 128, 0, s>>>(m.priors, m.means, m.covs, (int)m.K, (int)m.D,
+                                                               half_dim_log_2pi<T>(m.D), der.inv, der.cst,
+                                                               der.sis, der.img));
 }
 
 // Capacity bound for any E-step kernel: the exact kernels write one partial
-// per 8 rows; the tensor-core E-step 8 per 128-row tile.
-i64 estep_ll_parts(i64 N) { return std::max<i64>((N + 7) / 8 + 1, 8 * ((N + 127) / 128) + 8); }
+// per 8 rows (4 for double with more than 128 components); the tensor-core
+// E-step 8 per 128-row tile.
+i64 estep_ll_parts(i64 N) { return std::max<i64>((N + 3) / 4 + 1, 8 * ((N + 127) / 128) + 8); }
 
 template <typename T>
 i64 exact_estep(const T *X, i64 N, const DevModel<T> &m, const DevDerived<T> &der, T *q,
                 double *ll_part, bool fast, cudaStream_t s) {
   if (N <= 0) return 0;
-  constexpr int TM = 128, TK = 64, DC = sizeof(T) == 4 ? 32 : 16;  // 34 KB of tiles either way
-  dim3 g(grid1(N, TM), grid1(m.K, TK));
-  VLB_LAUNCH("exact_logp", s,
-             (k_logp<T, TM, TK, DC><<<g, kThreads, 0, s>>>(X, N, (int)m.D, (int)m.K, m.means,
-                                                           der.inv, der.cst, q)));
+  int per = 0;
+  VLB_LAUNCH("exact_estep", s,
+             per = launch_estep<T>(X, N, m.D, m.K, der.img, der.cst, q, fast, ll_part, s));
+  if (per > 0) return (N + per - 1) / per;
   VLB_LAUNCH("exact_normalize", s,
              k_normalize<T><<<grid1(N, 8), kThreads, 0, s>>>(q, N, (int)m.K, fast ? 1 : 0,
                                                              ll_part));
@@ -1105,7 +1365,7 @@ void exact_fisher_batch(const T *X, const i64 *h_offsets, i64 numImages, const D
   const i64 kSegBudget = std::max<i64>(64, (i64)(256u << 20) / (2 * K * D * 8));
   Scratch &sc = thread_scratch(kArenaExact);
   DevDerived<T> der;
-  der.inv = sc.slot[0].get<T>(K * D);
+  der.img = sc.slot[0].get<T>(exact_image_elems<T>(K, D));
   der.sis = sc.slot[1].get<T>(K * D);
   der.cst = sc.slot[2].get<double>(K);
   exact_prepare(m, der, s);
@@ -1207,19 +1467,13 @@ void exact_fisher_single_fixed(const float *X, i64 N, const DevModel<float> &m, 
                                unsigned long long *nterms, int flags, const ExactFvScratch &sc,
                                cudaStream_t s) {
   constexpr int TKC = 32, RC = 32, JMAX = 10, DB = 8 * JMAX;
-  constexpr int TM = 128, TK = 64, DC = 32;
   const i64 K = m.K, D = m.D, nseg = exact_fv_segments(N);
   VLB_LAUNCH_PLAIN(s, k_single_segments<<<1, 32, 0, s>>>(N, nseg, sc.segs, sc.segBegin, sc.rows));
-  VLB_LAUNCH_PLAIN(s, k_prepare<float><<<grid1(K, 128), 128, 0, s>>>(
-                          m.priors, m.covs, (int)K, (int)D, half_dim_log_2pi<float>(D), sc.inv,
-                          sc.cst, sc.sis));
-  if (N > 0) {
-    dim3 g(grid1(N, TM), grid1(K, TK));
-    VLB_LAUNCH_PLAIN(s, (k_logp<float, TM, TK, DC><<<g, kThreads, 0, s>>>(X, N, (int)D, (int)K, m.means,
-                                                                         sc.inv, sc.cst, sc.q)));
-    VLB_LAUNCH_PLAIN(s, k_normalize<float><<<grid1(N, 8), kThreads, 0, s>>>(sc.q, N, (int)K,
-                                                                         (flags & 4) ? 1 : 0, sc.llp));
-  }
+  VLB_LAUNCH_PLAIN(s, k_prepare<float><<<prepare_grid<float>(K), 128, 0, s>>>(
+                          m.priors, m.means, m.covs, (int)K, (int)D, half_dim_log_2pi<float>(D), nullptr,
+                          sc.cst, sc.sis, sc.img));
+  if (N > 0)  // numClusters <= 256 here: one kernel
+    VLB_LAUNCH_PLAIN(s, launch_estep<float>(X, N, D, K, sc.img, sc.cst, sc.q, (flags & 4) != 0, nullptr, s));
   dim3 g2((unsigned)nseg, grid1(K, TKC), grid1(D, DB));
   VLB_LAUNCH_PLAIN(s, (k_fisher_stats<float, TKC, RC, JMAX><<<g2, kThreads, 0, s>>>(
                           X, sc.q, 0, (int)K, (int)D, sc.segs, m.means, sc.sis, m.priors, sc.pu,
@@ -1395,6 +1649,7 @@ void kmeanspp(const T *X, i64 N, i64 D, i64 K, T *centers, i64 x0, const std::ve
 // ------------------------------------------------------ instantiations
 #define VLB_INST(T)                                                                          \
   template void exact_prepare<T>(const DevModel<T> &, DevDerived<T> &, cudaStream_t);        \
+  template size_t exact_image_elems<T>(i64, i64);                                            \
   template i64 exact_estep<T>(const T *, i64, const DevModel<T> &, const DevDerived<T> &,    \
                               T *, double *, bool, cudaStream_t);                            \
   template void exact_mstep<T>(const T *, i64, const T *, T *, T *, T *, i64, i64,           \

@@ -58,11 +58,10 @@ size_t carve(char *base, i64 N, i64 K, i64 D, ExactFvScratch &sc) {
     off += up256(bytes);
     return p;
   };
-  sc.inv = (float *)take(sizeof(float) * K * D);
+  sc.img = (float *)take(sizeof(float) * exact_image_elems<float>(K, D));
   sc.sis = (float *)take(sizeof(float) * K * D);
   sc.cst = (double *)take(sizeof(double) * K);
   sc.q = (float *)take(sizeof(float) * std::max<i64>(1, N) * K);
-  sc.llp = (double *)take(sizeof(double) * ((N + 7) / 8 + 1));
   sc.segs = (Segment *)take(sizeof(Segment) * nseg);
   sc.segBegin = (int *)take(sizeof(int) * 2);
   sc.rows = (i64 *)take(sizeof(i64));
