@@ -871,60 +871,112 @@ __global__ void __launch_bounds__(kThreads) k_fisher_stats(
 }
 
 // Thresholded statistics visiting only the (row, component) pairs that pass
-// the skip, for float data up to 128 dimensions:
+// the skip, for data of up to 128 dimensions:
 //  - kSpFisher: k_fisher_stats' statistics (vl/fisher.c:419-449): per segment,
 //    for pi_k >= 1e-6 and q >= 1e-6, u += q df, v += q (df^2 - 1) with
 //    df = (x - mu) s, and the term counts;
 //  - kSpMstep: k_mstep_stats' statistics (vl/gmm.c:1093-1149): per slab, for
 //    q >= 1e-2/K, mass += q, S1 += q x, S2 += q (x - mu_old)^2.
-// A block takes one segment (or slab) and KB components, all dimensions;
-// 32-row chunks of x and of the block's posterior columns are double-buffered
-// in shared memory by cp.async.  Warp w owns the components w, w + 16, ...:
-// per chunk and component it ballots the rows that pass and walks them in row
-// order, lanes over dimensions, with the accumulators in registers.  Per
-// (component, dimension) the operations and their order are the dense
-// kernels' (fused multiply-adds as there, rows ascending), so the partials are
-// the same bits; the dense kernels spend their time on the pairs the skip
-// removes (about 94% of them on typical posteriors).
-constexpr int kFsThreads = 512, kFsRC = 32;
+// A block takes one segment (or slab) and 16 CPW components, all dimensions;
+// chunks of R rows of x and of the block's posterior columns are
+// double-buffered in shared memory.  Warp w owns CPW neighbouring components:
+// a lane reads its rows' CPW posteriors, ballots list the rows that pass per
+// component, and the warp walks the list in row order, four rows in flight,
+// lanes over pairs of dimensions, the component's constants and sums in
+// registers.  Per (component, dimension) the operations and their order are
+// the dense kernels' (fused multiply-adds as there, rows ascending), so the
+// partials are the same bits; the dense kernels spend their time on the pairs
+// the skip removes (about 94% of them on typical posteriors).
+// Bound by issue: packed operations hold the port two clocks, about 25 clocks
+// a passing pair at D = 80 beside the ballots, and by the blocks' barriers
+// (warps' lists differ in length).  1.04 M rows, K = 256, D = 80, about 21
+// passing components a row: 0.96 ms; a kernel that took one passing row at a
+// time from each ballot, over chunks of 32 rows, took 1.83.
+constexpr int kFsThreads = 512;
 enum { kSpFisher = 0, kSpMstep = 1 };
 
+template <typename T>
 struct SparseStatsArgs {
-  const float *X;        // rows indexed from the call's first row
-  const float *q;        // N x K posteriors, row (r - qbase)
+  const T *X;            // rows indexed from the call's first row
+  const T *q;            // N x K posteriors, row (r - qbase)
   i64 qbase;
-  float thr;             // the smallest float >= the skip threshold
+  T thr;                 // the smallest value of the type >= the skip threshold
   int K, D;
   const Segment *segs;   // kSpFisher: the segments
   i64 N, rowsPerSlab;    // kSpMstep: slab s is rows [s rps, min(N, (s + 1) rps))
-  const float *mu;       // means (kSpFisher) or old means (kSpMstep)
-  const float *sis;      // kSpFisher: 1 / sigma
-  const float *priors;   // kSpFisher
+  const T *mu;           // means (kSpFisher) or old means (kSpMstep)
+  const T *sis;          // kSpFisher: 1 / sigma
+  const T *priors;       // kSpFisher
   double *p1, *p2;       // u, v (kSpFisher) or S1, S2 (kSpMstep): [block][K][D]
   unsigned long long *pnt;  // kSpFisher: term counts [segment][K]
   double *pmass;            // kSpMstep: [slab][K]
-  int vec16;
+  int xvec, qvec;           // bytes per copied piece of X and q
 };
 
-// KB: components per block (128, or 64 above 96 dimensions, where the
-// accumulators of 8 components per warp would not fit in registers).
-size_t sparse_stats_smem(int D, int KB) {
-  return sizeof(float) * ((size_t)2 * KB * D + (size_t)2 * kFsRC * D + (size_t)2 * kFsRC * (KB + 4));
+// Two dimensions of one row: packed for float, two values for double.
+struct PairF {
+  unsigned long long v;
+};
+struct PairD {
+  double a, b;
+};
+template <typename T>
+using PairOf = typename std::conditional<sizeof(T) == 4, PairF, PairD>::type;
+__device__ __forceinline__ PairF ld_pair(const float *p) { return {*(const unsigned long long *)p}; }
+__device__ __forceinline__ PairD ld_pair(const double *p) {
+  const double2 d = *(const double2 *)p;
+  return {d.x, d.y};
+}
+__device__ __forceinline__ PairF mk_pair(float a, float b) { return {tc::f2u(a, b)}; }
+__device__ __forceinline__ PairD mk_pair(double a, double b) { return {a, b}; }
+__device__ __forceinline__ PairF p_add(PairF a, PairF b) { return {tc::add2(a.v, b.v)}; }
+__device__ __forceinline__ PairD p_add(PairD a, PairD b) { return {a.a + b.a, a.b + b.b}; }
+__device__ __forceinline__ PairF p_mul(PairF a, PairF b) { return {tc::mul2(a.v, b.v)}; }
+__device__ __forceinline__ PairD p_mul(PairD a, PairD b) { return {a.a * b.a, a.b * b.b}; }
+__device__ __forceinline__ PairF p_fma(PairF a, PairF b, PairF c) { return {tc::fma2(a.v, b.v, c.v)}; }
+__device__ __forceinline__ PairD p_fma(PairD a, PairD b, PairD c) { return {fma(a.a, b.a, c.a), fma(a.b, b.b, c.b)}; }
+__device__ __forceinline__ double p_lo(PairF a) { return (double)tc::lo32(a.v); }
+__device__ __forceinline__ double p_hi(PairF a) { return (double)tc::hi32(a.v); }
+__device__ __forceinline__ double p_lo(PairD a) { return a.a; }
+__device__ __forceinline__ double p_hi(PairD a) { return a.b; }
+
+template <typename T, int CPW>
+__host__ __device__ constexpr int fs_rows() { return sizeof(T) == 4 ? 128 : 64; }
+// Posterior columns of a row in shared memory: 16 bytes of padding keep the
+// rows 16-byte aligned and, with 64 float columns, eight lanes' 16-byte reads
+// on distinct banks.
+template <typename T, int CPW>
+__host__ __device__ constexpr int fs_qpitch() { return 16 * CPW + 16 / (int)sizeof(T); }
+// A passing row: its posterior and its offset in the chunk's x rows.
+template <typename T>
+struct __align__(2 * sizeof(T)) RowEntry {
+  T p;
+  int off;
+};
+template <typename T, int CPW>
+size_t sparse_stats_smem(int D) {
+  return sizeof(T) * (size_t)2 * fs_rows<T, CPW>() * ((D + 1) / 2 * 2 + fs_qpitch<T, CPW>()) +
+         sizeof(RowEntry<T>) * (size_t)(kFsThreads / 32) * fs_rows<T, CPW>();
 }
 
-template <int MODE, int DPL, int kFsKB>
-__global__ void __launch_bounds__(kFsThreads, 1) k_stats_sparse(const SparseStatsArgs a) {
-  constexpr int NW = kFsThreads / 32, CPW = kFsKB / NW, kFsQP = kFsKB + 4;
-  extern __shared__ __align__(16) float fs_smem[];
-  const int K = a.K, D = a.D;
-  const float *__restrict__ X = a.X;
-  const float *__restrict__ q = a.q;
-  float *smu = fs_smem;               // [KB][D]
-  float *ssi = smu + kFsKB * D;       // [KB][D] (kSpFisher)
-  float *sx = ssi + kFsKB * D;        // [2][RC][D]
-  float *sq = sx + 2 * kFsRC * D;     // [2][RC][QP]
+// NP: pairs of dimensions per lane (dimensions up to 64 NP); NS: single
+// dimensions per lane after them (0 or 1, up to 32 more).
+template <typename T, int MODE, int NP, int NS, int CPW>
+__global__ void __launch_bounds__(kFsThreads, 1) k_stats_sparse(const SparseStatsArgs<T> a) {
+  constexpr int NW = kFsThreads / 32, KB = NW * CPW, R = fs_rows<T, CPW>(), QP = fs_qpitch<T, CPW>(), NWD = R / 32;
+  using P = PairOf<T>;
+  extern __shared__ __align__(16) unsigned char fs_smem[];
+  const int K = a.K, D = a.D, Dp = (D + 1) / 2 * 2;
+  const T *__restrict__ X = a.X;
+  const T *__restrict__ q = a.q;
+  T *sx = (T *)fs_smem;        // [2][R][Dp]
+  T *sq = sx + 2 * R * Dp;     // [2][R][QP]
   const int tid = threadIdx.x, w = tid / 32, lane = tid % 32;
-  const int sidx = blockIdx.x, k0 = blockIdx.y * kFsKB;
+  using Entry = RowEntry<T>;
+  constexpr int U = 4;         // rows of a list in flight
+  Entry *list = (Entry *)(sq + 2 * R * QP) + w * R;  // this warp's passing rows of one component
+  const unsigned below = (1u << lane) - 1u;
+  const int sidx = blockIdx.x, k0 = blockIdx.y * KB;
   i64 row0, row1;
   if constexpr (MODE == kSpFisher) {
     const Segment sg = a.segs[sidx];
@@ -935,56 +987,82 @@ __global__ void __launch_bounds__(kFsThreads, 1) k_stats_sparse(const SparseStat
     row1 = min(a.N, row0 + a.rowsPerSlab);
   }
   const i64 rows = row1 - row0;
-  const int nch = (int)((rows + kFsRC - 1) / kFsRC);
+  const int nch = (int)((rows + R - 1) / R);
   const i64 qbase = a.qbase;
 
   auto issue = [&](int ch) {
     const int b = ch & 1;
-    const i64 rb = row0 + (i64)ch * kFsRC;
-    const int rc = (int)min((i64)kFsRC, row1 - rb);
-    float *bx = sx + b * kFsRC * D, *bq = sq + b * kFsRC * kFsQP;
-    // The chunk's x rows are one contiguous range (rows past rc are never read).
-    const float *xs = X + rb * D;
-    if (a.vec16) {
-      for (int e = tid; e < rc * D / 4; e += kFsThreads) cp_async16(tc::smem_u32(bx + 4 * e), xs + 4 * e, 16u);
-      for (int e = tid; e < kFsRC * (kFsKB / 4); e += kFsThreads) {
-        const int r = e / (kFsKB / 4), c4 = e % (kFsKB / 4), kk = k0 + 4 * c4;
+    const i64 rb = row0 + (i64)ch * R;
+    const int rc = (int)min((i64)R, row1 - rb);
+    const uint32_t bx = tc::smem_u32(sx + b * R * Dp), bq = tc::smem_u32(sq + b * R * QP);
+    const T *xs = X + rb * D;
+    // The chunk's x rows are one contiguous range (rows past rc are never
+    // used), except that rows of an odd dimension are padded to an even one.
+    if (a.xvec == 16) {
+      for (int e = tid; e < rc * D * (int)sizeof(T) / 16; e += kFsThreads) cp_async16(bx + 16 * e, (const char *)xs + 16 * e, 16u);
+    } else if (a.xvec == 8 && D == Dp) {
+      for (int e = tid; e < rc * D * (int)sizeof(T) / 8; e += kFsThreads) cp_async8(bx + 8 * e, (const char *)xs + 8 * e, 8u);
+    } else {
+      for (int r = w; r < rc; r += NW)
+        for (int d = lane; d < D; d += 32)
+          cp_async_piece<(int)sizeof(T)>(bx + (uint32_t)sizeof(T) * (r * Dp + d), xs + r * D + d, true);
+    }
+    if (a.qvec == 16) {
+      constexpr int V = 16 / (int)sizeof(T);
+      for (int e = tid; e < R * (KB / V); e += kFsThreads) {
+        const int r = e / (KB / V), c = e % (KB / V) * V, kk = k0 + c;
         const bool ok = r < rc && kk < K;
-        cp_async16(tc::smem_u32(bq + r * kFsQP + 4 * c4), ok ? q + (rb + r - qbase) * K + kk : q, ok ? 16u : 0u);
+        cp_async16(bq + (uint32_t)sizeof(T) * (r * QP + c), ok ? q + (rb + r - qbase) * K + kk : q, ok ? 16u : 0u);
       }
     } else {
-      for (int e = tid; e < rc * D; e += kFsThreads) cp_async4(tc::smem_u32(bx + e), xs + e, 4u);
-      for (int e = tid; e < kFsRC * kFsKB; e += kFsThreads) {
-        const int r = e / kFsKB, c = e % kFsKB, kk = k0 + c;
+      for (int e = tid; e < R * KB; e += kFsThreads) {
+        const int r = e / KB, c = e % KB, kk = k0 + c;
         const bool ok = r < rc && kk < K;
-        cp_async4(tc::smem_u32(bq + r * kFsQP + c), ok ? q + (rb + r - qbase) * K + kk : q, ok ? 4u : 0u);
+        cp_async_piece<(int)sizeof(T)>(bq + (uint32_t)sizeof(T) * (r * QP + c), ok ? q + (rb + r - qbase) * K + kk : q, ok);
       }
     }
     cp_async_commit();
   };
 
   if (nch > 0) issue(0);
-  for (int e = tid; e < kFsKB * D; e += kFsThreads) {
-    const int kl = e / D, d = e - kl * D, k = k0 + kl;
-    smu[e] = k < K ? a.mu[(i64)k * D + d] : 0.f;
-    if constexpr (MODE == kSpFisher) ssi[e] = k < K ? a.sis[(i64)k * D + d] : 0.f;
+  // This lane's dimension pairs 2 (lane + 32 j), 2 (lane + 32 j) + 1; lanes
+  // past the last pair read pair 0 and write nothing.
+  int off[NP];
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    const int d = 2 * (lane + 32 * j);
+    off[j] = d < D ? d : 0;
   }
-  // The skip: values below thr (compared in double, i.e. below a.thr as
-  // floats; NaN passes in both) and zeros.
-  const float thr = a.thr;
+  const int ds = 64 * NP + lane, offs = NS && ds < D ? ds : 0;
+  // The skip: values below thr (compared in double, i.e. below a.thr in the
+  // data type; NaN passes in both, zeros and rows past the end do not).
+  const T thr = a.thr;
   bool act[CPW];
-  float u[CPW][DPL], v[CPW][DPL], mass[CPW];
+  P mn[CPW][NP], si[CPW][NP], u[CPW][NP], v[CPW][NP];
+  T smn[CPW], ssi[CPW], su[CPW], sv[CPW];  // the single dimension's
+  T mass[CPW];
   unsigned nt[CPW];  // at most the segment's rows
 #pragma unroll
   for (int c = 0; c < CPW; ++c) {
-    const int k = k0 + w + NW * c;
+    const int k = k0 + w * CPW + c;
     if constexpr (MODE == kSpFisher) act[c] = k < K && (double)a.priors[k] >= 1e-6;
     else act[c] = k < K;
     nt[c] = 0;
-    mass[c] = 0.f;
+    mass[c] = su[c] = sv[c] = (T)0;
+    if constexpr (NS > 0) {
+      smn[c] = act[c] ? a.mu[(i64)k * D + offs] : (T)0;
+      if constexpr (MODE == kSpFisher) ssi[c] = act[c] ? a.sis[(i64)k * D + offs] : (T)0;
+    }
 #pragma unroll
-    for (int j = 0; j < DPL; ++j) u[c][j] = v[c][j] = 0.f;
+    for (int j = 0; j < NP; ++j) {
+      u[c][j] = v[c][j] = mk_pair((T)0, (T)0);
+      const bool o0 = act[c], o1 = act[c] && off[j] + 1 < D;
+      const i64 e = (i64)k * D + off[j];
+      mn[c][j] = mk_pair(o0 ? -a.mu[e] : (T)0, o1 ? -a.mu[e + 1] : (T)0);
+      if constexpr (MODE == kSpFisher) si[c][j] = mk_pair(o0 ? a.sis[e] : (T)0, o1 ? a.sis[e + 1] : (T)0);
+    }
   }
+  const P minus1 = mk_pair((T)-1, (T)-1);
   for (int ch = 0; ch < nch; ++ch) {
     if (ch + 1 < nch) {
       issue(ch + 1);
@@ -993,59 +1071,108 @@ __global__ void __launch_bounds__(kFsThreads, 1) k_stats_sparse(const SparseStat
       cp_async_wait<0>();
     }
     __syncthreads();
-    const float *bx = sx + (ch & 1) * kFsRC * D, *bq = sq + (ch & 1) * kFsRC * kFsQP;
-    const int rc = (int)min((i64)kFsRC, rows - (i64)ch * kFsRC);
+    const T *bx = sx + (ch & 1) * R * Dp, *bq = sq + (ch & 1) * R * QP + w * CPW;
+    T val[NWD][CPW];
+#pragma unroll
+    for (int wd = 0; wd < NWD; ++wd) {
+      if constexpr (sizeof(T) == 4 && CPW == 4) {
+        const float4 f = *(const float4 *)(bq + (32 * wd + lane) * QP);
+        val[wd][0] = f.x; val[wd][1] = f.y; val[wd][2] = f.z; val[wd][3] = f.w;
+      } else {
+#pragma unroll
+        for (int c = 0; c < CPW; ++c) val[wd][c] = bq[(32 * wd + lane) * QP + c];
+      }
+    }
 #pragma unroll
     for (int c = 0; c < CPW; ++c) {
       if (!act[c]) continue;  // warp-uniform
-      const int kl = w + NW * c;
-      const float val = bq[lane * kFsQP + kl];
-      unsigned m = __ballot_sync(0xffffffffu, lane < rc && !(val < thr) && val != 0.f);
-      nt[c] += (unsigned)__popc(m);
-      float mu[DPL], si[DPL];
+      // The chunk's passing rows of this component, in row order.
+      int n = 0;
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) {
-        const int d = lane + 32 * j;
-        mu[j] = d < D ? smu[kl * D + d] : 0.f;
-        if constexpr (MODE == kSpFisher) si[j] = d < D ? ssi[kl * D + d] : 0.f;
+      for (int wd = 0; wd < NWD; ++wd) {
+        const bool pass = !(val[wd][c] < thr);
+        const unsigned m = __ballot_sync(0xffffffffu, pass);
+        if (pass) list[n + __popc(m & below)] = Entry{val[wd][c], (32 * wd + lane) * Dp};
+        n += __popc(m);
       }
-      while (m) {
-        const int r = __ffs(m) - 1;
-        m &= m - 1;
-        const float p = bq[r * kFsQP + kl];
+      __syncwarp();
+      nt[c] += (unsigned)n;
+      auto add = [&](T p, const P(&x)[NP], T xs) {
+        const P pp = mk_pair(p, p);
         if constexpr (MODE == kSpMstep) mass[c] += p;
 #pragma unroll
-        for (int j = 0; j < DPL; ++j) {
-          const int d = lane + 32 * j;
-          if (d < D) {
-            const float x = bx[r * D + d];
-            if constexpr (MODE == kSpFisher) {
-              const float df = (x - mu[j]) * si[j];
-              u[c][j] = fmaf(p, df, u[c][j]);
-              v[c][j] = fmaf(p, fmaf(df, df, -1.f), v[c][j]);
-            } else {
-              const float df = x - mu[j];
-              u[c][j] = fmaf(p, x, u[c][j]);
-              v[c][j] = fmaf(p, df * df, v[c][j]);
-            }
+        for (int j = 0; j < NP; ++j) {
+          if constexpr (MODE == kSpFisher) {
+            const P df = p_mul(p_add(x[j], mn[c][j]), si[c][j]);
+            u[c][j] = p_fma(pp, df, u[c][j]);
+            v[c][j] = p_fma(pp, p_fma(df, df, minus1), v[c][j]);
+          } else {
+            const P df = p_add(x[j], mn[c][j]);
+            u[c][j] = p_fma(pp, x[j], u[c][j]);
+            v[c][j] = p_fma(pp, p_mul(df, df), v[c][j]);
           }
         }
+        if constexpr (NS > 0) {
+          if constexpr (MODE == kSpFisher) {
+            const T df = (xs - smn[c]) * ssi[c];
+            su[c] = fma(p, df, su[c]);
+            sv[c] = fma(p, fma(df, df, (T)-1), sv[c]);
+          } else {
+            const T df = xs - smn[c];
+            su[c] = fma(p, xs, su[c]);
+            sv[c] = fma(p, df * df, sv[c]);
+          }
+        }
+      };
+      int i = 0;
+#pragma unroll 1
+      for (; i + U <= n; i += U) {
+        Entry en[U];
+        P x[U][NP];
+        T xs[U];
+#pragma unroll
+        for (int g = 0; g < U; ++g) en[g] = list[i + g];
+#pragma unroll
+        for (int g = 0; g < U; ++g)
+#pragma unroll
+          for (int j = 0; j < NP; ++j) x[g][j] = ld_pair(bx + en[g].off + off[j]);
+#pragma unroll
+        for (int g = 0; g < U; ++g) xs[g] = NS > 0 ? bx[en[g].off + offs] : (T)0;
+#pragma unroll
+        for (int g = 0; g < U; ++g) add(en[g].p, x[g], xs[g]);
       }
+#pragma unroll 1
+      for (; i < n; ++i) {
+        const Entry en = list[i];
+        P x[NP];
+#pragma unroll
+        for (int j = 0; j < NP; ++j) x[j] = ld_pair(bx + en.off + off[j]);
+        add(en.p, x, NS > 0 ? bx[en.off + offs] : (T)0);
+      }
+      __syncwarp();  // the list is read before the next component's is written
     }
     __syncthreads();
   }
 #pragma unroll
   for (int c = 0; c < CPW; ++c) {
-    const int k = k0 + w + NW * c;
+    const int k = k0 + w * CPW + c;
     if (k >= K) continue;
     const i64 base = ((i64)sidx * K + k) * D;
 #pragma unroll
-    for (int j = 0; j < DPL; ++j) {
-      const int d = lane + 32 * j;
+    for (int j = 0; j < NP; ++j) {
+      const int d = 2 * (lane + 32 * j);
       if (d < D) {
-        a.p1[base + d] = (double)u[c][j];
-        a.p2[base + d] = (double)v[c][j];
+        a.p1[base + d] = p_lo(u[c][j]);
+        a.p2[base + d] = p_lo(v[c][j]);
       }
+      if (d + 1 < D) {
+        a.p1[base + d + 1] = p_hi(u[c][j]);
+        a.p2[base + d + 1] = p_hi(v[c][j]);
+      }
+    }
+    if (NS > 0 && ds < D) {
+      a.p1[base + ds] = (double)su[c];
+      a.p2[base + ds] = (double)sv[c];
     }
     if (lane == 0) {
       if constexpr (MODE == kSpFisher) a.pnt[(i64)sidx * K + k] = (unsigned long long)nt[c];
@@ -1054,27 +1181,51 @@ __global__ void __launch_bounds__(kFsThreads, 1) k_stats_sparse(const SparseStat
   }
 }
 
+template <typename T, int MODE, int NP, int NS, int CPW>
+void launch_stats_sparse_as(const SparseStatsArgs<T> &a, i64 nblk, cudaStream_t s) {
+  auto kern = k_stats_sparse<T, MODE, NP, NS, CPW>;
+  const size_t smem = sparse_stats_smem<T, CPW>(a.D);
+  VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int kb = kFsThreads / 32 * CPW;
+  kern<<<dim3((unsigned)nblk, (unsigned)((a.K + kb - 1) / kb)), kFsThreads, smem, s>>>(a);
+}
+
 // Launches k_stats_sparse over nblk segments (or slabs); false when the shape
 // is outside it (the dense kernel runs instead).
-template <int MODE>
-bool launch_stats_sparse(SparseStatsArgs a, i64 nblk, cudaStream_t s) {
+template <int MODE, typename T>
+bool launch_stats_sparse(SparseStatsArgs<T> a, i64 nblk, cudaStream_t s) {
   if (a.D > 128 || nblk <= 0) return false;
-  const int dpl = (a.D + 31) / 32, kb = dpl == 4 ? 64 : 128;
-  auto kern = dpl == 1 ? k_stats_sparse<MODE, 1, 128>
-              : dpl == 2 ? k_stats_sparse<MODE, 2, 128>
-              : dpl == 3 ? k_stats_sparse<MODE, 3, 128>
-                         : k_stats_sparse<MODE, 4, 64>;
-  const size_t smem = sparse_stats_smem(a.D, kb);
-  VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  a.vec16 = (a.D % 4 == 0 && a.K % 4 == 0 && ((uintptr_t)a.X & 15) == 0 && ((uintptr_t)a.q & 15) == 0) ? 1 : 0;
-  // (double)v < t for a float v exactly when v < tf, tf the smallest float >= t.
+  const int VE = 16 / (int)sizeof(T);
+  const uintptr_t xa = (uintptr_t)a.X, qa = (uintptr_t)a.q;
+  a.xvec = a.D % VE == 0 && xa % 16 == 0 ? 16 : a.D % 2 == 0 && xa % 8 == 0 ? 8 : (int)sizeof(T);
+  a.qvec = a.K % VE == 0 && qa % 16 == 0 ? 16 : (int)sizeof(T);
+  // (double)v < t for a value v of the type exactly when v < tf, tf the
+  // smallest such value >= t.
   const double t = MODE == kSpFisher ? 1e-6 : 1e-2 / (double)a.K;
-  float tf = (float)t;
-  if ((double)tf < t) tf = std::nextafter(tf, INFINITY);
+  T tf = (T)t;
+  if ((double)tf < t) tf = std::nextafter(tf, (T)INFINITY);
   a.thr = tf;
-  dim3 g((unsigned)nblk, (unsigned)((a.K + kb - 1) / kb));
-  VLB_LAUNCH(MODE == kSpFisher ? "exact_fisher_stats" : "exact_mstep_stats", s,
-             kern<<<g, kFsThreads, smem, s>>>(a));
+  // Four components per warp read x a quarter as often; with too few segments
+  // to give every SM a block that way, one per warp spreads the components
+  // over four times the blocks.  One image of 500 rows, K = 64, D = 64: 15 us
+  // with one, 27 with four; 1.04 M rows in 256 images, K = 256, D = 80: 1485 and
+  // 965 us.  In double four components' constants and sums do not fit in
+  // registers.
+  // Up to 96 dimensions the ones past 64 are single dimensions: half the issue
+  // time of a second, mostly empty round of pairs.
+  auto go = [&](auto cpw) {
+    constexpr int C = decltype(cpw)::value;
+    if (a.D <= 64) launch_stats_sparse_as<T, MODE, 1, 0, C>(a, nblk, s);
+    else if (a.D <= 96) launch_stats_sparse_as<T, MODE, 1, 1, C>(a, nblk, s);
+    else launch_stats_sparse_as<T, MODE, 2, 0, C>(a, nblk, s);
+  };
+  if constexpr (sizeof(T) == 4) {
+    if (nblk * ((a.K + 63) / 64) >= (i64)sm_count()) {
+      go(std::integral_constant<int, 4>());
+      return true;
+    }
+  }
+  go(std::integral_constant<int, 1>());
   return true;
 }
 
@@ -1218,18 +1369,18 @@ i64 pick_slab_rows(i64 N) {
 }
 }  // namespace
 
-// The M-step statistics of nslab slabs of rows by the sparse kernel (float
-// data up to 128 dimensions); false when the dense kernel is to run.
+// The M-step statistics of nslab slabs of rows by the sparse kernel (up to 128
+// dimensions); false when the dense kernel is to run.
 template <typename T>
 bool mstep_stats_sparse(const T *X, const T *q, i64 N, i64 K, i64 D, i64 rps, i64 nslab, const T *oldMeans,
                         double *pmass, double *ps1, double *ps2, cudaStream_t s) {
-  if constexpr (sizeof(T) == 4) {
-    SparseStatsArgs a{};
-    a.X = X; a.q = q; a.qbase = 0; a.K = (int)K; a.D = (int)D; a.N = N; a.rowsPerSlab = rps;
-    a.mu = oldMeans; a.p1 = ps1; a.p2 = ps2; a.pmass = pmass;
-    return launch_stats_sparse<kSpMstep>(a, nslab, s);
-  }
-  return false;
+  if (D > 128) return false;
+  SparseStatsArgs<T> a{};
+  a.X = X; a.q = q; a.qbase = 0; a.K = (int)K; a.D = (int)D; a.N = N; a.rowsPerSlab = rps;
+  a.mu = oldMeans; a.p1 = ps1; a.p2 = ps2; a.pmass = pmass;
+  bool done = false;
+  VLB_LAUNCH("exact_mstep_stats", s, done = launch_stats_sparse<kSpMstep>(a, nslab, s));
+  return done;
 }
 
 template <typename T>
@@ -1422,14 +1573,11 @@ void exact_fisher_batch(const T *X, const i64 *h_offsets, i64 numImages, const D
     VLB_CUDA(cudaMemcpyAsync(dsegs, segs.data(), sizeof(Segment) * nseg, cudaMemcpyHostToDevice, s));
     VLB_CUDA(cudaMemcpyAsync(dbeg, segBegin.data(), sizeof(int) * (nimg + 1), cudaMemcpyHostToDevice, s));
     VLB_CUDA(cudaMemcpyAsync(drows, rows.data(), sizeof(i64) * nimg, cudaMemcpyHostToDevice, s));
+    SparseStatsArgs<T> a{};
+    a.X = X; a.q = q; a.qbase = row0; a.K = (int)K; a.D = (int)D; a.segs = dsegs;
+    a.mu = m.means; a.sis = der.sis; a.priors = m.priors; a.p1 = pu; a.p2 = pv; a.pnt = pnt;
     bool sparse = false;
-    if constexpr (sizeof(T) == 4) {
-      // The sparse statistics kernel (same partials, float data up to 128 dimensions).
-      SparseStatsArgs a{};
-      a.X = X; a.q = q; a.qbase = row0; a.K = (int)K; a.D = (int)D; a.segs = dsegs;
-      a.mu = m.means; a.sis = der.sis; a.priors = m.priors; a.p1 = pu; a.p2 = pv; a.pnt = pnt;
-      sparse = launch_stats_sparse<kSpFisher>(a, nseg, s);
-    }
+    if (D <= 128) VLB_LAUNCH("exact_fisher_stats", s, sparse = launch_stats_sparse<kSpFisher>(a, nseg, s));
     if (!sparse) {
       dim3 g((unsigned)nseg, grid1(K, TKC), grid1(D, DB));
       VLB_LAUNCH("exact_fisher_stats", s,
@@ -1466,18 +1614,17 @@ i64 exact_fv_segments(i64 N) { return N > 0 ? (N + kFixedSegRows - 1) / kFixedSe
 void exact_fisher_single_fixed(const float *X, i64 N, const DevModel<float> &m, float *enc,
                                unsigned long long *nterms, int flags, const ExactFvScratch &sc,
                                cudaStream_t s) {
-  constexpr int TKC = 32, RC = 32, JMAX = 10, DB = 8 * JMAX;
-  const i64 K = m.K, D = m.D, nseg = exact_fv_segments(N);
+  const i64 K = m.K, D = m.D, nseg = exact_fv_segments(N);  // D <= 128 here
   VLB_LAUNCH_PLAIN(s, k_single_segments<<<1, 32, 0, s>>>(N, nseg, sc.segs, sc.segBegin, sc.rows));
   VLB_LAUNCH_PLAIN(s, k_prepare<float><<<prepare_grid<float>(K), 128, 0, s>>>(
                           m.priors, m.means, m.covs, (int)K, (int)D, half_dim_log_2pi<float>(D), nullptr,
                           sc.cst, sc.sis, sc.img));
   if (N > 0)  // numClusters <= 256 here: one kernel
     VLB_LAUNCH_PLAIN(s, launch_estep<float>(X, N, D, K, sc.img, sc.cst, sc.q, (flags & 4) != 0, nullptr, s));
-  dim3 g2((unsigned)nseg, grid1(K, TKC), grid1(D, DB));
-  VLB_LAUNCH_PLAIN(s, (k_fisher_stats<float, TKC, RC, JMAX><<<g2, kThreads, 0, s>>>(
-                          X, sc.q, 0, (int)K, (int)D, sc.segs, m.means, sc.sis, m.priors, sc.pu,
-                          sc.pv, sc.pnt)));
+  SparseStatsArgs<float> a{};
+  a.X = X; a.q = sc.q; a.qbase = 0; a.K = (int)K; a.D = (int)D; a.segs = sc.segs;
+  a.mu = m.means; a.sis = sc.sis; a.priors = m.priors; a.p1 = sc.pu; a.p2 = sc.pv; a.pnt = sc.pnt;
+  VLB_LAUNCH_PLAIN(s, launch_stats_sparse<kSpFisher>(a, nseg, s));
   VLB_LAUNCH_PLAIN(s, k_fisher_finalize<float><<<1, kThreads, 0, s>>>(
                           (int)K, (int)D, sc.segBegin, sc.rows, sc.pu, sc.pv, sc.pnt, m.priors,
                           flags, 0, enc, nterms));
