@@ -70,3 +70,32 @@ def test_em_step(vl, restatement, K, D, N, dtype):
     out = restatement.maximization(q, x, pr, mu, cv, np.full(D, 1e-4))
     for got, ref in zip((g.priors, g.means, g.covariances), out):
         assert rel_err(got, ref) < TOL[dtype]
+
+
+@pytest.mark.parametrize("flags", [0, 3])
+@pytest.mark.parametrize("dtype,K,D,N", [(np.float64, 1604, 130, 40), (np.float32, 2, 3, 5000), (np.float64, 9, 7, 4097)])
+def test_fisher_finalize_parts(vl, restatement, dtype, K, D, N, flags):
+    """A vector too long for the blocks' shared memory, one shorter than the
+    cluster, and images of several segments."""
+    vl.set_precision("exact")
+    r, pr, mu, cv = _model(K, D, dtype, K + D)
+    x = (mu[r.integers(0, K, N)] + r.standard_normal((N, D))).astype(dtype)
+    enc, _ = vl.fisher_encode(x, mu, cv, pr, flags)
+    ref, _ = restatement.fisher(x, mu, cv, pr, flags)
+    assert rel_err(enc, ref) < TOL[dtype]
+
+
+@pytest.mark.parametrize("N", [1, 255, 256, 257, 64 * 256, 64 * 256 + 1, 129 * 256])
+def test_em_slab_counts(vl, restatement, N):
+    """Slab sums of 1, 2, 64, 65 and 129 slabs (rounds of 64), in double."""
+    r, pr, mu, cv = _model(3, 11, np.float64, N)
+    x = mu[r.integers(0, 3, N)] + r.standard_normal((N, 11))
+    g = vl.GMM(11, 3, np.float64)
+    g.set_initialization("custom")
+    g.set_means(mu); g.set_covariances(cv); g.set_priors(pr)
+    g.set_max_num_iterations(1)
+    g.set_covariance_lower_bound(1e-4)
+    g.cluster(x)
+    q, _ = restatement.posteriors(x, pr, mu, cv)
+    for got, ref in zip((g.priors, g.means, g.covariances), restatement.maximization(q, x, pr, mu, cv, np.full(11, 1e-4))):
+        assert rel_err(got, ref) < TOL[np.float64]

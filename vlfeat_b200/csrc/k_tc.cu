@@ -43,6 +43,7 @@
 #include <cooperative_groups.h>
 
 #include "engine.h"
+#include "ordered_sum.cuh"
 #include "tc_common.cuh"
 
 extern "C" {
@@ -1390,24 +1391,27 @@ __global__ void __cluster_dims__(kFinCluster, 1, 1) __launch_bounds__(kFinThread
 // Sums of the item partials in f64, item order: S0[k] = sum q, S1[k][d] =
 // sum q x'', S2[k][d] = sum q x''^2, with the q 2^14 and x'' = x' scale
 // factors (powers of two, so exact) taken out.
-__global__ void k_tc_mstep_sums(int nitems, int K, int Kp, int D, const float *__restrict__ partial,
-                                const float *__restrict__ scale, double *__restrict__ S0,
-                                double *__restrict__ S1, double *__restrict__ S2) {
-  const i64 idx = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (i64)K * D) return;
-  const int k = (int)(idx / D), d = (int)(idx % D);
+// 32 (component, dimension) elements per block; 123 items of K = 256, D = 128:
+// 23 us (a thread per element: 58).
+__global__ void __launch_bounds__(kOrdThreads) k_tc_mstep_sums(int nitems, int K, int Kp, int D,
+                                                               const float *__restrict__ partial,
+                                                               const float *__restrict__ scale,
+                                                               double *__restrict__ S0, double *__restrict__ S1,
+                                                               double *__restrict__ S2) {
+  __shared__ OrdShared<3> sh;
+  const i64 KD = (i64)K * D, idx = (i64)blockIdx.x * 32 + threadIdx.x % 32, at = min(idx, KD - 1);
+  const int k = (int)(at / D), d = (int)(at % D);
   const int NST = 2 * D + 16;
-  double s0 = 0, s1 = 0, s2 = 0;
-  for (int it = 0; it < nitems; ++it) {
-    const float *pp = partial + ((size_t)it * Kp + k) * NST;
-    s0 += (double)pp[2 * D];
-    s1 += (double)pp[d];
-    s2 += (double)pp[D + d];
-  }
+  const size_t stride = (size_t)Kp * NST;
+  const float *pp = partial + (size_t)k * NST;
+  double s[3];
+  ordered_sums<3>(
+      nitems, [&](int it, int q) { return (double)pp[it * stride + (q == 0 ? 2 * D : q == 1 ? d : D + d)]; }, sh, s);
+  if (threadIdx.x >= 32 || idx >= KD) return;
   const double is = scale ? 1.0 / (double)scale[d] : 1.0, iq = 1.0 / (double)kQScale;
-  if (d == 0) S0[k] = s0 * iq;
-  S1[idx] = s1 * (is * iq);
-  S2[idx] = s2 * (is * is * iq);
+  if (d == 0) S0[k] = s[0] * iq;
+  S1[idx] = s[1] * (is * iq);
+  S2[idx] = s[2] * (is * is * iq);
 }
 
 // The M-step from those sums: the reference's mean and variance about the
@@ -2001,7 +2005,7 @@ void tc_em_sums(int nitems, const float *partial, i64 K, i64 D, double *S0, doub
                 cudaStream_t s) {
   Scratch &sc = thread_scratch(kArenaTc);
   VLB_LAUNCH("tc_mstep_sums", s,
-             k_tc_mstep_sums<<<(unsigned)((K * D + 255) / 256), 256, 0, s>>>(
+             k_tc_mstep_sums<<<(unsigned)((K * D + 31) / 32), kOrdThreads, 0, s>>>(
                  nitems, (int)K, padK(K), (int)D, partial, (const float *)sc.slot[12].p, S0, S1, S2));
 }
 
