@@ -17,6 +17,28 @@ __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(
 __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
 
+// The lane sums v over elements [0, i) reduced in the SIMD pattern, then the
+// remaining elements added in order.
+template <typename T, int L>
+__device__ __forceinline__ T l2_ordered_tail(const T (&v)[L], const T *__restrict__ a, int as, const T *__restrict__ b,
+                                             int i, int D) {
+  T acc;
+  if constexpr (L == 8) {
+    acc = add_rn(add_rn(add_rn(v[0], v[1]), add_rn(v[4], v[5])), add_rn(add_rn(v[2], v[3]), add_rn(v[6], v[7])));
+  } else if constexpr (L == 4) {
+    acc = add_rn(add_rn(v[0], v[2]), add_rn(v[1], v[3]));
+  } else if constexpr (L == 2) {
+    acc = add_rn(v[0], v[1]);
+  } else {
+    acc = v[0];
+  }
+  for (; i < D; ++i) {
+    const T dl = sub_rn(a[i * as], b[i]);
+    acc = add_rn(acc, mul_rn(dl, dl));
+  }
+  return acc;
+}
+
 // Squared L2 distance in the order of the reference's kernel for VlDistanceL2
 // (vl/mathop.c:472-513): L lanes accumulate (a - b)^2 over consecutive groups
 // of L elements (lane l takes elements l, l + L, ...), the lanes are reduced
@@ -38,23 +60,8 @@ __device__ __forceinline__ T l2_ordered_s(const T *__restrict__ a, int as, const
       v[l] = add_rn(v[l], mul_rn(dl, dl));
     }
   }
-  T acc;
-  if constexpr (L == 8) {
-    acc = add_rn(add_rn(add_rn(v[0], v[1]), add_rn(v[4], v[5])), add_rn(add_rn(v[2], v[3]), add_rn(v[6], v[7])));
-  } else if constexpr (L == 4) {
-    acc = add_rn(add_rn(v[0], v[2]), add_rn(v[1], v[3]));
-  } else if constexpr (L == 2) {
-    acc = add_rn(v[0], v[1]);
-  } else {
-    acc = v[0];
-  }
-  for (; i < D; ++i) {
-    const T dl = sub_rn(a[i * as], b[i]);
-    acc = add_rn(acc, mul_rn(dl, dl));
-  }
-  return acc;
+  return l2_ordered_tail<T, L>(v, a, as, b, i, D);
 }
-
 template <typename T, int L>
 __device__ __forceinline__ T l2_ordered(const T *__restrict__ a, const T *__restrict__ b, int D) {
   return l2_ordered_s<T, L>(a, 1, b, D);

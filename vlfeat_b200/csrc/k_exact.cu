@@ -1720,121 +1720,397 @@ void exact_fisher_single_fixed(const float *X, i64 N, const DevModel<float> &m, 
 
 // Global data variance, vl/gmm.c:1376-1413: per dimension the mean, then the
 // sum of squared deviations, each accumulated over the rows in order and
-// divided by N and N - 1 (0 when N <= 1).  One thread per dimension.
+// divided by N and N - 1 (0 when N <= 1).  A block takes 32 dimensions: one
+// warp adds, a lane per dimension, out of a shared-memory ring of row tiles
+// that the other warps fill asynchronously several tiles ahead.  Bound by the
+// addition's latency, two chains of N additions: 100,000 rows take 0.76 ms
+// of 64 dimensions (a thread per dimension reading the rows from memory: 5.35).
+constexpr int kGvStages = 4, kGvUnroll = 32;
 template <typename T>
-__global__ void k_global_variance(const T *__restrict__ X, i64 N, int D, T *__restrict__ sigma) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= D) return;
-  if (N <= 1) {
-    sigma[d] = (T)0;
-    return;
-  }
-  T mean = (T)0;
-  for (i64 i = 0; i < N; ++i) mean = add_rn(mean, X[i * D + d]);
-  mean = div_rn(mean, (T)N);
-  T ss = (T)0;
-  for (i64 i = 0; i < N; ++i) {
-    const T diff = sub_rn(X[i * D + d], mean);
-    ss = add_rn(ss, mul_rn(diff, diff));
-  }
-  sigma[d] = div_rn(ss, (T)(N - 1));
+__host__ __device__ constexpr int gv_rows() { return 1024 / (int)sizeof(T); }  // rows per tile
+
+// A shared-memory load that stays where it is written.
+__device__ __forceinline__ float ld_volatile(const float *p) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(tc::smem_u32(p)));
+  return v;
+}
+__device__ __forceinline__ double ld_volatile(const double *p) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(tc::smem_u32(p)));
+  return v;
 }
 
-// minDist[x] = min(minDist[x], ||c - x||^2) with the reference's VL_MIN.
-template <typename T, int L>
-__global__ void k_kpp_update(const T *__restrict__ X, i64 N, int D, const T *__restrict__ center,
-                             T *__restrict__ minDist) {
-  extern __shared__ unsigned char kpp_smem[];
+// n rows of a tile added to acc: the values, or with SQ their squared
+// deviations from mean.
+template <bool SQ, typename T>
+__device__ __forceinline__ T gv_add(T acc, T mean, const T *__restrict__ src, int n) {
+  auto term = [&](T x) {
+    if constexpr (!SQ) return x;
+    const T diff = sub_rn(x, mean);
+    return mul_rn(diff, diff);
+  };
+  int r = 0;
+  // A group's loads beside the additions of the group before, in a loop short
+  // enough for the instruction cache.
+  if (n >= kGvUnroll) {
+    T v[kGvUnroll];
+#pragma unroll
+    for (int u = 0; u < kGvUnroll; ++u) v[u] = ld_volatile(src + u * 32);
+#pragma unroll 1
+    for (r = kGvUnroll; r + kGvUnroll <= n; r += kGvUnroll) {
+#pragma unroll
+      for (int u = 0; u < kGvUnroll; ++u) {
+        acc = add_rn(acc, term(v[u]));
+        v[u] = ld_volatile(src + (r + u) * 32);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kGvUnroll; ++u) acc = add_rn(acc, term(v[u]));
+  }
+  for (; r < n; ++r) acc = add_rn(acc, term(src[r * 32]));
+  return acc;
+}
+
+// VB: bytes per asynchronous copy (16 when rows are whole 16-byte pieces).
+template <typename T, int VB>
+__global__ void __launch_bounds__(256) k_global_variance(const T *__restrict__ X, i64 N, int D, T *__restrict__ sigma) {
+  extern __shared__ __align__(16) unsigned char gv_smem[];
+  constexpr int VE = VB / (int)sizeof(T), PR = 32 / VE;  // pieces per tile row
+  T *ring = (T *)gv_smem;  // [stage][row][32]
+  const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int d = blockIdx.x * 32 + lane;
+  if (N <= 1) {
+    if (w == 0 && d < D) sigma[d] = (T)0;
+    return;
+  }
+  constexpr int R = gv_rows<T>();
+  const int nt = (int)((N + R - 1) / R);  // tiles of one pass over the rows
+  const int dc = blockIdx.x * 32 + lane % PR * VE;
+  int jt = 0, js = 0;  // the next tile to copy, of two passes, and its stage
+  i64 jr = 0;          // its first row
+  auto issue = [&]() {
+    if (jt < 2 * nt) {
+      T *dst = ring + js * R * 32 + lane % PR * VE;
+      for (int r = (w - 1) * (32 / PR) + lane / PR; r < R; r += 7 * (32 / PR)) {
+        const bool in = jr + r < N && dc < D;
+        cp_async_piece<VB>(tc::smem_u32(dst + r * 32), in ? X + (jr + r) * D + dc : X, in);
+      }
+    }
+    cp_async_commit();
+    ++jt;
+    js = js + 1 == kGvStages ? 0 : js + 1;
+    jr = jt == nt ? 0 : jr + R;
+  };
+  if (w > 0) {
+    for (int t = 0; t < kGvStages - 1; ++t) issue();
+    for (int t = 0; t < 2 * nt; ++t) {
+      cp_async_wait<kGvStages - 2>();
+      __syncthreads();  // tile t has landed; the adding warp is done with tile t - 1
+      issue();
+    }
+    return;
+  }
+  T mean = (T)0, acc = (T)0;
+  int st = 0;
+  auto tile = [&]() {
+    __syncthreads();
+    const T *src = ring + st * R * 32 + lane;
+    st = st + 1 == kGvStages ? 0 : st + 1;
+    return src;
+  };
+  const int last = (int)(N - (i64)(nt - 1) * R);  // rows of the last tile
+  for (int t = 0; t < nt; ++t) acc = gv_add<false>(acc, mean, tile(), t + 1 < nt ? R : last);
+  mean = div_rn(acc, (T)N);
+  acc = (T)0;
+  for (int t = 0; t < nt; ++t) acc = gv_add<true>(acc, mean, tile(), t + 1 < nt ? R : last);
+  if (d < D) sigma[d] = div_rn(acc, (T)(N - 1));
+}
+
+// minDist[x] = min(minDist[x], ||c - x||^2) with the reference's VL_MIN, c the
+// row *xDev (or xHost when xDev is null, the first centre, whose distances
+// start minDist); block 0 copies the row to dst.  A row per thread, read 16
+// bytes at a time when VEC (D a multiple of 16 bytes, aligned data).
+template <typename T, int L, bool VEC>
+__global__ void __launch_bounds__(kThreads) k_kpp_update(const T *__restrict__ X, i64 N, int D,
+                                                         const i64 *__restrict__ xDev, i64 xHost, T *__restrict__ dst,
+                                                         T *__restrict__ minDist) {
+  extern __shared__ __align__(16) unsigned char kpp_smem[];
   T *c = (T *)kpp_smem;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) c[d] = center[d];
+  const i64 row = xDev ? *xDev : xHost;
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    const T v = X[row * D + d];
+    c[d] = v;
+    if (blockIdx.x == 0) dst[d] = v;
+  }
   __syncthreads();
   const i64 x = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= N) return;
-  const T dist = l2_ordered<T, L>(c, X + x * D, D);
-  const T m = minDist[x];
-  minDist[x] = m < dist ? m : dist;
-}
-
-template <typename T>
-__global__ void k_fill(T *__restrict__ p, i64 n, T v) {
-  const i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
-}
-
-// The next centre, vl/kmeans.c:631-641: the energy (sum of minDist in
-// order), then the first x with acc >= thresh * energy, or N - 1.
-// The scan's running sum acc is the energy's own prefix sum (both add minDist
-// in order from 0).  So the energy pass keeps every 32nd prefix; the scan
-// bisects these checkpoints (prefixes of non-negative terms never decrease, and
-// a NaN prefix, then every later one, fails the test as in the loop) and
-// re-adds at most 32 terms from the checkpoint before, which reproduces the
-// prefixes exactly.  One sequential pass of N additions instead of two.
-// One block: thread 0 adds in order out of shared memory while the warps on
-// the other three schedulers stage the next chunk of minDist, so the chain
-// waits on no load and shares its scheduler with no loader.
-constexpr int kKppCk = 32;  // terms per checkpoint
-
-template <typename T>
-__global__ void __launch_bounds__(1024) k_kpp_select(const T *__restrict__ minDist, i64 N, T thresh,
-                                                     T *__restrict__ ck, i64 *__restrict__ xOut) {
-  constexpr int kChunk = 16384 / (int)sizeof(T);  // 32 KB of staging in all
-  __shared__ T buf[2][kChunk];
-  const int tid = threadIdx.x;
-  const i64 nch = (N + kChunk - 1) / kChunk;
-  auto stage = [&](i64 ch, int b, int t0, int nt) {
-    const i64 base = ch * kChunk;
-    const int n = (int)min((i64)kChunk, N - base);
-    for (int e = t0; e < n; e += nt) buf[b][e] = minDist[base + e];
-  };
-  stage(0, 0, tid, blockDim.x);
-  __syncthreads();
-  T energy = (T)0;
-  for (i64 ch = 0; ch < nch; ++ch) {
-    const int b = (int)(ch & 1);
-    if (tid == 0) {
-      const i64 base = ch * kChunk;
-      const int n = (int)min((i64)kChunk, N - base);
-      int e = 0;
-      for (; e + kKppCk <= n; e += kKppCk) {  // kChunk is a multiple of kKppCk
+  T dist;
+  if constexpr (VEC) {
+    // l2_ordered's lane sums with the row in registers one group at a time.
+    constexpr int VE = 16 / (int)sizeof(T);
+    using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+    constexpr int G = L > VE ? L : VE;  // elements per step: whole lane groups and whole vectors
+    T v[L];
 #pragma unroll
-        for (int g = 0; g < kKppCk; g += 8) {
-          T v[8];
+    for (int l = 0; l < L; ++l) v[l] = (T)0;
+    const T *xr = X + x * D;
+    int i = 0;
+#pragma unroll 4
+    for (; i + G <= D; i += G) {
 #pragma unroll
-          for (int u = 0; u < 8; ++u) v[u] = buf[b][e + g + u];
+      for (int g = 0; g < G / VE; ++g) {
+        const V w = __ldg((const V *)(xr + i) + g);
+        const T *wp = (const T *)&w;
 #pragma unroll
-          for (int u = 0; u < 8; ++u) energy = add_rn(energy, v[u]);
+        for (int e = 0; e < VE; ++e) {
+          const T dl = sub_rn(c[i + g * VE + e], wp[e]);
+          v[(g * VE + e) % L] = add_rn(v[(g * VE + e) % L], mul_rn(dl, dl));
         }
-        ck[(base + e) / kKppCk] = energy;
       }
-      for (; e < n; ++e) energy = add_rn(energy, buf[b][e]);
-    } else if ((tid >> 5) & 3) {
-      const int w = tid >> 5, li = (w - w / 4 - 1) * 32 + (tid & 31), nl = (int)blockDim.x / 4 * 3;
-      if (ch + 1 < nch) stage(ch + 1, b ^ 1, li, nl);
     }
-    __syncthreads();
+    dist = l2_ordered_tail<T, L>(v, c, 1, xr, i, D);
+  } else {
+    dist = l2_ordered<T, L>(c, X + x * D, D);
   }
-  if (tid != 0) return;
-  const T t = mul_rn(thresh, energy);
-  // The first checkpoint j with ck[j] >= t (nck if none); the answer lies in
-  // terms [32 j, 32 j + 32), re-added from checkpoint j - 1.
-  const i64 nck = N / kKppCk;
-  i64 lo = 0, hi = nck;
-  while (lo < hi) {
-    const i64 mid = lo + (hi - lo) / 2;
-    if (ck[mid] >= t) hi = mid;
-    else lo = mid + 1;
+  if (!xDev) {
+    minDist[x] = dist;
+  } else {
+    const T m = minDist[x];
+    minDist[x] = m < dist ? m : dist;
   }
-  T acc = lo > 0 ? ck[lo - 1] : (T)0;
-  i64 x = lo * kKppCk;
-  const i64 end = min(N, x + kKppCk);
-  for (; x < end; ++x) {
-    acc = add_rn(acc, minDist[x]);
-    if (acc >= t) break;
-  }
-  *xOut = min(x, N - 1);  // none before N - 1: the last row
 }
 
-// centers[c] = X[x] with x the selected row (device) or the first row (host).
+// ---- a sequential floating-point sum, formed in parallel ----
+// The sum acc = rn(acc + v_i), in order, of non-negative terms: while acc stays
+// in one binade [2^e, 2^(e+1)) it is an integer A times the binade's ulp u, and
+// an addition adds to A the term rounded to a multiple of u; only an exact tie
+// depends on acc, through A's parity (round half to even).  So a run of terms
+// maps A's parity to an increment, such maps compose associatively, and a
+// block scans them; the term that takes acc past the binade (or is not a
+// finite non-negative number) is added by its thread as it is, and the scan
+// goes on from there with the next binade.  Zero and subnormal acc count as
+// the lowest binade, whose ulp they share.  Every prefix has the bits of the
+// loop's.
+template <typename T>
+struct SeqFloat;
+template <>
+struct SeqFloat<float> {
+  using U = uint32_t;
+  static constexpr int kMant = 23, kExpMax = 255;
+  static __device__ __forceinline__ U bits(float v) { return __float_as_uint(v); }
+  static __device__ __forceinline__ float value(U b) { return __uint_as_float(b); }
+};
+template <>
+struct SeqFloat<double> {
+  using U = unsigned long long;
+  static constexpr int kMant = 52, kExpMax = 2047;
+  static __device__ __forceinline__ U bits(double v) { return (U)__double_as_longlong(v); }
+  static __device__ __forceinline__ double value(U b) { return __longlong_as_double((long long)b); }
+};
+template <typename T>
+struct Seq {
+  using F = SeqFloat<T>;
+  using U = typename F::U;
+  static constexpr U kOne = (U)1 << F::kMant, kLim = kOne * 2, kSat = kOne * 4;
+  // A map is 4 i + (d + 1): i is the increment of an even A (at most kSat), d in
+  // {-1, 0, 1} how much more an odd A gains.  (A tie sends one of the two
+  // starts up and the other down; from then on both have the same parity, so
+  // d stays.)
+  static constexpr U kIdentity = 1;
+  static __device__ __forceinline__ U pack(U i, int d) { return ((i < kSat ? i : kSat) << 2) | (U)(d + 1); }
+  static __device__ __forceinline__ int diff(U m) { return (int)(m & 3) - 1; }
+  static __device__ __forceinline__ U gain(U m, bool odd) { return (m >> 2) + (U)(odd ? diff(m) : 0); }
+  static __device__ __forceinline__ U then(U a, U b) {
+    const bool odd = ((a >> 2) & 1) != 0;
+    const int da = diff(a), db = diff(b);
+    return pack((a >> 2) + gain(b, odd), da ? da : odd ? -db : db);
+  }
+  // Biased exponent (at least 1) and integer of a finite non-negative value.
+  static __device__ __forceinline__ int exponent(U b) { return max(1, (int)(b >> F::kMant)); }
+  static __device__ __forceinline__ U integer(U b) { return (b & (kOne - 1)) | (b >> F::kMant ? kOne : (U)0); }
+  static __device__ __forceinline__ T value(int be, U A) {
+    return F::value(A < kOne ? A : ((U)be << F::kMant) + (A - kOne));  // A < kOne only in the lowest binade
+  }
+  // The map of a run of terms, acc in the binade with biased exponent be: the
+  // run added to the binade's first value (an even A) and to the next (odd).
+  // A sum that leaves the binade, or is not a number, saturates: whatever A it
+  // starts from, its thread adds the terms as they are.
+  template <int EPT>
+  static __device__ __forceinline__ U run(const T (&v)[EPT], int be) {
+    const U b0 = (U)be << F::kMant;
+    T x0 = F::value(b0), x1 = F::value(b0 + 1);
+    const T lim = add_rn(x0, x0);
+#pragma unroll
+    for (int u = 0; u < EPT; ++u) {
+      x0 = add_rn(x0, v[u]);
+      x1 = add_rn(x1, v[u]);
+    }
+    if (!(x0 < lim && x1 < lim && x0 >= F::value(b0))) return pack(kSat, 0);
+    const U i = F::bits(x0) - b0;
+    return pack(i, (int)(F::bits(x1) - b0 - 1 - i));
+  }
+};
+
+constexpr int kKppThreads = 256, kKppStages = 4;
+template <typename T>
+__host__ __device__ constexpr int kpp_ept() { return 128 / (int)sizeof(T); }  // terms per thread and tile
+template <typename T>
+__host__ __device__ constexpr int kpp_tile() { return kKppThreads * kpp_ept<T>(); }
+
+// The next centre, vl/kmeans.c:631-641: the energy (sum of minDist in order),
+// then the first x whose prefix sum is >= thresh * energy, or N - 1 (a NaN
+// energy fails every test).  The prefixes are the energy's own, so the energy
+// pass keeps one per tile (8192 terms, 4096 in double) and only the tile that holds the answer
+// is scanned again.  One block: 100,000 terms take 28 us, 1 M 138 us; a
+// thread that adds in order takes 290 and 2,900 (7 clocks a term).
+template <typename T>
+__global__ void __launch_bounds__(kKppThreads) k_kpp_select(const T *__restrict__ minDist, i64 N, T thresh,
+                                                            T *__restrict__ ck, i64 *__restrict__ xOut) {
+  using S = Seq<T>;
+  using U = typename S::U;
+  constexpr int NW = kKppThreads / 32, EPT = kpp_ept<T>(), kTile = kpp_tile<T>();
+  __shared__ U s_warp[2][NW];
+  __shared__ T s_acc;
+  __shared__ int s_next, s_tile;
+  __shared__ i64 s_x;
+  extern __shared__ __align__(16) unsigned char kps_smem[];
+  constexpr int VE = 16 / (int)sizeof(T), P = EPT + VE;  // a thread's terms and 16 bytes, so that its reads spread over the banks
+  T *ring = (T *)kps_smem;                               // [stage][thread][P]
+  const int tid = threadIdx.x, lane = tid % 32, w = tid / 32;
+  const i64 ntile = (N + kTile - 1) / kTile;
+  int pb = 0;  // warp totals' buffer: a pass writes the one the pass before did not
+  // Terms of a tile to its stage, zeros past the end; and this thread's terms from there.
+  auto issue = [&](i64 tile, int stage) {
+    if (tile < ntile)
+#pragma unroll
+      for (int u = 0; u < kTile / VE / kKppThreads; ++u) {
+        const int e = (u * kKppThreads + tid) * VE;
+        const i64 i = tile * kTile + e;
+        const i64 left = N - i;
+        const uint32_t bytes = left >= VE ? 16u : left > 0 ? (uint32_t)(left * (i64)sizeof(T)) : 0u;
+        cp_async16(tc::smem_u32(ring + ((size_t)stage * kKppThreads + e / EPT) * P + e % EPT),
+                   bytes ? minDist + i : minDist, bytes);
+      }
+    cp_async_commit();
+  };
+  auto load = [&](int stage, T(&v)[EPT]) {
+    const T *src = ring + ((size_t)stage * kKppThreads + tid) * P;
+#pragma unroll
+    for (int u = 0; u < EPT; u += VE) {
+      using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+      const V x = *(const V *)(src + u);
+#pragma unroll
+      for (int e = 0; e < VE; ++e) v[u + e] = ((const T *)&x)[e];
+    }
+  };
+  auto scan = [&](U m, int width) {
+    if (!__any_sync(0xffffffffu, S::diff(m) != 0)) {  // no ties: plain saturating sums
+      U i = m >> 2;
+#pragma unroll
+      for (int o = 1; o < width; o <<= 1) {
+        const U p = __shfl_up_sync(0xffffffffu, i, o);
+        if (lane >= o) i = min(i + p, S::kSat);
+      }
+      return S::pack(i, 0);
+    }
+#pragma unroll
+    for (int o = 1; o < width; o <<= 1) {
+      const U p = __shfl_up_sync(0xffffffffu, m, o);
+      if (lane >= o) m = S::then(p, m);
+    }
+    return m;
+  };
+  // Adds the tile's terms to acc; with find, stops at the first prefix >= t and
+  // returns true (its index in s_x).  All threads hold the same acc.
+  auto run = [&](const T(&v)[EPT], T &acc, bool find, T t, i64 base) -> bool {
+    int from = 0;  // first thread whose terms are not in acc
+    while (from < kKppThreads) {
+      if (!(acc < (T)INFINITY)) {
+        // NaN stays; infinity turns into NaN at a NaN or -infinity.
+        bool nan = false;
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) nan |= tid >= from && !(v[u] > -(T)INFINITY);
+        if (__syncthreads_or(nan)) acc = add_rn(acc, (T)NAN);
+        return false;
+      }
+      const U ab = S::F::bits(acc), A = S::integer(ab);
+      const int be = S::exponent(ab);
+      const bool odd = (A & 1) != 0;
+      const U m = scan(tid >= from ? S::run(v, be) : S::kIdentity, 32);
+      if (lane == 31) s_warp[pb][w] = m;
+      __syncthreads();
+      const U x = scan(lane < NW ? s_warp[pb][lane] : S::kIdentity, NW);  // inclusive over the warps, in every warp
+      pb ^= 1;
+      auto stops = [&](U end) { return end >= S::kLim || (find && S::value(be, end) >= t); };
+      const unsigned at = __ballot_sync(0xffffffffu, lane < NW && stops(A + S::gain(x, odd)));
+      if (!at) {
+        acc = S::value(be, A + S::gain(__shfl_sync(0xffffffffu, x, NW - 1), odd));
+        return false;
+      }
+      // The first thread whose terms leave the binade (or reach t) adds them.
+      const U before = __shfl_sync(0xffffffffu, x, max(w - 1, 0));
+      if (w == __ffs(at) - 1) {
+        const U prev = w > 0 ? before : S::kIdentity;
+        const U incl = S::then(prev, m), up = __shfl_up_sync(0xffffffffu, incl, 1);
+        const unsigned in = __ballot_sync(0xffffffffu, stops(A + S::gain(incl, odd)));
+        if (lane == __ffs(in) - 1) {
+          T y = S::value(be, A + S::gain(lane > 0 ? up : prev, odd));
+          i64 hit = -1;
+#pragma unroll
+          for (int u = 0; u < EPT; ++u) {
+            y = add_rn(y, v[u]);
+            if (find && hit < 0 && y >= t) hit = base + tid * EPT + u;
+          }
+          s_acc = y;
+          s_next = tid + 1;
+          s_x = hit;
+        }
+      }
+      __syncthreads();
+      acc = s_acc;
+      from = s_next;
+      if (find && s_x >= 0) return true;
+    }
+    return false;
+  };
+  T v[EPT];
+  T acc = (T)0;
+  for (int t = 0; t < kKppStages - 1; ++t) issue(t, t);
+  for (i64 tile = 0; tile < ntile; ++tile) {
+    cp_async_wait<kKppStages - 2>();
+    __syncthreads();  // the tile has landed; every thread has read the one before
+    load((int)(tile % kKppStages), v);
+    issue(tile + kKppStages - 1, (int)((tile + kKppStages - 1) % kKppStages));
+    run(v, acc, false, (T)0, 0);
+    if (tid == 0) ck[tile] = acc;
+  }
+  cp_async_wait<0>();
+  // The first tile whose last prefix reaches the threshold.
+  const T t = mul_rn(thresh, acc);
+  if (tid == 0) s_tile = 0x7fffffff;
+  __syncthreads();
+  for (i64 j = tid; j < ntile; j += kKppThreads)
+    if (ck[j] >= t) {
+      atomicMin(&s_tile, (int)j);
+      break;
+    }
+  __syncthreads();
+  const int tile = s_tile;
+  if (tile == 0x7fffffff) {
+    if (tid == 0) *xOut = N - 1;
+    return;
+  }
+  acc = tile > 0 ? ck[tile - 1] : (T)0;
+  issue(tile, 0);
+  cp_async_wait<0>();
+  __syncthreads();
+  load(0, v);
+  const bool found = run(v, acc, true, t, (i64)tile * kTile);
+  if (tid == 0) *xOut = found ? min(s_x, N - 1) : N - 1;
+}
+
 template <typename T>
 __global__ void k_kpp_copy(const T *__restrict__ X, int D, const i64 *__restrict__ xDev, i64 xHost,
                            T *__restrict__ dst) {
@@ -1844,8 +2120,21 @@ __global__ void k_kpp_copy(const T *__restrict__ X, int D, const i64 *__restrict
 
 template <typename T>
 void global_variance(const T *X, i64 N, i64 D, T *sigma, cudaStream_t s) {
-  VLB_LAUNCH("global_variance", s, k_global_variance<T><<<grid1(D, 128), 128, 0, s>>>(X, N, (int)D, sigma));
+  constexpr size_t smem = sizeof(T) * kGvStages * gv_rows<T>() * 32;
+  const bool vec = D % (16 / (i64)sizeof(T)) == 0 && ((uintptr_t)X & 15) == 0;
+  auto kern = vec ? k_global_variance<T, 16> : k_global_variance<T, (int)sizeof(T)>;
+  VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  VLB_LAUNCH("global_variance", s, kern<<<grid1(D, 32), 256, smem, s>>>(X, N, (int)D, sigma));
 }
+
+namespace {
+template <typename T, int L>
+void launch_kpp_update(const T *X, i64 N, i64 D, const i64 *xDev, i64 x0, T *dst, T *minDist, cudaStream_t s) {
+  const bool vec = D % (16 / (i64)sizeof(T)) == 0 && ((uintptr_t)X & 15) == 0;
+  auto kern = vec ? k_kpp_update<T, L, true> : k_kpp_update<T, L, false>;
+  VLB_LAUNCH("kpp_update", s, kern<<<grid1(N, kThreads), kThreads, sizeof(T) * D, s>>>(X, N, (int)D, xDev, x0, dst, minDist));
+}
+}  // namespace
 
 template <typename T>
 void kmeanspp(const T *X, i64 N, i64 D, i64 K, T *centers, i64 x0, const std::vector<T> &thresh, int lanes,
@@ -1855,22 +2144,22 @@ void kmeanspp(const T *X, i64 N, i64 D, i64 K, T *centers, i64 x0, const std::ve
   Scratch &sc = thread_scratch(kArenaExact);
   T *minDist = sc.slot[20].get<T>(N);
   i64 *xdev = sc.slot[21].get<i64>(1);
-  T *ck = sc.slot[22].get<T>(N / kKppCk + 1);
-  const T inf = (T)INFINITY;
-  VLB_LAUNCH("kpp_fill", s, k_fill<T><<<grid1(N, kThreads), kThreads, 0, s>>>(minDist, N, inf));
-  const size_t smem = sizeof(T) * D;
+  T *ck = sc.slot[22].get<T>(N / kpp_tile<T>() + 1);
+  constexpr size_t ssmem = (size_t)kKppStages * kKppThreads * (kpp_ept<T>() * sizeof(T) + 16);
+  VLB_CUDA(cudaFuncSetAttribute(k_kpp_select<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem));
   for (i64 c = 0; c < K; ++c) {
-    VLB_LAUNCH("kpp_copy", s, k_kpp_copy<T><<<1, 128, 0, s>>>(X, (int)D, c == 0 ? nullptr : xdev, x0,
-                                                               centers + c * D));
-    if (c + 1 == K) break;
-    const T *ctr = centers + c * D;
-    switch (lanes) {
-      case 8: VLB_LAUNCH("kpp_update", s, (k_kpp_update<T, 8><<<grid1(N, kThreads), kThreads, smem, s>>>(X, N, (int)D, ctr, minDist))); break;
-      case 4: VLB_LAUNCH("kpp_update", s, (k_kpp_update<T, 4><<<grid1(N, kThreads), kThreads, smem, s>>>(X, N, (int)D, ctr, minDist))); break;
-      case 2: VLB_LAUNCH("kpp_update", s, (k_kpp_update<T, 2><<<grid1(N, kThreads), kThreads, smem, s>>>(X, N, (int)D, ctr, minDist))); break;
-      default: VLB_LAUNCH("kpp_update", s, (k_kpp_update<T, 1><<<grid1(N, kThreads), kThreads, smem, s>>>(X, N, (int)D, ctr, minDist))); break;
+    const i64 *xp = c == 0 ? nullptr : xdev;
+    if (c + 1 == K) {
+      VLB_LAUNCH("kpp_copy", s, k_kpp_copy<T><<<1, 128, 0, s>>>(X, (int)D, xp, x0, centers + c * D));
+      break;
     }
-    VLB_LAUNCH("kpp_select", s, k_kpp_select<T><<<1, 1024, 0, s>>>(minDist, N, thresh[c], ck, xdev));
+    switch (lanes) {
+      case 8: launch_kpp_update<T, 8>(X, N, D, xp, x0, centers + c * D, minDist, s); break;
+      case 4: launch_kpp_update<T, 4>(X, N, D, xp, x0, centers + c * D, minDist, s); break;
+      case 2: launch_kpp_update<T, 2>(X, N, D, xp, x0, centers + c * D, minDist, s); break;
+      default: launch_kpp_update<T, 1>(X, N, D, xp, x0, centers + c * D, minDist, s); break;
+    }
+    VLB_LAUNCH("kpp_select", s, k_kpp_select<T><<<1, kKppThreads, ssmem, s>>>(minDist, N, thresh[c], ck, xdev));
   }
 }
 
