@@ -38,6 +38,7 @@
 #include <functional>
 #include <memory>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -88,163 +89,249 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Centre m_d = mean over components of mu_kd.  One warp per dimension.
-__global__ void k_tc_center(const float *__restrict__ means, int K, int D, float *__restrict__ ctr) {
-  const int d = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
-  if (d >= D) return;
-  double s = 0;
-  for (int k = lane; k < K; k += 32) s += (double)means[(i64)k * D + d];
-  s = warp_sum(s);
-  if (lane == 0) ctr[d] = (float)(s / (double)K);
-}
-
 // The x''^2 weight of component k and dimension d, -1/2 / s2_kd / scale_d^2
 // log2(e), before the common part is taken out.
-__device__ __forceinline__ double tc_weight2(const float *__restrict__ covs, const float *__restrict__ scale,
-                                             int k, int d, int D) {
-  const double s2 = (double)covs[(i64)k * D + d], sc = (double)scale[d];
+__device__ __forceinline__ double tc_weight2(const float *__restrict__ covs, double sc, int k, int d, int D) {
+  const double s2 = (double)covs[(i64)k * D + d];
   return -0.5 / s2 / (sc * sc) * 1.4426950408889634;
 }
-
-// Common part of the x''^2 weights: wbar_d = mean over the components of
-// tc_weight2 (fixed-order sums, one warp per dimension).  The logits of a
-// row change by the same amount sum_d wbar_d x''_d^2 when it is taken out of
-// every component's weights, so the posteriors do not change, while the
-// terms the fp32 accumulator adds (and the logit it rounds) shrink by about
-// an order of magnitude; the log-likelihood adds the common part back.
-__global__ void k_tc_wbar(const float *__restrict__ covs, const float *__restrict__ scale, int K, int D,
-                          float *__restrict__ wbar) {
-  const int d = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
-  if (d >= D) return;
-  double s = 0;
-  for (int k = lane; k < K; k += 32) s += tc_weight2(covs, scale, k, d, D);
-  s = warp_sum(s);
-  if (lane == 0) wbar[d] = (float)(s / (double)K);
-}
-
-// Entries of the E-step's weight matrix for component k and K-order element
-// e (chunk c = e / 32 holds x''_d for d = 16c .. 16c+15, then x''_d^2 for the
-// same d, so that the producers read each element of x once):
-//   [mu'_kd / s2_kd / scale_d, -1/2 / s2_kd / scale_d^2 - wbar_d] log2(e),
-// the producers multiplying x' by the power of two scale_d.
-__device__ __forceinline__ double tc_weight(const float *__restrict__ means, const float *__restrict__ covs,
-                                            const float *__restrict__ ctr, const float *__restrict__ scale,
-                                            const float *__restrict__ wbar, int k, int e, int D) {
-  const int c = e / 32, ee = e % 32, d = 16 * c + (ee & 15);
-  if (ee >= 16) return tc_weight2(covs, scale, k, d, D) - (double)wbar[d];
-  const double s2 = (double)covs[(i64)k * D + d], sc = (double)scale[d];
-  const double mup = (double)means[(i64)k * D + d] - (double)ctr[d];
+// The x'' weight of component k and dimension d, mu'_kd / s2_kd / scale_d log2(e).
+__device__ __forceinline__ double tc_weight1(const float *__restrict__ means, const float *__restrict__ covs,
+                                             double ctr, double sc, int k, int d, int D) {
+  const double s2 = (double)covs[(i64)k * D + d];
+  const double mup = (double)means[(i64)k * D + d] - ctr;
   return mup / s2 / sc * 1.4426950408889634;
 }
 
-// max |w| over the model: one element per thread, a warp maximum, then an
-// atomic maximum on the float's bits (non-negative floats order as their bits;
-// *wmax is zeroed before the launch).  The maximum does not depend on order.
-__global__ void k_tc_wmax(const float *__restrict__ means, const float *__restrict__ covs,
-                          const float *__restrict__ ctr, const float *__restrict__ scale,
-                          const float *__restrict__ wbar, int K, int D, float *__restrict__ wmax) {
-  const i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  float m = 0.f;
-  if (i < (i64)K * 2 * D)
-    m = (float)fabs(tc_weight(means, covs, ctr, scale, wbar, (int)(i / (2 * D)), (int)(i % (2 * D)), D));
+// Per dimension d (one block each, fixed-order sums over the components):
+//  ctr_d    the mean over the components of mu_kd;
+//  scale_d  the power of two 2^-ceil(log2(max_k |mu'_kd| + 4 sigma_kd)), so
+//           that x'' = x' scale_d is O(1) for data the model describes;
+//  wbar_d   the mean over the components of tc_weight2: the logits of a row
+//           change by the same amount sum_d wbar_d x''_d^2 when it is taken
+//           out of every component's weights, so the posteriors do not change,
+//           while the terms the fp32 accumulator adds (and the logit it
+//           rounds) shrink by about an order of magnitude; the log-likelihood
+//           adds the common part back;
+//  wmax_d   the largest |weight| of the dimension (a maximum has no order).
+// Block 0 also clears the error word and the next kernel's block counter.
+// Bound by the latency of the sums and f64 divisions: about 6 us a launch at
+// K = 256, D = 80, where four kernels in a row took about 17 and their gaps.
+constexpr int kDimsThreads = 256;
+__global__ void __launch_bounds__(kDimsThreads) k_tc_dims(const float *__restrict__ means,
+                                                          const float *__restrict__ covs, int K, int D,
+                                                          float *__restrict__ ctr, float *__restrict__ scale,
+                                                          float *__restrict__ wbar, float *__restrict__ wmax,
+                                                          int *__restrict__ err, unsigned *__restrict__ counter) {
+  extern __shared__ double s_val[];  // K values
+  __shared__ double s_red[kDimsThreads / 32];
+  __shared__ double s_sum;
+  const int d = blockIdx.x, tid = threadIdx.x, lane = tid % 32, w = tid / 32;
+  if (d == 0 && tid == 0) {
+    *err = 0;
+    *counter = 0u;
+  }
+  // The sum of f(k): the values side by side, then one warp's lanes over
+  // k = lane, lane + 32, ... and a butterfly.
+  auto sum = [&](auto f) {
+    for (int k = tid; k < K; k += kDimsThreads) s_val[k] = f(k);
+    __syncthreads();
+    if (w == 0) {
+      double s = 0;
+#pragma unroll 8
+      for (int k = lane; k < K; k += 32) s += s_val[k];
+      s = warp_sum(s);
+      if (lane == 0) s_sum = s;
+    }
+    __syncthreads();
+    return s_sum;
+  };
+  auto largest = [&](double v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax((unsigned *)wmax, __float_as_uint(m));
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (lane == 0) s_red[w] = v;
+    __syncthreads();
+    double m = s_red[0];
+#pragma unroll
+    for (int i = 1; i < kDimsThreads / 32; ++i) m = fmax(m, s_red[i]);
+    __syncthreads();
+    return m;
+  };
+  const float cf = (float)(sum([&](int k) { return (double)means[(i64)k * D + d]; }) / (double)K);
+  const double c = (double)cf;
+  double m = 0;
+  for (int k = tid; k < K; k += kDimsThreads) {
+    const double v = fabs((double)means[(i64)k * D + d] - c) + 4.0 * sqrt((double)covs[(i64)k * D + d]);
+    m = v > m ? v : m;
+  }
+  m = largest(m);
+  int e = 0;
+  if (m > 0) frexp(m, &e);
+  const float sf = (float)ldexp(1.0, -e);
+  const double sc = (double)sf;
+  const float wf = (float)(sum([&](int k) { return tc_weight2(covs, sc, k, d, D); }) / (double)K);
+  float mx = 0.f;
+  for (int k = tid; k < K; k += kDimsThreads) {
+    mx = fmaxf(mx, (float)fabs(tc_weight1(means, covs, c, sc, k, d, D)));
+    mx = fmaxf(mx, (float)fabs(s_val[k] - (double)wf));  // tc_weight2
+  }
+  const float top = (float)largest((double)mx);
+  if (tid == 0) {
+    ctr[d] = cf;
+    scale[d] = sf;
+    wbar[d] = wf;
+    wmax[d] = top;
+  }
 }
+
+// What is left of the preparation, in one launch of blocks with three tasks.
+struct PrepParams {
+  const float *priors, *means, *covs;
+  const float *ctr, *scale, *wbar, *wmax;
+  int K, Kp, D;
+  __half *wimg;
+  float *wsc;
+  double *cst64;
+  float *cst2;
+  double *cbar;
+  unsigned *counter;
+  int nw, nc;  // blocks of the first and second task
+  // Fisher constants (null: none): of the caller's model, dimension Df.
+  const float *fmeans, *fcovs, *fpriors;
+  int Df;
+  double *cmu, *cis2, *cisd, *cup, *cvp;
+};
 
 // W image (hi then lo, fp16), K-major 64-byte-swizzled k-atoms of 32 elements:
 // part p, atom c, row k, element e -> p*wbytes + c*Kp*64 + swizzled(k, e).
-// The entries are divided by 2^g, the power of two that puts max |w| in
+// Atom c holds the weights of x''_d for d = 16c .. 16c+15, then of x''_d^2
+// (less wbar_d) for the same d, so that the producers read each element of x
+// once.  The entries are divided by 2^g, the power of two that puts max |w| in
 // [2^14, 2^15) (fp16 keeps 11 bits per part there); *wsc = 2^g, which the
 // E-step multiplies back onto every logit.
-__global__ void k_tc_wimg(const float *__restrict__ means, const float *__restrict__ covs,
-                          const float *__restrict__ ctr, const float *__restrict__ scale,
-                          const float *__restrict__ wbar, const float *__restrict__ wmax, int K, int Kp,
-                          int D, __half *__restrict__ wimg, float *__restrict__ wsc) {
-  const int KD2 = 2 * D;
-  i64 idx = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void prep_wimg(const PrepParams &p, int block, float mx) {
+  const int KD2 = 2 * p.D;
+  const i64 idx = (i64)block * blockDim.x + threadIdx.x;
   int g = 0;
-  const float mx = *wmax;
   if (mx > 0.f) {
     frexpf(mx, &g);  // mx = m 2^g, m in [0.5, 1)
     g -= 15;
   }
-  if (idx == 0) *wsc = ldexpf(1.f, g);
-  if (idx >= (i64)Kp * KD2) return;
+  if (idx == 0) *p.wsc = ldexpf(1.f, g);
+  if (idx >= (i64)p.Kp * KD2) return;
   const int k = (int)(idx / KD2), e = (int)(idx % KD2);
-  const int c = e / 32, ee = e % 32;
+  const int c = e / 32, ee = e % 32, d = 16 * c + (ee & 15);
   float w = 0.f;
-  if (k < K) w = (float)ldexp(tc_weight(means, covs, ctr, scale, wbar, k, e, D), -g);
+  if (k < p.K) {
+    const double sc = (double)p.scale[d];
+    const double v = ee >= 16 ? tc_weight2(p.covs, sc, k, d, p.D) - (double)p.wbar[d]
+                              : tc_weight1(p.means, p.covs, (double)p.ctr[d], sc, k, d, p.D);
+    w = (float)ldexp(v, -g);
+  }
   const __half hi = __float2half_rn(w);
   const __half lo = __float2half_rn(w - __half2float(hi));
-  const size_t wbytes = (size_t)(KD2 / 32) * Kp * 64;
-  const size_t off = (size_t)c * Kp * 64 + kmajor_sw64_off(k, ee / 8) + (ee % 8) * 2;
-  char *base = (char *)wimg;
+  const size_t wbytes = (size_t)(KD2 / 32) * p.Kp * 64;
+  const size_t off = (size_t)c * p.Kp * 64 + kmajor_sw64_off(k, ee / 8) + (ee % 8) * 2;
+  char *base = (char *)p.wimg;
   *(__half *)(base + off) = hi;
   *(__half *)(base + wbytes + off) = lo;
 }
 
 // c_k = log2(e) * (log pi_k - D/2 log 2pi - 1/2 sum log s2 - 1/2 sum mu'^2/s2)
 // in double, -inf for padding and for priors below 1e-6 (vl/gmm.c:746-747).
-__global__ void k_tc_cst(const float *__restrict__ priors, const float *__restrict__ means,
-                         const float *__restrict__ covs, const float *__restrict__ ctr, int K,
-                         int Kp, int D, double *__restrict__ cst64) {
-  // One warp per component; lanes take dimensions d = lane, lane + 32, ...
-  const int k = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
-  if (k >= Kp) return;
-  if (k >= K || (double)priors[k] < 1e-6) {
-    if (lane == 0) cst64[k] = -INFINITY;
+// One warp per component; lanes take dimensions d = lane, lane + 32, ...
+__device__ __forceinline__ void prep_cst(const PrepParams &p, int block) {
+  const int k = block * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32, D = p.D;
+  if (k >= p.Kp) return;
+  if (k >= p.K || (double)p.priors[k] < 1e-6) {
+    if (lane == 0) p.cst64[k] = -INFINITY;
     return;
   }
   double c = 0;
+#pragma unroll 4
   for (int d = lane; d < D; d += 32) {
-    const double s2 = (double)covs[(i64)k * D + d];
-    const double mup = (double)means[(i64)k * D + d] - (double)ctr[d];
+    const double s2 = (double)p.covs[(i64)k * D + d];
+    const double mup = (double)p.means[(i64)k * D + d] - (double)p.ctr[d];
     c += 0.5 * log(s2) + 0.5 * mup * mup / s2;
   }
-  c = log((double)priors[k]) - 0.5 * (double)D * log(2.0 * 3.141592653589793) - warp_sum(c);
-  if (lane == 0) cst64[k] = c * 1.4426950408889634;
+  c = log((double)p.priors[k]) - 0.5 * (double)D * log(2.0 * 3.141592653589793) - warp_sum(c);
+  if (lane == 0) p.cst64[k] = c * 1.4426950408889634;
 }
 
 // cst2_k = c_k - cbar in float, with cbar the mean of the finite c_k (one
 // warp, fixed-order sums; 0 when every component is skipped).  Like wbar,
 // cbar is common to all components: the posteriors do not see it, the float
 // constants carry less rounding, and the log-likelihood adds it back.
-__global__ void k_tc_cst_center(const double *__restrict__ cst64, int Kp, float *__restrict__ cst2,
-                                double *__restrict__ cbar) {
+__device__ __forceinline__ void prep_center(const PrepParams &p) {
   const int lane = threadIdx.x;
+  const volatile double *cst64 = p.cst64;  // written by other blocks
   double s = 0, n = 0;
-  for (int k = lane; k < Kp; k += 32)
-    if (cst64[k] != -INFINITY) {
-      s += cst64[k];
+  for (int k = lane; k < p.Kp; k += 32) {
+    const double c = cst64[k];
+    if (c != -INFINITY) {
+      s += c;
       n += 1;
     }
+  }
   s = warp_sum(s);
   n = warp_sum(n);
   const double c = n > 0 ? s / n : 0.0;
-  for (int k = lane; k < Kp; k += 32) cst2[k] = cst64[k] == -INFINITY ? -INFINITY : (float)(cst64[k] - c);
-  if (lane == 0) *cbar = c;
+  for (int k = lane; k < p.Kp; k += 32) {
+    const double v = cst64[k];
+    p.cst2[k] = v == -INFINITY ? -INFINITY : (float)(v - c);
+  }
+  if (lane == 0) *p.cbar = c;
 }
 
-// Per-dimension power-of-two scale for fp16 statistics operands, chosen from
-// the model so that x'' = x' * scale is O(1) for data the model describes:
-// scale_d = 2^-ceil(log2(max_k |mu'_kd| + 4 sigma_kd)).
-__global__ void k_tc_scale(const float *__restrict__ means, const float *__restrict__ covs,
-                           const float *__restrict__ ctr, int K, int D, float *__restrict__ scale) {
-  // One warp per dimension; the maximum does not depend on the order.
-  const int d = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
-  if (d >= D) return;
-  double b = 0;
-  for (int k = lane; k < K; k += 32) {
-    const double v = fabs((double)means[(i64)k * D + d] - (double)ctr[d]) + 4.0 * sqrt((double)covs[(i64)k * D + d]);
-    b = v > b ? v : b;
+// Per-component constants of the Fisher finalisation: mu' = mu - m, 1/sigma2,
+// 1/sigma (K x D) and the prefactors 1/sqrt(pi), 1/sqrt(2 pi) (0 for
+// components skipped by vl/fisher.c:436).
+__device__ __forceinline__ void prep_fv(const PrepParams &p, int block) {
+  const i64 e = (i64)block * blockDim.x + threadIdx.x;
+  if (e < (i64)p.K * p.Df) {
+    const int d = (int)(e % p.Df);
+    const double s2 = (double)p.fcovs[e];
+    p.cmu[e] = (double)p.fmeans[e] - (double)p.ctr[d];
+    p.cis2[e] = 1.0 / s2;
+    p.cisd[e] = 1.0 / sqrt(s2);
   }
+  if (e < p.K) {
+    const double pk = (double)p.fpriors[e];
+    p.cup[e] = pk >= 1e-6 ? 1.0 / sqrt(pk) : 0.0;
+    p.cvp[e] = pk >= 1e-6 ? 1.0 / sqrt(2.0 * pk) : 0.0;
+  }
+}
+
+// Blocks [0, nw): the W image; [nw, nw + nc): the components' constants, whose
+// last block to finish centres them; the rest: the Fisher constants.  About 7 us
+// a launch at K = 256, D = 80 (four kernels took about 9 and their gaps).
+__global__ void __launch_bounds__(256) k_tc_prep(const PrepParams p) {
+  const int b = blockIdx.x;
+  if (b < p.nw) {
+    __shared__ float s_mx[8];
+    float mx = 0.f;
+    for (int d = threadIdx.x; d < p.D; d += 256) mx = fmaxf(mx, p.wmax[d]);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-  if (lane != 0) return;
-  int e = 0;
-  if (b > 0) frexp(b, &e);
-  scale[d] = (float)ldexp(1.0, -e);
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (threadIdx.x % 32 == 0) s_mx[threadIdx.x / 32] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, s_mx[i]);
+    prep_wimg(p, b, mx);
+  } else if (b < p.nw + p.nc) {
+    __shared__ bool s_last;
+    prep_cst(p, b - p.nw);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(p.counter, 1u) == (unsigned)p.nc - 1u;
+    __syncthreads();
+    if (s_last && threadIdx.x < 32) {
+      __threadfence();
+      prep_center(p);
+    }
+  } else {
+    prep_fv(p, b - p.nw - p.nc);
+  }
 }
 
 // ============================================================ E-step
@@ -946,11 +1033,14 @@ struct SParams {
 // Operands are fp16: q 2^14 from the E-step's image and x'' = x' * scale.
 // SPLIT 2: both split hi/lo, products hi.hi + hi.lo + lo.hi (fp16x3).
 // SPLIT 1: q single fp16, x'' split hi/lo.
-template <int DIM, int MT, int SPLIT>
+// FS: features per CTA, a multiple of 16 up to 64 (0: all of them).
+template <int DIM, int MT, int SPLIT, int FS>
 struct SLayout {
   static constexpr int NST = 2 * DIM + 16;            // x', x'^2, [1, 0 x 15]
-  static constexpr int NB = (NST + 63) / 64;           // 64-feature MN blocks
-  static constexpr int NCH = (NST + 255) / 256;        // MMA N chunks
+  static constexpr int NF = FS ? FS : NST;             // this CTA's features (the last CTA's may be fewer)
+  static constexpr int NSPLIT = (NST + NF - 1) / NF;   // CTAs over the features
+  static constexpr int NB = (NF + 63) / 64;            // 64-feature MN blocks
+  static constexpr int NCH = (NF + 255) / 256;         // MMA N chunks
   static constexpr int NPA = SPLIT == 2 ? 2 : 1;       // q^T parts
   static constexpr int NPB = 2;                        // [x'', x''^2, 1] parts
   static constexpr int A_PART = MT * 4 * 4 * 512;      // [mnblk 4MT][kgroup 4][512 B atom]
@@ -960,13 +1050,19 @@ struct SLayout {
   static constexpr size_t fixed = 1024 /*ctr*/ + 1024 /*scale*/ + 1024 /*bars*/ + 1024;
   static int max_stages() { return (int)((kSmemLimit - fixed) / kStage); }
   static size_t bytes(int nst) { return fixed + (size_t)nst * kStage; }
-  static_assert(MT * NST <= 512, "accumulators exceed TMEM");
+  static_assert(MT * NF <= 512, "accumulators exceed TMEM");
 };
 
 // Statistics block: converter warps 0-3 and 10-13, epilogue warps 4-7, MMA
 // warp 8, loader warp 9.
 constexpr int kStatsThreads = 448;
 constexpr int kStatsConv = 256;  // converter threads
+// With the features split, the converter warps work in two groups, each on its
+// own stages (stage mod 2, so that a group sees every phase of its stages'
+// barriers): a chunk's conversion is a chain of a wait, shared-memory reads,
+// stores, a proxy fence and an arrival, and the groups run theirs side by side
+// (one item of 3,000 rows, K = 256, D = 80: 75 us with one group, 62 with two).  With all features in one CTA two groups were 3% slower.
+__host__ __device__ constexpr int stats_groups(int fs) { return fs ? 2 : 1; }
 
 // Statistics over work items (runs of rows of one image): for each 32-row
 // chunk, the loader warp bulk-copies the chunk's q^T operand (four 8-row
@@ -974,10 +1070,17 @@ constexpr int kStatsConv = 256;  // converter threads
 // chunk's x rows into a staging buffer; converter warps build the x-side
 // operand [x'', x''^2, 1] (zero rows outside the item); one thread issues the
 // MMAs; the epilogue drains the item's accumulators to its partial.
-template <int DIM, int MT, int SPLIT>
+// FS (features per CTA, blockIdx.z the part): with few items, as for one image,
+// the CTAs of an item's row run split the features too.  Each accumulator sees
+// the same products in the same order (the same bits), and a CTA's chunk takes
+// a quarter of the MMA and conversion time, so that the item's chain of chunks
+// runs at the copies' latency over six stages instead of three.
+template <int DIM, int MT, int SPLIT, int FS>
 __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_constant__ SParams p) {
-  using L = SLayout<DIM, MT, SPLIT>;
+  using L = SLayout<DIM, MT, SPLIT, FS>;
   constexpr int NST = L::NST, NB = L::NB, NPA = L::NPA;
+  const int f0 = FS ? (int)blockIdx.z * FS : 0;     // this CTA's features: [f0, f0 + nf)
+  const int nf = FS ? min(FS, NST - f0) : NST;
   constexpr bool F16 = true;  // fp16 operands: the q image and x'' = x' scale
   constexpr int NF4 = DIM / 4;
   extern __shared__ uint8_t smem_raw[];
@@ -990,11 +1093,12 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
   uint32_t *s_tmem = (uint32_t *)(bars + 56);
   volatile int *s_abort = (volatile int *)(s_tmem + 1);
 
+  constexpr int G = stats_groups(FS), TG = kStatsConv / G;  // converter groups, threads of one
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int comp0 = blockIdx.y * MT * 128;  // first component of this CTA's M tiles
   if (tid == 0) {
     for (int s = 0; s < p.nst; ++s) {
-      mbar_init(&full[s], kStatsConv);
+      mbar_init(&full[s], TG);
       mbar_init(&empty[s], 1);
       mbar_init(&xfull[s], 1);
     }
@@ -1052,13 +1156,15 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
     }
   } else if (warp < 4 || warp >= 10) {
     // ---------------------------------------------------- converters
-    const int ctid = (warp < 4 ? warp : warp - 6) * 32 + lane;
-    int it = 0;
+    const int cw = warp < 4 ? warp : warp - 6;  // converter warp
+    const int ctid = (cw % (8 / G)) * 32 + lane, group = cw / (8 / G);
+    int it = -1;
     bool ok = true;
     for (int ii = ib; ii < ie && ok; ++ii) {
       const SItem item = p.items[p.order[ii]];
       for (i64 cb = p.qbase + ((item.row0 - p.qbase) & ~(i64)7); cb < item.row1; cb += 32) {
-        const int stage = it % p.nst;
+        const int stage = ++it % p.nst;
+        if (G > 1 && stage % G != group) continue;
         if (!mbar_wait(&xfull[stage], (it / p.nst) & 1, s_abort, p.err, 11)) {
           ok = false;
           break;
@@ -1066,50 +1172,87 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
         const uint32_t sa = smem_u32(sS + (size_t)stage * L::kStage);
         const uint32_t sb = sa + NPA * L::A_PART;
         const float *xs = (const float *)(sS + (size_t)stage * L::kStage + NPA * L::A_PART + L::NPB * L::B_PART);
+        if constexpr (FS == 0) {
 #pragma unroll
-        for (int j = 0; j < (32 * NF4 + kStatsConv - 1) / kStatsConv; ++j) {
-          const int i = ctid + kStatsConv * j;
-          if (i >= 32 * NF4) break;
-          const int rs = i / NF4, pp = i % NF4;
-          const i64 row = cb + rs;
-          const bool in = row >= item.row0 && row < item.row1;
-          const int d0 = 4 * pp;
-          float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-          if (in) {
-            const float4 x = *(const float4 *)(xs + rs * DIM + d0);
-            v0 = (x.x - s_ctr[d0]) * s_scl[d0];
-            v1 = (x.y - s_ctr[d0 + 1]) * s_scl[d0 + 1];
-            v2 = (x.z - s_ctr[d0 + 2]) * s_scl[d0 + 2];
-            v3 = (x.w - s_ctr[d0 + 3]) * s_scl[d0 + 3];
+          for (int j = 0; j < (32 * NF4 + TG - 1) / TG; ++j) {
+            const int i = ctid + TG * j;
+            if (i >= 32 * NF4) break;
+            const int rs = i / NF4, pp = i % NF4;
+            const i64 row = cb + rs;
+            const bool in = row >= item.row0 && row < item.row1;
+            const int d0 = 4 * pp;
+            float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
+            if (in) {
+              const float4 x = *(const float4 *)(xs + rs * DIM + d0);
+              v0 = (x.x - s_ctr[d0]) * s_scl[d0];
+              v1 = (x.y - s_ctr[d0 + 1]) * s_scl[d0 + 1];
+              v2 = (x.z - s_ctr[d0 + 2]) * s_scl[d0 + 2];
+              v3 = (x.w - s_ctr[d0 + 3]) * s_scl[d0 + 3];
+            }
+            const int kr = rs & 7, kg = rs >> 3;
+            uint32_t h0, l0, h1, l1;
+            {
+              split2<F16>(clamp_f16(v0), clamp_f16(v1), h0, l0);
+              split2<F16>(clamp_f16(v2), clamp_f16(v3), h1, l1);
+              const int f = d0;
+              const uint32_t off = kg * (NB * 1024) + (f >> 6) * 1024 + mnmajor_sw128_off(kr, (f & 63) >> 3) + ((f >> 2) & 1) * 8;
+              st_shared_v2(sb + off, h0, h1);
+              st_shared_v2(sb + L::B_PART + off, l0, l1);
+            }
+            {
+              split2<F16>(clamp_f16(v0 * v0), clamp_f16(v1 * v1), h0, l0);
+              split2<F16>(clamp_f16(v2 * v2), clamp_f16(v3 * v3), h1, l1);
+              const int f = DIM + d0;
+              const uint32_t off = kg * (NB * 1024) + (f >> 6) * 1024 + mnmajor_sw128_off(kr, (f & 63) >> 3) + ((f >> 2) & 1) * 8;
+              st_shared_v2(sb + off, h0, h1);
+              st_shared_v2(sb + L::B_PART + off, l0, l1);
+            }
+            if (pp == 0) {  // ones column: counts the posterior mass of in-item rows
+              const int f = 2 * DIM;
+              const uint32_t off = kg * (NB * 1024) + (f >> 6) * 1024 + mnmajor_sw128_off(kr, (f & 63) >> 3);
+              const uint16_t one = F16 ? (uint16_t)0x3C00 : (uint16_t)0x3F80;
+              asm volatile("st.shared.u16 [%0], %1;" ::"r"(sb + off), "h"(in ? one : (uint16_t)0) : "memory");
+            }
           }
-          const int kr = rs & 7, kg = rs >> 3;
-          uint32_t h0, l0, h1, l1;
-          {
-            split2<F16>(clamp_f16(v0), clamp_f16(v1), h0, l0);
-            split2<F16>(clamp_f16(v2), clamp_f16(v3), h1, l1);
-            const int f = d0;
-            const uint32_t off = kg * (NB * 1024) + (f >> 6) * 1024 + mnmajor_sw128_off(kr, (f & 63) >> 3) + ((f >> 2) & 1) * 8;
-            st_shared_v2(sb + off, h0, h1);
-            st_shared_v2(sb + L::B_PART + off, l0, l1);
-          }
-          {
-            split2<F16>(clamp_f16(v0 * v0), clamp_f16(v1 * v1), h0, l0);
-            split2<F16>(clamp_f16(v2 * v2), clamp_f16(v3 * v3), h1, l1);
-            const int f = DIM + d0;
-            const uint32_t off = kg * (NB * 1024) + (f >> 6) * 1024 + mnmajor_sw128_off(kr, (f & 63) >> 3) + ((f >> 2) & 1) * 8;
-            st_shared_v2(sb + off, h0, h1);
-            st_shared_v2(sb + L::B_PART + off, l0, l1);
-          }
-          if (pp == 0) {  // ones column: counts the posterior mass of in-item rows
-            const int f = 2 * DIM;
-            const uint32_t off = kg * (NB * 1024) + (f >> 6) * 1024 + mnmajor_sw128_off(kr, (f & 63) >> 3);
-            const uint16_t one = F16 ? (uint16_t)0x3C00 : (uint16_t)0x3F80;
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(sb + off), "h"(in ? one : (uint16_t)0) : "memory");
+        } else {
+          // Quads of features: x'' of four dimensions, their squares, or the
+          // ones column (whose other 15 columns stay zero).
+          const int nq = nf / 4;
+          for (int i = ctid; i < 32 * nq; i += TG) {
+            const int rs = i / nq, f = 4 * (i % nq), ff = f0 + f;
+            const i64 row = cb + rs;
+            const bool in = row >= item.row0 && row < item.row1;
+            const int kr = rs & 7, kg = rs >> 3;
+            const uint32_t off = kg * (NB * 1024) + mnmajor_sw128_off(kr, f >> 3) + ((f >> 2) & 1) * 8;
+            if (ff < 2 * DIM) {
+              const bool sq = ff >= DIM;
+              const int d0 = sq ? ff - DIM : ff;
+              float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
+              if (in) {
+                const float4 x = *(const float4 *)(xs + rs * DIM + d0);
+                v0 = (x.x - s_ctr[d0]) * s_scl[d0];
+                v1 = (x.y - s_ctr[d0 + 1]) * s_scl[d0 + 1];
+                v2 = (x.z - s_ctr[d0 + 2]) * s_scl[d0 + 2];
+                v3 = (x.w - s_ctr[d0 + 3]) * s_scl[d0 + 3];
+              }
+              if (sq) {
+                v0 *= v0;
+                v1 *= v1;
+                v2 *= v2;
+                v3 *= v3;
+              }
+              uint32_t h0, l0, h1, l1;
+              split2<F16>(clamp_f16(v0), clamp_f16(v1), h0, l0);
+              split2<F16>(clamp_f16(v2), clamp_f16(v3), h1, l1);
+              st_shared_v2(sb + off, h0, h1);
+              st_shared_v2(sb + L::B_PART + off, l0, l1);
+            } else if (ff == 2 * DIM) {
+              asm volatile("st.shared.u16 [%0], %1;" ::"r"(sb + off), "h"(in ? (uint16_t)0x3C00 : (uint16_t)0) : "memory");
+            }
           }
         }
         fence_proxy_async_smem();
         mbar_arrive(&full[stage]);
-        ++it;
       }
     }
   } else if (warp < 8) {
@@ -1123,15 +1266,15 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
 #pragma unroll 1
       for (int mt = 0; mt < MT; ++mt) {
         const int comp = comp0 + mt * 128 + ew * 32 + lane;
-        float *dst = p.partial + ((size_t)item.slot * p.Kp + comp) * NST;
-        const uint32_t tb = tmem + ((uint32_t)(ew * 32) << 16) + (uint32_t)(mt * NST);
+        float *dst = p.partial + ((size_t)item.slot * p.Kp + comp) * NST + f0;
+        const uint32_t tb = tmem + ((uint32_t)(ew * 32) << 16) + (uint32_t)(mt * L::NF);
 #pragma unroll 1
-        for (int cc = 0; cc < (NST + 31) / 32; ++cc) {
+        for (int cc = 0; cc < (nf + 31) / 32; ++cc) {
           uint32_t v[32];
           tmem_ld32(tb + cc * 32, v);
           tmem_wait_ld();
           if (comp < p.Kp) {
-            if (cc * 32 + 32 <= NST) {
+            if (cc * 32 + 32 <= nf) {
 #pragma unroll
               for (int j = 0; j < 32; j += 4)
                 *(float4 *)(dst + cc * 32 + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
@@ -1139,7 +1282,7 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
             } else {
 #pragma unroll
               for (int j = 0; j < 32; ++j)
-                if (cc * 32 + j < NST) dst[cc * 32 + j] = __uint_as_float(v[j]);
+                if (cc * 32 + j < nf) dst[cc * 32 + j] = __uint_as_float(v[j]);
             }
           }
         }
@@ -1176,12 +1319,12 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
             const uint64_t ah = sdesc(a0, 2048, 512, kSw64);
 #pragma unroll
             for (int nc = 0; nc < L::NCH; ++nc) {
-              const int nn = (NST - nc * 256) < 256 ? (NST - nc * 256) : 256;
+              const int nn = FS ? nf : (NST - nc * 256) < 256 ? (NST - nc * 256) : 256;
               const uint32_t idesc = F16 ? idesc_f16(128, nn, true, true) : idesc_bf16(128, nn, true, true);
               const uint32_t b0 = sb + ks * 2 * (NB * 1024) + nc * 4 * 1024;
               const uint64_t bh = sdesc(b0, 1024, NB * 1024, kSw128);
               const uint64_t bl = sdesc(b0 + L::B_PART, 1024, NB * 1024, kSw128);
-              const uint32_t d = tmem + (uint32_t)(mt * NST + nc * 256);
+              const uint32_t d = tmem + (uint32_t)(mt * L::NF + nc * 256);
               mma_bf16(d, ah, bh, idesc, (chunk > 0 || ks > 0) ? 1u : 0u);
               mma_bf16(d, ah, bl, idesc, 1u);
               if (NPA == 2) mma_bf16(d, sdesc(a0 + L::A_PART, 2048, 512, kSw64), bh, idesc, 1u);
@@ -1203,52 +1346,31 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
 }
 
 // ======================================================= finalize (FV)
-// Per-component constants of the Fisher finalisation, computed once per call:
-// mu' = mu - m, 1/sigma2, 1/sigma (K x D) and the prefactors 1/sqrt(pi),
-// 1/sqrt(2 pi) (0 for components skipped by vl/fisher.c:436).
-__global__ void k_tc_fv_consts(const float *__restrict__ means, const float *__restrict__ covs,
-                               const float *__restrict__ priors, const float *__restrict__ ctr, int K,
-                               int D, double *__restrict__ cmu, double *__restrict__ cis2,
-                               double *__restrict__ cisd, double *__restrict__ cup,
-                               double *__restrict__ cvp) {
-  const i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < (i64)K * D) {
-    const int d = (int)(e % D);
-    const double s2 = (double)covs[e];
-    cmu[e] = (double)means[e] - (double)ctr[d];
-    cis2[e] = 1.0 / s2;
-    cisd[e] = 1.0 / sqrt(s2);
-  }
-  if (e < K) {
-    const double pk = (double)priors[e];
-    cup[e] = pk >= 1e-6 ? 1.0 / sqrt(pk) : 0.0;
-    cvp[e] = pk >= 1e-6 ? 1.0 / sqrt(2.0 * pk) : 0.0;
-  }
-}
-
 // Per image: reduce the item partials in double and form the Fisher vector
 // (vl/fisher.c:419-485) from S0 = sum q, S1 = sum q x', S2 = sum q x'^2:
 //   u = (S1 - mu' S0) / sigma,  v = (S2 - 2 mu' S1 + mu'^2 S0) / sigma2 - S0,
 // scaled by 1/(N sqrt pi) and 1/(N sqrt(2 pi)); signed sqrt; L2.
-// One cluster of kFinCluster CTAs per image: CTA r forms the outputs of
+// One cluster of NC CTAs of NT threads per image: CTA r forms the outputs of
 // components [r K/C, (r+1) K/C) in shared memory (2 (K/C) DIM floats), the
 // CTAs exchange their partial L2 norms and term counts through distributed
 // shared memory (summed in rank order on every CTA, so every CTA scales by
 // the same bits), and each writes its normalised part once, coalesced.
-constexpr int kFinThreads = 256;
-constexpr int kFinCluster = 4;  // divides K (a multiple of 8 on this path)
+// 256 threads and 4 CTAs when there are images enough to fill the chip (4,096
+// images of K = 256, D = 80: 1.09 ms; 8 CTAs of 1,024 threads: 2.43); for a few
+// images 1,024 threads and 8 CTAs, since each CTA is one chain of loads and f64
+// operations over its components (one image in 12 items: 12 us; 68 the other way).
 
 // DIM: the dimension the statistics were taken in; Dr <= DIM: the model's own
 // dimension (dimensions past it are zero padding, left out of the vector).
-template <int DIM>
-__global__ void __cluster_dims__(kFinCluster, 1, 1) __launch_bounds__(kFinThreads) k_tc_fv_finalize(
+template <int DIM, int NT, int NC>
+__global__ void __launch_bounds__(NT) k_tc_fv_finalize(
     int K, int Kp, int Dr, const float *__restrict__ partial, const int *__restrict__ imgSlot0,
     const i64 *__restrict__ imgRow0, const double *__restrict__ cmu, const double *__restrict__ cis2,
     const double *__restrict__ cisd, const double *__restrict__ cup, const double *__restrict__ cvp,
     const float *__restrict__ scale, const unsigned *__restrict__ rowcnt, i64 rowcntBase, int flags,
     i64 imgBase, float *__restrict__ enc, unsigned long long *__restrict__ nterms) {
   constexpr int NST = 2 * DIM + 16;
-  constexpr int NW = kFinThreads / 32;
+  constexpr int NW = NT / 32;
   extern __shared__ float s_fv[];  // 2 E: this CTA's u values, then its v values
   __shared__ double s_sq[NW];
   __shared__ unsigned long long s_nt[NW];
@@ -1257,16 +1379,16 @@ __global__ void __cluster_dims__(kFinCluster, 1, 1) __launch_bounds__(kFinThread
   __shared__ unsigned long long s_partn;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
-  const int img = blockIdx.x / kFinCluster;
+  const int img = blockIdx.x / NC;
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int Kc = K / kFinCluster, k0 = rank * Kc;
+  const int Kc = K / NC, k0 = rank * Kc;
   const int E = Kc * Dr, KD = K * Dr, eBase = k0 * Dr;
   const int s0 = imgSlot0[img], s1 = imgSlot0[img + 1];
   const i64 r0 = imgRow0[img], r1 = imgRow0[img + 1];
   const i64 n = r1 - r0;
   const double in = n > 0 ? 1.0 / (double)n : 0.0;
   const size_t slotStride = (size_t)Kp * NST;
-  for (int d = tid; d < DIM; d += kFinThreads) s_is[d] = scale ? 1.0 / (double)scale[d] : 1.0;
+  for (int d = tid; d < DIM; d += NT) s_is[d] = scale ? 1.0 / (double)scale[d] : 1.0;
   const double iq = 1.0 / (double)kQScale;
   __syncthreads();
   // Element (component kl, dimension d) is el = kl Dr + d.  Warp w takes the
@@ -1319,7 +1441,7 @@ __global__ void __cluster_dims__(kFinCluster, 1, 1) __launch_bounds__(kFinThread
   unsigned long long nt = 0;
   if (rowcnt)
 #pragma unroll 4
-    for (i64 r = r0 + rank * kFinThreads + tid; r < r1; r += kFinThreads * kFinCluster)
+    for (i64 r = r0 + rank * NT + tid; r < r1; r += NT * NC)
       nt += rowcnt[r - rowcntBase];
   sq = warp_sum(sq);
 #pragma unroll
@@ -1343,7 +1465,7 @@ __global__ void __cluster_dims__(kFinCluster, 1, 1) __launch_bounds__(kFinThread
   if (tid == 0) {
     double t = 0;
     unsigned long long c = 0;
-    for (int q = 0; q < kFinCluster; ++q) {
+    for (int q = 0; q < NC; ++q) {
       t += *cluster.map_shared_rank(&s_part, q);
       c += *cluster.map_shared_rank(&s_partn, q);
     }
@@ -1361,7 +1483,7 @@ __global__ void __cluster_dims__(kFinCluster, 1, 1) __launch_bounds__(kFinThread
   }
   // Both halves in 16-byte pieces where E and the output allow it.
   if (E % 4 == 0 && (((uintptr_t)out | (uintptr_t)(out + KD)) & 15) == 0) {
-    for (int el = 4 * tid; el < E; el += 4 * kFinThreads) {
+    for (int el = 4 * tid; el < E; el += 4 * NT) {
       float4 a = *(const float4 *)(s_fv + el), b = *(const float4 *)(s_fv + E + el);
       if (nrmz) {
         a = make_float4(a.x / nf, a.y / nf, a.z / nf, a.w / nf);
@@ -1371,7 +1493,7 @@ __global__ void __cluster_dims__(kFinCluster, 1, 1) __launch_bounds__(kFinThread
       *(float4 *)(out + KD + el) = b;
     }
   } else {
-    for (int el = tid; el < E; el += kFinThreads) {
+    for (int el = tid; el < E; el += NT) {
       out[el] = nrmz ? s_fv[el] / nf : s_fv[el];
       out[KD + el] = nrmz ? s_fv[E + el] / nf : s_fv[E + el];
     }
@@ -1533,10 +1655,16 @@ int padK(i64 K) {
 }
 int kblocks(int Kp) { return (Kp + 255) / 256; }
 
+// Fisher constants that tc_prepare fills on request (device arrays).
+struct FvConsts {
+  const DevModel<float> *m = nullptr;  // the caller's model
+  double *cmu, *cis2, *cisd, *cup, *cvp;
+};
+
 // Model-derived operands of the tensor-core path: the centre, the
 // per-dimension scales, the fp16 W image with its scale, and the constants.
-void tc_prepare(const DevModel<float> &m, TcPrep &tp, bool want_scale, Scratch &sc, cudaStream_t s) {
-  (void)want_scale;  // the E-step's operands are always scaled
+// Also clears the arena's error word (slot 3).
+void tc_prepare(const DevModel<float> &m, TcPrep &tp, Scratch &sc, cudaStream_t s, const FvConsts *fv = nullptr) {
   tp.K = (int)m.K;
   tp.Kp = padK(m.K);
   tp.D = (int)m.D;
@@ -1544,29 +1672,31 @@ void tc_prepare(const DevModel<float> &m, TcPrep &tp, bool want_scale, Scratch &
   tp.ctr = sc.slot[0].get<float>(256);
   tp.cst2 = sc.slot[1].get<float>(std::max(256, tp.Kp));
   tp.wimg = sc.slot[2].get<__half>((size_t)2 * tp.Kp * KD2);
+  int *err = sc.slot[3].get<int>(1);
   tp.scale = sc.slot[12].get<float>(256);
-  float *wm = sc.slot[19].get<float>(2);
-  tp.wsc = wm + 1;
+  float *wm = sc.slot[19].get<float>(260);  // 256 maxima, the W scale, a block counter
+  tp.wsc = wm + 256;
   tp.wbar = sc.slot[20].get<float>(256);
   double *c64 = sc.slot[21].get<double>((size_t)std::max(256, tp.Kp) + 1);
   tp.cbar = c64 + std::max(256, tp.Kp);
-  VLB_LAUNCH("tc_center", s, k_tc_center<<<(tp.D + 7) / 8, 256, 0, s>>>(m.means, tp.K, tp.D, tp.ctr));
-  VLB_LAUNCH("tc_scale", s,
-             k_tc_scale<<<(tp.D + 7) / 8, 256, 0, s>>>(m.means, m.covs, tp.ctr, tp.K, tp.D, tp.scale));
-  VLB_LAUNCH("tc_wbar", s, k_tc_wbar<<<(tp.D + 7) / 8, 256, 0, s>>>(m.covs, tp.scale, tp.K, tp.D, tp.wbar));
-  VLB_CUDA(cudaMemsetAsync(wm, 0, sizeof(float), s));
-  const i64 nw = (i64)tp.K * KD2;
-  VLB_LAUNCH("tc_wmax", s,
-             k_tc_wmax<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(m.means, m.covs, tp.ctr, tp.scale, tp.wbar,
-                                                                    tp.K, tp.D, wm));
-  const i64 n = (i64)tp.Kp * KD2;
-  VLB_LAUNCH("tc_wimage", s,
-             k_tc_wimg<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(m.means, m.covs, tp.ctr, tp.scale, tp.wbar,
-                                                                  wm, tp.K, tp.Kp, tp.D, tp.wimg, tp.wsc));
-  VLB_LAUNCH("tc_constants", s,
-             k_tc_cst<<<(tp.Kp + 7) / 8, 256, 0, s>>>(m.priors, m.means, m.covs, tp.ctr, tp.K,
-                                                          tp.Kp, tp.D, c64));
-  VLB_LAUNCH("tc_constants_center", s, k_tc_cst_center<<<1, 32, 0, s>>>(c64, tp.Kp, tp.cst2, tp.cbar));
+  unsigned *counter = (unsigned *)(wm + 257);
+  VLB_LAUNCH("tc_dims", s,
+             k_tc_dims<<<tp.D, kDimsThreads, sizeof(double) * tp.K, s>>>(m.means, m.covs, tp.K, tp.D, tp.ctr, tp.scale, tp.wbar, wm, err, counter));
+  PrepParams p{};
+  p.priors = m.priors; p.means = m.means; p.covs = m.covs;
+  p.ctr = tp.ctr; p.scale = tp.scale; p.wbar = tp.wbar; p.wmax = wm;
+  p.K = tp.K; p.Kp = tp.Kp; p.D = tp.D;
+  p.wimg = tp.wimg; p.wsc = tp.wsc; p.cst64 = c64; p.cst2 = tp.cst2; p.cbar = tp.cbar; p.counter = counter;
+  p.nw = (tp.Kp * KD2 + 255) / 256;
+  p.nc = (tp.Kp + 7) / 8;
+  int nf = 0;
+  if (fv) {
+    p.fmeans = fv->m->means; p.fcovs = fv->m->covs; p.fpriors = fv->m->priors;
+    p.Df = (int)fv->m->D;
+    p.cmu = fv->cmu; p.cis2 = fv->cis2; p.cisd = fv->cisd; p.cup = fv->cup; p.cvp = fv->cvp;
+    nf = (tp.K * p.Df + 255) / 256;
+  }
+  VLB_LAUNCH("tc_prep", s, k_tc_prep<<<p.nw + p.nc + nf, 256, 0, s>>>(p));
 }
 
 int padQ(int Kp) { return (Kp + 127) / 128 * 128; }
@@ -1678,14 +1808,15 @@ i64 launch_estep(const float *X, i64 N, const TcPrep &tp, void *q, int ldq, bool
   return launch_estep_impl<DIM, QF, true, false>(X, N, tp, q, ldq, fast, rowcnt, ll_part, err, nst_req, s, eo);
 }
 
-template <int DIM, int MT, int SPLIT>
+template <int DIM, int MT, int SPLIT, int FS = 0>
 void launch_stats(const SParams &p0, int grid_x, int grid_y, int nst_req, cudaStream_t s) {
-  using L = SLayout<DIM, MT, SPLIT>;
+  using L = SLayout<DIM, MT, SPLIT, FS>;
   SParams p = p0;
   p.nst = std::min(nst_req > 0 ? nst_req : 8, L::max_stages());
+  p.nst -= p.nst % stats_groups(FS);
   VLB_CHECK(p.nst >= 2, VL_ERR_BAD_ARG, "tensor-core statistics: operands exceed shared memory");
   const size_t smem = L::bytes(p.nst);
-  auto kern = k_tc_stats<DIM, MT, SPLIT>;
+  auto kern = k_tc_stats<DIM, MT, SPLIT, FS>;
   VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   {
     // The image (parts of ngroups 8-row groups per 32-component block) for
@@ -1699,8 +1830,10 @@ void launch_stats(const SParams &p0, int grid_x, int grid_y, int nst_req, cudaSt
     tc::tma_map(&p.qmap, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, p.qimg, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
   }
   VLB_LAUNCH(SPLIT == 2 ? "tc_stats_f16x3" : "tc_stats_f16x2", s,
-             kern<<<dim3(grid_x, grid_y), kStatsThreads, smem, s>>>(p));
+             kern<<<dim3(grid_x, grid_y, L::NSPLIT), kStatsThreads, smem, s>>>(p));
 }
+
+constexpr int kStatsFeat = 48;  // features per CTA when they are split
 
 template <int DIM>
 struct Tc {
@@ -1719,6 +1852,15 @@ struct Tc {
   // mt: 128-component M tiles per CTA (0: two when they fit in TMEM).
   static void stats(int split, const SParams &p, int grid_x, int mt, int nst, cudaStream_t s) {
     const int mtiles = p.Kq / 128;
+    // Few items: one M tile and kStatsFeat features per CTA while those CTAs
+    // still all run at once (3,000 rows in one item, K = 256, D = 80: 98 us with
+    // two M tiles and all features in a CTA, 62 split).
+    constexpr int kFeat = kStatsFeat;
+    if (mt == 0 && grid_x * mtiles * SLayout<DIM, 1, 2, kFeat>::NSPLIT <= num_sms()) {
+      if (split == 1) launch_stats<DIM, 1, 1, kFeat>(p, grid_x, mtiles, nst, s);
+      else launch_stats<DIM, 1, 2, kFeat>(p, grid_x, mtiles, nst, s);
+      return;
+    }
     if (kTwo && mtiles % 2 == 0 && mt != 1) {
       if (split == 1) launch_stats<DIM, (kTwo ? 2 : 1), 1>(p, grid_x, mtiles / 2, nst, s);
       else launch_stats<DIM, (kTwo ? 2 : 1), 2>(p, grid_x, mtiles / 2, nst, s);
@@ -1835,8 +1977,7 @@ bool tc_supported_padded(i64 K, i64 D) { return tc_pad_dim(D) > 0 && tc_supporte
 
 bool tc_fv_supported_padded(i64 K, i64 D) {
   const int Dp = tc_pad_dim(D);
-  return Dp > 0 && tc_supported(K, Dp) && K % kFinCluster == 0 &&
-         sizeof(float) * 2 * (size_t)(K / kFinCluster) * D <= (size_t)kSmemLimit;
+  return Dp > 0 && tc_supported(K, Dp) && K % 4 == 0 && sizeof(float) * 2 * (size_t)(K / 4) * D <= (size_t)kSmemLimit;
 }
 
 // Zero-padded copies of rows and model in `sc` (slots 22-24).
@@ -1862,9 +2003,9 @@ Padded pad_inputs(const float *X, i64 N, const DevModel<float> &m, Scratch &sc, 
 }
 
 bool tc_fv_supported(i64 K, i64 D) {
-  // The finalize keeps 2 (K / kFinCluster) D floats per CTA in shared memory.
-  return tc_supported(K, D) && K % kFinCluster == 0 &&
-         sizeof(float) * 2 * (size_t)(K / kFinCluster) * D <= (size_t)kSmemLimit;
+  // A quarter of the vector within a CTA's shared memory: larger ones take the
+  // exact path.
+  return tc_supported(K, D) && K % 4 == 0 && sizeof(float) * 2 * (size_t)(K / 4) * D <= (size_t)kSmemLimit;
 }
 
 i64 tc_estep(const float *X, i64 N, const DevModel<float> &m, float *q, double *ll_part, bool fast,
@@ -1884,9 +2025,8 @@ i64 tc_estep(const float *X, i64 N, const DevModel<float> &m, float *q, double *
     return n + 1;
   }
   TcPrep tp;
-  tc_prepare(m, tp, false, sc, s);
+  tc_prepare(m, tp, sc, s);
   int *err = sc.slot[3].get<int>(1);
-  VLB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   const i64 n = estep_dispatch(tp.D, kQRow, X, N, tp, (void *)q, (int)m.K, fast, nullptr, ll_part, err, 0, s);
   check_err(err, s);
   return n;
@@ -1906,14 +2046,13 @@ i64 tc_estep_em(const float *X, i64 N, const DevModel<float> &m, float *q, doubl
   Scratch &sc = thread_scratch(kArenaTc);
   const bool fp32 = (precision == VLB200_PREC_FP32);
   TcPrep tp;
-  tc_prepare(m, tp, !fp32, sc, s);
+  tc_prepare(m, tp, sc, s);
   const int Kq = padQ(tp.Kp);
   const i64 ntiles = (N + 127) / 128;
   EOut eo;
   eo.qimg = sc.slot[4].get<char>((size_t)std::max<i64>(1, ntiles) * 128 * Kq * (fp32 ? 4 : 2));
   eo.qthr = 1e-2 / (double)m.K;  // vl/gmm.c:1099
   int *err = sc.slot[3].get<int>(1);
-  VLB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   const i64 n = estep_dispatch(tp.D, fp32 ? kQRowImg32 : kQRowImg16, X, N, tp, (void *)q, (int)m.K, false,
                                nullptr, ll_part, err, 0, s, eo);
   check_err(err, s);
@@ -1962,7 +2101,7 @@ void tc_mstep(const float *X, i64 N, float *means, float *covs, float *priors, i
 void tc_em_image_from_rows(const float *qrows, i64 n, const DevModel<float> &m, cudaStream_t s) {
   Scratch &sc = thread_scratch(kArenaTc);
   TcPrep tp;
-  tc_prepare(m, tp, true, sc, s);
+  tc_prepare(m, tp, sc, s);
   const int Kq = padQ(tp.Kp);
   const i64 ntiles = (n + 127) / 128, rowsPad = ntiles * 128;
   __half *img = sc.slot[4].get<__half>((size_t)std::max<i64>(1, ntiles) * 128 * Kq);
@@ -2057,8 +2196,29 @@ i64 default_row_budget(int Kp, bool fp32) {
   return std::max<i64>(1 << 16, (i64)(4ull << 30) / (Kp * qsz));
 }
 
-void fv_layout(const i64 *off, i64 numImages, i64 rowBudget, i64 itemRows, int nsm, FvLayout &L) {
+// Rows per work item: itemRows, except that a batch of up to kSmallRows rows
+// (one image, or a few small ones) is cut into the shortest items (multiples
+// of 128 rows) whose CTAs (M tiles times feature parts) all run at once: an
+// item is one chain of dependent MMAs, about 0.6 us per 32 rows however few
+// features and components a CTA has (3,000 rows in 12 items: 12 us, in one: 62).  Shorter fp32 chains are also closer to
+// FP64 (one image of 3,000 rows, D = 80, K = 256, plain vector: 6.6e-6 with
+// one item, 1.6e-6 with 12; longer images keep their items, so that their
+// vectors stay within a few 1e-6 of what they were).
+constexpr i64 kSmallRows = 4096;
+i64 fv_item_rows(const i64 *off, i64 numImages, i64 itemRows, int Kp, i64 D, int nsm) {
+  if (off[numImages] - off[0] > kSmallRows) return itemRows;
+  const i64 per = (i64)(padQ(Kp) / 128) * ((2 * D + 16 + kStatsFeat - 1) / kStatsFeat);
+  for (i64 r = 256; r < itemRows; r *= 2) {
+    i64 items = 0;
+    for (i64 j = 0; j < numImages; ++j) items += (off[j + 1] - off[j] + r - 1) / r;
+    if (items * per <= nsm) return r;
+  }
+  return itemRows;
+}
+
+void fv_layout(const i64 *off, i64 numImages, i64 rowBudget, i64 itemRows, int Kp, i64 D, int nsm, FvLayout &L) {
   L = FvLayout();
+  itemRows = fv_item_rows(off, numImages, itemRows, Kp, D, nsm);
   i64 img = 0;
   while (img < numImages) {
     FvChunk c;
@@ -2109,6 +2269,37 @@ void fv_upload(const FvLayout &L, int Kp, int Kq, int NST, bool fp32, Scratch &s
   upload(sc.slot[11], L.row0, s);
 }
 
+template <int DIM, int NT, int NC, typename... Args>
+void launch_fv_finalize_as(i64 nimg, i64 K, i64 Dr, cudaStream_t s, Args... args) {
+  auto kern = k_tc_fv_finalize<DIM, NT, NC>;
+  const size_t smem = sizeof(float) * 2 * (size_t)(K / NC) * Dr;
+  VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = NC;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(nimg * NC));
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  VLB_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+template <typename... Args>
+void launch_fv_finalize(int D, i64 nimg, cudaStream_t s, int K, int Kp, int Dr, Args... args) {
+  const bool few = nimg * 8 <= num_sms() && K % 8 == 0;
+  auto go = [&](auto dim) {
+    constexpr int DIM = decltype(dim)::value;
+    if (few) launch_fv_finalize_as<DIM, 1024, 8>(nimg, K, Dr, s, K, Kp, Dr, args...);
+    else launch_fv_finalize_as<DIM, 256, 4>(nimg, K, Dr, s, K, Kp, Dr, args...);
+  };
+  if (D == 64) go(std::integral_constant<int, 64>());
+  else if (D == 80) go(std::integral_constant<int, 80>());
+  else go(std::integral_constant<int, 128>());
+}
+
 // Called with a chunk's index before its launches and after its finalize.
 using ChunkHook = std::function<void(size_t)>;
 
@@ -2122,21 +2313,18 @@ void fv_run(const FvLayout &L, Scratch &sc, const float *X, const DevModel<float
             const DevModel<float> *mreal = nullptr) {
   const bool fp32 = (precision == VLB200_PREC_FP32);
   TcPrep tp;
-  tc_prepare(m, tp, !fp32, sc, s);
   const int qf = fp32 ? kQImg32 : kQImg16;
   const int split = fp32 ? 2 : 1;
-  const int Kq = padQ(tp.Kp);
   const i64 K = m.K, D = m.D;
-  int *err = sc.slot[3].get<int>(1);
-  VLB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   double *cmu = sc.slot[13].get<double>(K * D), *cis2 = sc.slot[14].get<double>(K * D);
   double *cisd = sc.slot[15].get<double>(K * D), *cup = sc.slot[16].get<double>(K);
   double *cvp = sc.slot[17].get<double>(K);
   const DevModel<float> &mr = mreal ? *mreal : m;
   const i64 Dr = mr.D;
-  VLB_LAUNCH("tc_fv_consts", s,
-             k_tc_fv_consts<<<(unsigned)((K * Dr + 255) / 256), 256, 0, s>>>(
-                 mr.means, mr.covs, mr.priors, tp.ctr, (int)K, (int)Dr, cmu, cis2, cisd, cup, cvp));
+  const FvConsts fc{&mr, cmu, cis2, cisd, cup, cvp};
+  tc_prepare(m, tp, sc, s, &fc);
+  const int Kq = padQ(tp.Kp);
+  int *err = sc.slot[3].get<int>(1);
   void *q = sc.slot[4].p;
   unsigned *rowcnt = (unsigned *)sc.slot[5].p;
   float *partial = (float *)sc.slot[6].p;
@@ -2144,9 +2332,6 @@ void fv_run(const FvLayout &L, Scratch &sc, const float *X, const DevModel<float
   const int *dorder = (const int *)sc.slot[8].p, *dbeg = (const int *)sc.slot[9].p;
   const int *dslot0 = (const int *)sc.slot[10].p;
   const i64 *drow0 = (const i64 *)sc.slot[11].p;
-  auto fin = D == 64 ? k_tc_fv_finalize<64> : D == 80 ? k_tc_fv_finalize<80> : k_tc_fv_finalize<128>;
-  const size_t finSmem = sizeof(float) * 2 * (K / kFinCluster) * Dr;
-  VLB_CUDA(cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)finSmem));
   for (size_t ci = 0; ci < L.chunks.size(); ++ci) {
     const FvChunk &c = L.chunks[ci];
     if (before) before(ci);
@@ -2173,10 +2358,9 @@ void fv_run(const FvLayout &L, Scratch &sc, const float *X, const DevModel<float
       stats_dispatch(tp.D, split, sp, c.gx, cfg.statsMT, cfg.statsStages, s);
     }
     VLB_LAUNCH("tc_fv_finalize", s,
-               fin<<<(unsigned)(c.nimg * kFinCluster), kFinThreads, finSmem, s>>>(
-                   (int)K, tp.Kp, (int)Dr, partial, dslot0 + c.img, drow0 + c.img, cmu, cis2, cisd, cup, cvp,
-                   tp.scale, c.nrows > 0 ? rowcnt : nullptr, c.row0, flags, c.img0, enc,
-                   nterms));
+               launch_fv_finalize((int)D, c.nimg, s, (int)K, tp.Kp, (int)Dr, (const float *)partial, dslot0 + c.img,
+                                  drow0 + c.img, cmu, cis2, cisd, cup, cvp, tp.scale,
+                                  c.nrows > 0 ? rowcnt : nullptr, c.row0, flags, c.img0, enc, nterms));
     if (after) after(ci);
   }
 }
@@ -2190,13 +2374,13 @@ void tc_fisher_batch(const float *X, const i64 *h_offsets, i64 numImages, const 
   const int Kp = padK(m.K);
   TcFvConfig cfg;
   FvLayout L;
-  fv_layout(h_offsets, numImages, default_row_budget(Kp, fp32), cfg.itemRows, num_sms(), L);
+  fv_layout(h_offsets, numImages, default_row_budget(Kp, fp32), cfg.itemRows, Kp, tc_pad_dim(m.D), num_sms(), L);
   if (!tc_fv_supported(m.K, m.D)) {
     const i64 N = h_offsets[numImages] - h_offsets[0];
     const Padded P = pad_inputs(X + h_offsets[0] * m.D, N, m, sc, s);
     std::vector<i64> offs(h_offsets, h_offsets + numImages + 1);
     for (auto &o : offs) o -= h_offsets[0];
-    fv_layout(offs.data(), numImages, default_row_budget(Kp, fp32), cfg.itemRows, num_sms(), L);
+    fv_layout(offs.data(), numImages, default_row_budget(Kp, fp32), cfg.itemRows, Kp, P.m.D, num_sms(), L);
     fv_upload(L, Kp, padQ(Kp), (int)(2 * P.m.D + 16), fp32, sc, s);
     fv_run(L, sc, P.X, P.m, enc, nterms, flags, precision, cfg, s, nullptr, nullptr, &m);
     check_err((int *)sc.slot[3].p, s);
@@ -2248,7 +2432,7 @@ namespace {
 void plan_build(TcFvPlan &p, cudaStream_t s) {
   const bool fp32 = (p.precision == VLB200_PREC_FP32);
   const i64 budget = p.cfg.rowBudget > 0 ? p.cfg.rowBudget : default_row_budget(p.Kp, fp32);
-  fv_layout(p.offsets.data(), p.numImages, budget, p.cfg.itemRows, num_sms(), p.layout);
+  fv_layout(p.offsets.data(), p.numImages, budget, p.cfg.itemRows, p.Kp, p.D, num_sms(), p.layout);
   fv_upload(p.layout, p.Kp, padQ(p.Kp), (int)(2 * p.D + 16), fp32, p.sc, s);
   VLB_CUDA(cudaStreamSynchronize(s));
 }
@@ -2304,7 +2488,7 @@ void tc_fv_plan_run_host(TcFvPlan *p, const DevModel<float> &m, const float *Xh,
   const i64 D = p->D, FV = 2 * p->K * p->D;
   if (!p->pipeBuilt) {
     const i64 budget = std::max<i64>(1, (total + TcFvPlan::kPipeChunks - 1) / TcFvPlan::kPipeChunks);
-    fv_layout(p->offsets.data(), p->numImages, budget, p->cfg.itemRows, num_sms(), p->pipe);
+    fv_layout(p->offsets.data(), p->numImages, budget, p->cfg.itemRows, p->Kp, p->D, num_sms(), p->pipe);
     fv_upload(p->pipe, p->Kp, padQ(p->Kp), (int)(2 * p->D + 16), fp32, p->scPipe, s);
     if (!p->h2d) VLB_CUDA(cudaStreamCreateWithFlags(&p->h2d, cudaStreamNonBlocking));
     if (!p->d2h) VLB_CUDA(cudaStreamCreateWithFlags(&p->d2h, cudaStreamNonBlocking));
