@@ -196,14 +196,16 @@ bool tc_fv_supported_padded(i64 K, i64 D);
 i64 tc_estep(const float *X, i64 N, const DevModel<float> &m, float *q, double *ll_part,
              bool fast, int precision, cudaStream_t s, Scratch *arena = nullptr);
 // EM with the tensor-core M-step.  tc_estep_em is the E-step of tc_estep that
-// also writes the posteriors as the statistics operand image, thresholded at
-// the M-step's skip (vl/gmm.c:1099); tc_mstep then runs the M-step
-// (vl/gmm.c:1036-1213) from that image and the centre of that E-step's model,
-// on the same thread, in place on means/covs/priors (device, fp32).
+// writes the posteriors as the statistics operand image, thresholded at the
+// M-step's skip (vl/gmm.c:1099), and also as rows when q is not null;
+// tc_mstep_sums then forms the M-step's f64 sums (S0: K, S1 and S2: K x D, one
+// array) from that image and the centre of that E-step's model, on the same
+// thread, and tc_em_apply the update (vl/gmm.c:1036-1213).
+// tc_em_image_held: the thread already holds an image buffer for these sizes.
 i64 tc_estep_em(const float *X, i64 N, const DevModel<float> &m, float *q, double *ll_part,
                 int precision, cudaStream_t s);
-void tc_mstep(const float *X, i64 N, float *means, float *covs, float *priors, i64 K, i64 D,
-              const double *lb, int precision, cudaStream_t s);
+const double *tc_mstep_sums(const float *X, i64 N, i64 K, i64 D, int precision, cudaStream_t s);
+bool tc_em_image_held(i64 N, i64 K, int precision);
 // Streaming EM, one chunk of rows at a time (N x K never resident).  After
 // tc_estep_em on a chunk (or tc_em_image_from_rows, which makes the chunk's
 // thresholded fp16 image from row-major posteriors), tc_em_stats adds the

@@ -95,9 +95,13 @@ auto guarded(F &&f, decltype(f()) sentinel) -> decltype(f()) {
   return sentinel;
 }
 
+// What an E-step leaves: the posteriors as rows (dq), the tensor-core M-step's
+// operand image (see vlb::tc_estep_em), or both.
+enum class EstepOut { kRows, kImage, kRowsAndImage };
+
 template <typename T>
 double device_estep(const T *dX, i64 N, const vlb::DevModel<T> &m, T *dq, int precision,
-                    bool fast, cudaStream_t s, bool em_image = false);
+                    bool fast, cudaStream_t s, EstepOut out = EstepOut::kRows);
 
 // Posteriors of a streamed EM, recomputed chunk by chunk from the data and
 // the final parameters with the final E-step's arithmetic (the loop ends
@@ -124,7 +128,7 @@ void lazy_posteriors(VlGMM *self) {
         done = true;
       }
     }
-    if (!done) device_estep<T>(X + r0 * D, n, m, dq, self->lazyPrec, false, s, false);
+    if (!done) device_estep<T>(X + r0 * D, n, m, dq, self->lazyPrec, false, s);
     VLB_CUDA(cudaMemcpyAsync((T *)self->posteriors + r0 * K, dq, sizeof(T) * n * K, cudaMemcpyDeviceToHost, s));
     VLB_CUDA(cudaStreamSynchronize(s));
   }
@@ -158,23 +162,22 @@ void sync_posteriors(VlGMM *self) {
   self->postOnDevice = false;
 }
 
-// em_image: also write the posteriors as the tensor-core M-step's operand
-// image (EM with the tensor-core path; see vlb::tc_estep_em).
 template <typename T>
 double device_estep(const T *dX, i64 N, const vlb::DevModel<T> &m, T *dq, int precision,
-                    bool fast, cudaStream_t s, bool em_image) {
+                    bool fast, cudaStream_t s, EstepOut out) {
   vlb::Scratch &sc = vlb::thread_scratch();
   double *llp = sc.slot[15].get<double>(vlb::estep_ll_parts(N));
   double *dll = sc.slot[16].get<double>(1);
   bool done = false;
   i64 nparts = 0;
+  const bool image = out != EstepOut::kRows;
   if constexpr (sizeof(T) == 4) {
     // The EM image format needs a dimension the kernels are built for; the
     // posteriors alone also run zero-padded (vlb::tc_supported_padded).
     if (precision != VLB200_PREC_EXACT &&
-        (em_image ? vlb::tc_supported(m.K, m.D) : vlb::tc_supported_padded(m.K, m.D))) {
-      nparts = em_image ? vlb::tc_estep_em(dX, N, m, dq, llp, precision, s)
-                        : vlb::tc_estep(dX, N, m, dq, llp, fast, precision, s);
+        (image ? vlb::tc_supported(m.K, m.D) : vlb::tc_supported_padded(m.K, m.D))) {
+      nparts = image ? vlb::tc_estep_em(dX, N, m, out == EstepOut::kImage ? nullptr : dq, llp, precision, s)
+                     : vlb::tc_estep(dX, N, m, dq, llp, fast, precision, s);
       done = true;
       vlb::note_precision(precision);
     }
@@ -196,6 +199,9 @@ double device_estep(const T *dX, i64 N, const vlb::DevModel<T> &m, T *dq, int pr
   return ll;
 }
 
+// Mass below which a mode counts as empty.
+double restart_cutoff(i64 N, i64 K) { return 1e-2 * std::max(1.0, (double)N / (double)K); }
+
 // Empty-mode restarts, vl/gmm.c:814-999, with the posteriors and parameters
 // on the device and the (cheap) selection logic on the host.
 template <typename T>
@@ -208,7 +214,7 @@ vl_size restart_empty_modes(VlGMM *self, const T *dX, i64 N, T *dq, T *dmeans, T
   std::vector<double> mass(K);
   VLB_CUDA(cudaMemcpyAsync(mass.data(), dmass, sizeof(double) * K, cudaMemcpyDeviceToHost, s));
   VLB_CUDA(cudaStreamSynchronize(s));
-  const double cutoff = 1e-2 * std::max(1.0, (double)N / (double)K);
+  const double cutoff = restart_cutoff(N, K);
   vl_size nsplit = 0;
   std::vector<T> pr(K), cv(K * D), mu(K * D);
   bool have = false;
@@ -276,7 +282,14 @@ template <typename T>
 double em_device(VlGMM *self, const T *dX, i64 N, int precision) {
   cudaStream_t s = vlb::thread_stream();
   const i64 K = (i64)self->numClusters, D = (i64)self->dimension;
-  {
+  // Tensor-core modes run the M-step's statistics on the tensor cores from
+  // the E-step's posterior image; EXACT and double stay on the CUDA cores.
+  bool tcm = false;
+  if constexpr (sizeof(T) == 4) tcm = precision != VLB200_PREC_EXACT && vlb::tc_supported(K, D);
+  // Asked only when the posteriors (and image) are not held already: the query
+  // takes from 60 us to tens of ms on a machine with other users.
+  if (self->dq.cap < sizeof(T) * (size_t)std::max<i64>(1, N) * (size_t)K ||
+      (tcm && !vlb::tc_em_image_held(N, K, precision))) {
     size_t freeB = 0, totalB = 0;
     VLB_CUDA(cudaMemGetInfo(&freeB, &totalB));
     const double need = (double)N * (double)K * (sizeof(T) + 4.0);
@@ -304,10 +317,7 @@ double em_device(VlGMM *self, const T *dX, i64 N, int precision) {
   m.D = D;
 
   vlb::apply_bounds<T>(dcovs, K, D, dlb, s);  // vl/gmm.c:1233
-  // Tensor-core modes run the M-step's statistics on the tensor cores from
-  // the E-step's posterior image; EXACT and double stay on the CUDA cores.
-  bool tcm = false;
-  if constexpr (sizeof(T) == 4) tcm = precision != VLB200_PREC_EXACT && vlb::tc_supported(K, D);
+  bool rows = false;  // dq holds the last E-step's posteriors
   double prevLL = -INFINITY, LL = -INFINITY;
   std::vector<T> snap;
   for (vl_size it = 0;; ++it) {
@@ -320,7 +330,11 @@ double em_device(VlGMM *self, const T *dX, i64 N, int precision) {
       VLB_CUDA(cudaStreamSynchronize(s));
       self->paramTrace.emplace_back(snap.begin(), snap.end());
     }
-    LL = device_estep<T>(dX, N, m, dq, precision, false, s, tcm);
+    // With the tensor-core M-step an iteration writes the posteriors' image
+    // alone; as rows they are needed after the last one (vl_gmm_get_posteriors)
+    // and for a restart.
+    rows = !tcm || it >= self->maxNumIterations;
+    LL = device_estep<T>(dX, N, m, dq, precision, false, s, rows ? EstepOut::kRows : EstepOut::kImage);
     self->llTrace.push_back(LL);
     if (self->verbosity)
       VLB_PRINTF("gmm: em: iteration %d: loglikelihood = %f (variation = %f)\n", (int)it, LL,
@@ -340,23 +354,44 @@ double em_device(VlGMM *self, const T *dX, i64 N, int precision) {
     }
     prevLL = LL;
     vl_size r = 0;
-    if (it > 1) {
+    const double *S = nullptr;  // the tensor-core M-step's sums
+    bool check = it > 1;
+    if constexpr (sizeof(T) == 4) {
+      if (tcm) {
+        S = vlb::tc_mstep_sums(dX, N, K, D, precision, s);
+        // The sums' masses leave out the skipped posteriors, so a component
+        // whose sum reaches the restart's cut-off (with a margin above the
+        // image's rounding) has the mass; only when one does not are the
+        // posteriors formed as rows and their masses taken.
+        if (check && K > 1) {
+          std::vector<double> s0(K);
+          VLB_CUDA(cudaMemcpyAsync(s0.data(), S, sizeof(double) * K, cudaMemcpyDeviceToHost, s));
+          VLB_CUDA(cudaStreamSynchronize(s));
+          const double safe = 1.01 * restart_cutoff(N, K);
+          check = false;
+          for (i64 k = 0; k < K; ++k) check = check || !(s0[k] >= safe);
+          if (check) device_estep<T>(dX, N, m, dq, precision, false, s);
+        }
+      }
+    }
+    if (check) {
       r = restart_empty_modes<T>(self, dX, N, dq, dmeans, dcovs, dpriors, dlb, s);
       self->numRestarts += r;
       if (r > 0 && self->verbosity)
         VLB_PRINTF("gmm: em: %d Gaussian modes restarted because they had become empty.\n", (int)r);
     }
-    // A restart rewrites posteriors (vl/gmm.c:969-989), so the image is stale:
+    // A restart rewrites posteriors (vl/gmm.c:969-989), so the sums are stale:
     // that iteration's M-step reads the rows.
     bool done = false;
     if constexpr (sizeof(T) == 4) {
       if (tcm && r == 0) {
-        vlb::tc_mstep(dX, N, dmeans, dcovs, dpriors, K, D, dlb, precision, s);
+        vlb::tc_em_apply(S, S + K, S + K + K * D, dmeans, dcovs, dpriors, K, D, dlb, s);
         done = true;
       }
     }
     if (!done) vlb::exact_mstep<T>(dX, N, dq, dmeans, dcovs, dpriors, K, D, dlb, s);
   }
+  if (!rows) device_estep<T>(dX, N, m, dq, precision, false, s);  // converged early
   VLB_CUDA(cudaMemcpyAsync(self->means, dmeans, sizeof(T) * K * D, cudaMemcpyDeviceToHost, s));
   VLB_CUDA(cudaMemcpyAsync(self->covariances, dcovs, sizeof(T) * K * D, cudaMemcpyDeviceToHost, s));
   VLB_CUDA(cudaMemcpyAsync(self->priors, dpriors, sizeof(T) * K, cudaMemcpyDeviceToHost, s));
@@ -482,7 +517,7 @@ double em_stream_device(VlGMM *self, const T *dX, i64 N, int precision, const St
         return ll;
       }
     }
-    return device_estep<T>(dX + r0 * D, n, mm, q, precision, false, s, tcm);
+    return device_estep<T>(dX + r0 * D, n, mm, q, precision, false, s, tcm ? EstepOut::kRowsAndImage : EstepOut::kRows);
   };
 
   double prevLL = -INFINITY, LL = -INFINITY;

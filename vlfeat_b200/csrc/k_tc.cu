@@ -2041,55 +2041,49 @@ T *upload(DevBuf &b, const std::vector<T> &v, cudaStream_t s) {
   return d;
 }
 
+namespace {
+size_t em_image_bytes(i64 N, i64 K, int precision) {
+  const i64 ntiles = std::max<i64>(1, (N + 127) / 128);
+  return (size_t)ntiles * 128 * padQ(padK(K)) * (precision == VLB200_PREC_FP32 ? 4 : 2);
+}
+}  // namespace
+
+bool tc_em_image_held(i64 N, i64 K, int precision) {
+  return thread_scratch(kArenaTc).slot[4].cap >= em_image_bytes(N, K, precision);
+}
+
 i64 tc_estep_em(const float *X, i64 N, const DevModel<float> &m, float *q, double *ll_part,
                 int precision, cudaStream_t s) {
   Scratch &sc = thread_scratch(kArenaTc);
   const bool fp32 = (precision == VLB200_PREC_FP32);
   TcPrep tp;
   tc_prepare(m, tp, sc, s);
-  const int Kq = padQ(tp.Kp);
-  const i64 ntiles = (N + 127) / 128;
+  void *img = sc.slot[4].get<char>(em_image_bytes(N, m.K, precision));
   EOut eo;
-  eo.qimg = sc.slot[4].get<char>((size_t)std::max<i64>(1, ntiles) * 128 * Kq * (fp32 ? 4 : 2));
   eo.qthr = 1e-2 / (double)m.K;  // vl/gmm.c:1099
   int *err = sc.slot[3].get<int>(1);
-  const i64 n = estep_dispatch(tp.D, fp32 ? kQRowImg32 : kQRowImg16, X, N, tp, (void *)q, (int)m.K, false,
-                               nullptr, ll_part, err, 0, s, eo);
+  i64 n;
+  if (q) {
+    eo.qimg = img;
+    n = estep_dispatch(tp.D, fp32 ? kQRowImg32 : kQRowImg16, X, N, tp, (void *)q, (int)m.K, false, nullptr, ll_part,
+                       err, 0, s, eo);
+  } else {
+    n = estep_dispatch(tp.D, fp32 ? kQImg32 : kQImg16, X, N, tp, img, (int)m.K, false, nullptr, ll_part, err, 0, s, eo);
+  }
   check_err(err, s);
   return n;
 }
 
 constexpr i64 kEmItemRows = 8192;  // rows per statistics work item in EM
 
-void tc_mstep(const float *X, i64 N, float *means, float *covs, float *priors, i64 K, i64 D,
-              const double *lb, int precision, cudaStream_t s) {
+const double *tc_mstep_sums(const float *X, i64 N, i64 K, i64 D, int precision, cudaStream_t s) {
   Scratch &sc = thread_scratch(kArenaTc);
-  const bool fp32 = (precision == VLB200_PREC_FP32);
-  const int Kp = padK(K), Kq = padQ(Kp), NST = (int)(2 * D + 16);
-  const i64 ntiles = (N + 127) / 128;
-  constexpr i64 kItemRows = 8192;
-  std::vector<SItem> items;
-  for (i64 r = 0; r < N; r += kItemRows) items.push_back({r, std::min(N, r + kItemRows), (int)items.size(), 0});
-  const int nitems = (int)items.size();
-  const int gx = std::max(1, std::min(nitems, num_sms()));
-  std::vector<int> order, beg;
-  lpt_assign(items, gx, order, beg);
-  SItem *ditems = upload(sc.slot[7], items, s);
-  int *dorder = upload(sc.slot[8], order, s);
-  int *dbeg = upload(sc.slot[9], beg, s);
-  float *partial = sc.slot[6].get<float>((size_t)std::max(1, nitems) * Kp * NST);
-  int *err = sc.slot[3].get<int>(1);
-  VLB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-  if (nitems > 0) {
-    SParams sp;
-    sp.X = X; sp.qimg = (const uint8_t *)sc.slot[4].p; sp.qpart = ntiles * 128 * (i64)Kq * 2; sp.qbase = 0;
-    sp.K = (int)K; sp.Kp = Kp; sp.Kq = Kq; sp.nst = 0;
-    sp.ctr = (const float *)sc.slot[0].p; sp.scale = (const float *)sc.slot[12].p;
-    sp.items = ditems; sp.order = dorder; sp.cta_beg = dbeg; sp.partial = partial; sp.err = err;
-    stats_dispatch((int)D, fp32 ? 2 : 1, sp, gx, 0, 0, s);
-  }
-  tc_em_finalize(nitems, partial, means, covs, priors, K, D, lb, s);
-  check_err(err, s);
+  const i64 nitems = tc_em_items(N);
+  float *partial = sc.slot[6].get<float>((size_t)std::max<i64>(1, nitems) * tc_em_partial_floats(K, D));
+  tc_em_stats(X, 0, N, K, D, precision == VLB200_PREC_FP32 ? 2 : 1, partial, 0, s);
+  double *S = sc.slot[25].get<double>((size_t)(2 * D + 1) * K);
+  tc_em_sums((int)nitems, partial, K, D, S, S + K, S + K + K * D, s);
+  return S;
 }
 
 // ------------------------------------------------- streaming EM pieces
