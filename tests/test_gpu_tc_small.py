@@ -57,3 +57,31 @@ def test_prior_below_floor_and_rerun(vl, restatement):
     ref, _ = restatement.fisher(*[a.astype(np.float64) for a in (x, mu, cv, pr)], 0)
     assert rel_err(enc[0][0].cpu().numpy(), ref) < 5e-5
     assert torch.equal(enc[0], enc[1]) and torch.equal(enc[0], enc[2])
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("K,D", [(64, 1), (64, 12), (64, 16), (72, 20), (256, 81), (264, 84), (256, 96), (264, 96),
+                                 (256, 97), (264, 100), (512, 36)])
+def test_padded_rows(vl, restatement, K, D, shift):
+    """Dimensions the kernels pad: rows read where they are (multiples of 4,
+    16-byte aligned) or copied (others; shift moves the data by one float),
+    alone and in clusters of blocks, against the C restatement in double."""
+    import torch
+    pr, mu, cv, off, x = _case(K, D, [700, 0, 333], K + D)
+    buf = torch.zeros(x.size + 1, device="cuda")
+    t = buf[shift:shift + x.size].view(x.shape)
+    t.copy_(torch.from_numpy(x))
+    p = [torch.from_numpy(a).cuda() for a in (mu, cv, pr)]
+    d = [a.astype(np.float64) for a in (x, mu, cv, pr)]
+    enc = torch.zeros((3, 2 * K * D), device="cuda")
+    vl.fisher_encode_batch_device(enc, *p, t, off, 0, "fp32")
+    assert vl.last_precision() == "fp32"
+    for j in (0, 2):
+        ref, _ = restatement.fisher(d[0][off[j]:off[j + 1]], *d[1:], 0)
+        assert rel_err(enc[j].cpu().numpy(), ref) < 5e-5
+    q = torch.zeros((len(x), K), device="cuda")
+    ll = vl.gmm_posteriors_device(q, p[2], p[0], p[1], t, "fp32")
+    assert vl.last_precision() == "fp32"
+    rq, rll = restatement.posteriors(d[0], d[3], d[1], d[2])
+    assert np.max(np.abs(q.cpu().numpy() - rq)) < 4e-5
+    assert abs(ll - rll) < 4e-6 * abs(rll) + 1e-4 * len(x)

@@ -189,7 +189,7 @@ void wait_selftest(double limit_ms, cudaStream_t s);
 bool tc_fv_supported(i64 K, i64 D);
 // Shapes the tensor-core E-step (posteriors) and Fisher encoding take with
 // the dimension zero-padded to the next one the kernels are built for (64,
-// 80 or 128; any D <= 128).
+// 80, 96 or 128; any D <= 128).
 int tc_pad_dim(i64 D);
 bool tc_supported_padded(i64 K, i64 D);
 bool tc_fv_supported_padded(i64 K, i64 D);

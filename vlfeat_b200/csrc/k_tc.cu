@@ -370,8 +370,9 @@ __host__ __device__ constexpr bool q_image(int qf) { return qf != kQRow; }
 __host__ __device__ constexpr bool q_image32(int qf) { return qf == kQImg32 || qf == kQRowImg32; }
 
 struct EParams {
-  CUtensorMap xmap;  // SW: X as a {D, N} fp32 tensor, boxes of 16 dimensions x 128 rows
+  CUtensorMap xmap;  // SW: X as a {ldx, N} fp32 tensor, boxes of 16 dimensions x 128 rows
   const float *X;
+  int ldx;  // floats between rows of X, at most DIM; dimensions past it are zeros
   i64 N;
   // Kp: this CTA's components (at most 256); Kg: all padded components (the
   // W image's and cst2's extent; Kp times the cluster size); Kq: components in
@@ -532,7 +533,7 @@ __global__ void __launch_bounds__(tc_threads(SW), 1) k_tc_estep(const __grid_con
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
         const i64 row = t * 128 + 32 * warp + 8 * s + rr;
-        buf[s] = row < p.N ? __ldg((const float4 *)(p.X + row * DIM + d0)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        buf[s] = row < p.N && d0 < p.ldx ? __ldg((const float4 *)(p.X + row * p.ldx + d0)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     };
     // Position (tile, chunk) of the chunk being converted and, with W
@@ -1017,6 +1018,7 @@ struct SItem {
 struct SParams {
   CUtensorMap qmap;     // the image as {256 (one atom, u16), groups, 32-component blocks, parts}
   const float *X;
+  int ldx;              // floats between rows of X, at most DIM; dimensions past it are zeros
   const uint8_t *qimg;  // q^T operand image written by the E-step
   i64 qpart;            // bytes of one image part
   i64 qbase;            // row of X that the image's first row corresponds to
@@ -1143,13 +1145,13 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
           const uint32_t sa = smem_u32(sS + (size_t)stage * L::kStage);
           const uint32_t sx = sa + NPA * L::A_PART + L::NPB * L::B_PART;
           const int nx = (int)min((i64)32, item.row1 - cb);
-          mbar_arrive_expect_tx(&xfull[stage], (uint32_t)(NPA * L::A_PART) + (uint32_t)nx * DIM * 4);
+          mbar_arrive_expect_tx(&xfull[stage], (uint32_t)(NPA * L::A_PART) + (uint32_t)(nx * p.ldx * 4));
           // q^T for the chunk: groups (cb - qbase) / 8 .. +3 of this CTA's
           // 4 MT blocks, all parts, as one box laid out [part][block][group]
           // (groups past the image read as zero; groups past the item are
           // finite and meet zero x-side rows).
           tma_load_4d(sa, &p.qmap, 0, (int)((cb - p.qbase) >> 3), comp0 / 32, 0, &xfull[stage]);
-          bulk_g2s(sx, p.X + cb * DIM, (uint32_t)nx * DIM * 4, &xfull[stage]);
+          bulk_g2s(sx, p.X + cb * p.ldx, (uint32_t)(nx * p.ldx * 4), &xfull[stage]);
           ++it;
         }
       }
@@ -1182,8 +1184,8 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
             const bool in = row >= item.row0 && row < item.row1;
             const int d0 = 4 * pp;
             float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-            if (in) {
-              const float4 x = *(const float4 *)(xs + rs * DIM + d0);
+            if (in && d0 < p.ldx) {
+              const float4 x = *(const float4 *)(xs + rs * p.ldx + d0);
               v0 = (x.x - s_ctr[d0]) * s_scl[d0];
               v1 = (x.y - s_ctr[d0 + 1]) * s_scl[d0 + 1];
               v2 = (x.z - s_ctr[d0 + 2]) * s_scl[d0 + 2];
@@ -1228,8 +1230,8 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
               const bool sq = ff >= DIM;
               const int d0 = sq ? ff - DIM : ff;
               float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-              if (in) {
-                const float4 x = *(const float4 *)(xs + rs * DIM + d0);
+              if (in && d0 < p.ldx) {
+                const float4 x = *(const float4 *)(xs + rs * p.ldx + d0);
                 v0 = (x.x - s_ctr[d0]) * s_scl[d0];
                 v1 = (x.y - s_ctr[d0 + 1]) * s_scl[d0 + 1];
                 v2 = (x.z - s_ctr[d0 + 2]) * s_scl[d0 + 2];
@@ -1613,17 +1615,37 @@ __global__ void k_rows_to_image16(const float *__restrict__ q, i64 n, int K, int
 
 // ============================================================ padding
 // Dimensions the kernels are built for take the data as it is; any other
-// dimension up to 128 runs zero-padded to the next of them: each row gets
-// zero columns, each component mean 0 and variance 1 there, which adds 0 to
+// dimension up to 128 runs zero-padded to the next of them (or to 96): each row
+// gets zero columns, each component mean 0 and variance 1 there, which adds 0 to
 // every (x - mu)^2 / sigma^2 and to every sum of log sigma^2, so the
 // posteriors and the Fisher statistics of the real dimensions are unchanged
 // (the log-likelihood's D/2 log(2 pi) term is corrected for the padding).
-__global__ void k_pad_rows(const float *__restrict__ X, i64 N, int D, int Dp, float *__restrict__ Xp) {
-  const i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N * Dp) return;
-  const i64 r = i / Dp;
-  const int d = (int)(i - r * Dp);
-  Xp[i] = d < D ? X[r * D + d] : 0.f;
+//
+// k_pad_rows copies rows of D floats to rows of ld >= D floats, zeros behind: a
+// warp takes four rows at a time, all their loads in flight.  Bound by HBM:
+// 2.5 M rows of 82 floats to 84, 0.28 ms (to 128 with an index division per
+// element: 0.95).
+constexpr int kPadRows = 32;  // rows per block and step: 8 warps of 4
+__global__ void __launch_bounds__(256) k_pad_rows(const float *__restrict__ X, i64 N, int D, int ld,
+                                                  float *__restrict__ Xp) {
+  const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
+  for (i64 r0 = ((i64)blockIdx.x * 8 + w) * 4; r0 < N; r0 += (i64)gridDim.x * kPadRows) {
+    float v[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int d = lane + 32 * j;
+        v[u][j] = r0 + u < N && d < D ? __ldg(X + (r0 + u) * D + d) : 0.f;
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int d = lane + 32 * j;
+        if (r0 + u < N && d < ld) Xp[(r0 + u) * ld + d] = v[u][j];
+      }
+  }
 }
 __global__ void k_pad_model(const float *__restrict__ means, const float *__restrict__ covs, int K, int D, int Dp,
                             float *__restrict__ mp, float *__restrict__ cp) {
@@ -1638,6 +1660,7 @@ __global__ void k_pad_model(const float *__restrict__ means, const float *__rest
 // ================================================================ host
 struct TcPrep {
   int K = 0, Kp = 0, D = 0;
+  int ldx = 0;  // floats between descriptor rows (a multiple of 4, at most D)
   float *ctr = nullptr, *cst2 = nullptr, *scale = nullptr, *wsc = nullptr, *wbar = nullptr;
   double *cbar = nullptr;
   __half *wimg = nullptr;
@@ -1664,10 +1687,12 @@ struct FvConsts {
 // Model-derived operands of the tensor-core path: the centre, the
 // per-dimension scales, the fp16 W image with its scale, and the constants.
 // Also clears the arena's error word (slot 3).
-void tc_prepare(const DevModel<float> &m, TcPrep &tp, Scratch &sc, cudaStream_t s, const FvConsts *fv = nullptr) {
+void tc_prepare(const DevModel<float> &m, TcPrep &tp, Scratch &sc, cudaStream_t s, const FvConsts *fv = nullptr,
+                int ldx = 0) {
   tp.K = (int)m.K;
   tp.Kp = padK(m.K);
   tp.D = (int)m.D;
+  tp.ldx = ldx > 0 ? ldx : tp.D;
   const int KD2 = 2 * tp.D;
   tp.ctr = sc.slot[0].get<float>(256);
   tp.cst2 = sc.slot[1].get<float>(std::max(256, tp.Kp));
@@ -1746,12 +1771,12 @@ i64 launch_estep_impl(const float *X, i64 N, const TcPrep &tp, void *q, int ldq,
   }
   VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   EParams p;
-  p.X = X; p.N = N; p.K = tp.K; p.Kp = Kb; p.Kg = tp.Kp; p.Kq = padQ(tp.Kp); p.nst = nst; p.nxs = nxs;
+  p.X = X; p.ldx = tp.ldx; p.N = N; p.K = tp.K; p.Kp = Kb; p.Kg = tp.Kp; p.Kq = padQ(tp.Kp); p.nst = nst; p.nxs = nxs;
   if constexpr (SW) {
     // Boxes of 16 dimensions (64 bytes, 16-byte aligned) x 128 rows; the row
     // coordinate is a 32-bit TMA coordinate.
     VLB_CHECK(ntiles * 128 <= (i64)INT32_MAX, VL_ERR_BAD_ARG, "tensor-core E-step: at most 2^31 - 128 rows per launch");
-    tc::tma_map_2d(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, X, N, DIM, 16, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
+    tc::tma_map_2d(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, X, N, tp.ldx, 16, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
   } else {
     std::memset(&p.xmap, 0, sizeof p.xmap);
   }
@@ -1799,7 +1824,7 @@ i64 launch_estep(const float *X, i64 N, const TcPrep &tp, void *q, int ldq, bool
                  const EOut &eo) {
   if (tp.Kp > 256) {
     const int Kb = tp.Kp / kblocks(tp.Kp);
-    if constexpr (DIM == 128) {
+    if constexpr (DIM > 80) {
       if (ELayout<DIM, false, true>::max_stages(Kb) < 2)
         return launch_estep_impl<DIM, QF, true, true>(X, N, tp, q, ldq, fast, rowcnt, ll_part, err, nst_req, s, eo);
     }
@@ -1840,11 +1865,13 @@ struct Tc {
   static constexpr bool kTwo = 2 * (2 * DIM + 16) <= 512;  // two M tiles fit in TMEM
   static i64 estep(int qf, const float *X, i64 N, const TcPrep &tp, void *q, int ldq, bool fast,
                    unsigned *rowcnt, double *ll, int *err, int nst, cudaStream_t s, const EOut &eo) {
+    if constexpr (DIM != 96) {  // EM runs unpadded dimensions only
+      if (qf == kQRowImg16) return launch_estep<DIM, kQRowImg16>(X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
+      if (qf == kQRowImg32) return launch_estep<DIM, kQRowImg32>(X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
+    }
     switch (qf) {
       case kQImg16: return launch_estep<DIM, kQImg16>(X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
       case kQImg32: return launch_estep<DIM, kQImg32>(X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
-      case kQRowImg16: return launch_estep<DIM, kQRowImg16>(X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
-      case kQRowImg32: return launch_estep<DIM, kQRowImg32>(X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
       default: return launch_estep<DIM, kQRow>(X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
     }
   }
@@ -1877,6 +1904,7 @@ i64 estep_dispatch(int D, int qf, const float *X, i64 N, const TcPrep &tp, void 
   switch (D) {
     case 64: return Tc<64>::estep(qf, X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
     case 80: return Tc<80>::estep(qf, X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
+    case 96: return Tc<96>::estep(qf, X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
     case 128: return Tc<128>::estep(qf, X, N, tp, q, ldq, fast, rowcnt, ll, err, nst, s, eo);
     default: throw Error(VL_ERR_BAD_ARG, "tensor-core path: unsupported dimension");
   }
@@ -1886,6 +1914,7 @@ void stats_dispatch(int D, int split, const SParams &p, int grid_x, int mt, int 
   switch (D) {
     case 64: Tc<64>::stats(split, p, grid_x, mt, nst, s); break;
     case 80: Tc<80>::stats(split, p, grid_x, mt, nst, s); break;
+    case 96: Tc<96>::stats(split, p, grid_x, mt, nst, s); break;
     case 128: Tc<128>::stats(split, p, grid_x, mt, nst, s); break;
     default: throw Error(VL_ERR_BAD_ARG, "tensor-core path: unsupported dimension");
   }
@@ -1971,30 +2000,51 @@ bool tc_supported(i64 K, i64 D) {
   return D == 64 ? ELayout<64, false, true>::max_stages(Kb) >= 2 : ELayout<80, false, true>::max_stages(Kb) >= 2;
 }
 
-int tc_pad_dim(i64 D) { return D <= 64 ? 64 : D <= 80 ? 80 : D <= 128 ? 128 : 0; }
+// The dimension D runs in: the next one the kernels are built for.  96 is built
+// for padded encoding and posteriors only (82 dimensions, 2.5 M rows, K = 256,
+// FP32: E-step 1.11 ms in 128 dimensions, 0.94 in 96; statistics 1.21 and 0.83).
+int tc_pad_dim(i64 D) { return D <= 64 ? 64 : D <= 80 ? 80 : D <= 96 ? 96 : D <= 128 ? 128 : 0; }
 
-bool tc_supported_padded(i64 K, i64 D) { return tc_pad_dim(D) > 0 && tc_supported(K, tc_pad_dim(D)); }
+namespace {
+// Whether a padded dimension takes the tensor cores is decided by the next
+// dimension that tc_supported takes (64, 80 or 128).
+i64 route_dim(i64 D) { return D <= 64 ? 64 : D <= 80 ? 80 : D <= 128 ? 128 : 0; }
+}  // namespace
+
+bool tc_supported_padded(i64 K, i64 D) { return route_dim(D) > 0 && tc_supported(K, route_dim(D)); }
 
 bool tc_fv_supported_padded(i64 K, i64 D) {
-  const int Dp = tc_pad_dim(D);
-  return Dp > 0 && tc_supported(K, Dp) && K % 4 == 0 && sizeof(float) * 2 * (size_t)(K / 4) * D <= (size_t)kSmemLimit;
+  return tc_supported_padded(K, D) && K % 4 == 0 && sizeof(float) * 2 * (size_t)(K / 4) * D <= (size_t)kSmemLimit;
 }
 
-// Zero-padded copies of rows and model in `sc` (slots 22-24).
+// The model zero-padded to dimension Dp, and the rows with ldx floats each, in
+// `sc` (slots 22-24).  The kernels take dimensions past a row's floats as zeros,
+// so rows that are whole 16-byte pieces are read where they are, and others are
+// copied with up to three zeros added.
 struct Padded {
   DevModel<float> m;
   const float *X = nullptr;
+  int ldx = 0;
 };
-Padded pad_inputs(const float *X, i64 N, const DevModel<float> &m, Scratch &sc, cudaStream_t s) {
+Padded pad_inputs(const float *X, i64 N, const DevModel<float> &m, int Dp, bool whole, Scratch &sc, cudaStream_t s) {
   Padded P;
-  const int Dp = tc_pad_dim(m.D), D = (int)m.D;
-  float *xp = sc.slot[22].get<float>((size_t)std::max<i64>(1, N) * Dp);
+  const int D = (int)m.D;
   float *mp = sc.slot[23].get<float>((size_t)m.K * Dp), *cp = sc.slot[24].get<float>((size_t)m.K * Dp);
-  if (N > 0)
-    VLB_LAUNCH("pad_rows", s, k_pad_rows<<<(unsigned)((N * Dp + 255) / 256), 256, 0, s>>>(X, N, D, Dp, xp));
+  if (!whole && D % 4 == 0 && D >= 16 && ((uintptr_t)X & 15) == 0) {
+    P.X = X;
+    P.ldx = D;
+  } else {
+    P.ldx = whole ? Dp : std::max(16, (D + 3) / 4 * 4);
+    float *xp = sc.slot[22].get<float>((size_t)std::max<i64>(1, N) * P.ldx);
+    if (N > 0) {
+      const i64 blocks = (N + kPadRows - 1) / kPadRows;
+      VLB_LAUNCH("pad_rows", s,
+                 k_pad_rows<<<(unsigned)std::min<i64>(blocks, 16 * num_sms()), 256, 0, s>>>(X, N, D, P.ldx, xp));
+    }
+    P.X = xp;
+  }
   VLB_LAUNCH("pad_model", s,
              k_pad_model<<<(unsigned)((m.K * Dp + 255) / 256), 256, 0, s>>>(m.means, m.covs, (int)m.K, D, Dp, mp, cp));
-  P.X = xp;
   P.m = m;
   P.m.means = mp;
   P.m.covs = cp;
@@ -2012,23 +2062,22 @@ i64 tc_estep(const float *X, i64 N, const DevModel<float> &m, float *q, double *
              int precision, cudaStream_t s, Scratch *arena) {
   (void)precision;
   Scratch &sc = arena ? *arena : thread_scratch(kArenaTc);
-  if (!tc_supported(m.K, m.D)) {
-    // Zero-padded dimension: the same posteriors; the log-likelihood's
-    // -D/2 log(2 pi) per row was taken with the padded D, so one more
-    // partial adds (Dp - D)/2 log(2 pi) for each row back.
-    const Padded P = pad_inputs(X, N, m, sc, s);
-    const i64 n = tc_estep(P.X, N, P.m, q, ll_part, fast, precision, s, &sc);
-    if (!ll_part) return n;
+  const bool padded = !tc_supported(m.K, m.D);
+  Padded P;
+  if (padded) P = pad_inputs(X, N, m, tc_pad_dim(m.D), false, sc, s);
+  TcPrep tp;
+  tc_prepare(padded ? P.m : m, tp, sc, s, nullptr, P.ldx);
+  int *err = sc.slot[3].get<int>(1);
+  i64 n = estep_dispatch(tp.D, kQRow, padded ? P.X : X, N, tp, (void *)q, (int)m.K, fast, nullptr, ll_part, err, 0, s);
+  check_err(err, s);
+  if (padded && ll_part) {
+    // The same posteriors, but the log-likelihood's -D/2 log(2 pi) per row was
+    // taken with the padded dimension: one more partial adds the difference.
     const double fix = 0.5 * (double)(P.m.D - m.D) * log(2.0 * 3.141592653589793) * (double)N;
     VLB_CUDA(cudaMemcpyAsync(ll_part + n, &fix, sizeof(double), cudaMemcpyHostToDevice, s));
     VLB_CUDA(cudaStreamSynchronize(s));
-    return n + 1;
+    ++n;
   }
-  TcPrep tp;
-  tc_prepare(m, tp, sc, s);
-  int *err = sc.slot[3].get<int>(1);
-  const i64 n = estep_dispatch(tp.D, kQRow, X, N, tp, (void *)q, (int)m.K, fast, nullptr, ll_part, err, 0, s);
-  check_err(err, s);
   return n;
 }
 
@@ -2126,7 +2175,7 @@ void tc_em_stats(const float *X, i64 row0, i64 n, i64 K, i64 D, int split, float
   int *err = sc.slot[3].get<int>(1);
   VLB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   SParams sp;
-  sp.X = X; sp.qimg = (const uint8_t *)sc.slot[4].p; sp.qpart = ntiles * 128 * (i64)Kq * 2; sp.qbase = row0;
+  sp.X = X; sp.ldx = (int)D; sp.qimg = (const uint8_t *)sc.slot[4].p; sp.qpart = ntiles * 128 * (i64)Kq * 2; sp.qbase = row0;
   sp.K = (int)K; sp.Kp = Kp; sp.Kq = Kq; sp.nst = 0;
   sp.ctr = (const float *)sc.slot[0].p; sp.scale = (const float *)sc.slot[12].p;
   sp.items = ditems; sp.order = dorder; sp.cta_beg = dbeg; sp.partial = partial; sp.err = err;
@@ -2291,6 +2340,7 @@ void launch_fv_finalize(int D, i64 nimg, cudaStream_t s, int K, int Kp, int Dr, 
   };
   if (D == 64) go(std::integral_constant<int, 64>());
   else if (D == 80) go(std::integral_constant<int, 80>());
+  else if (D == 96) go(std::integral_constant<int, 96>());
   else go(std::integral_constant<int, 128>());
 }
 
@@ -2304,7 +2354,7 @@ using ChunkHook = std::function<void(size_t)>;
 void fv_run(const FvLayout &L, Scratch &sc, const float *X, const DevModel<float> &m, float *enc,
             unsigned long long *nterms, int flags, int precision, const TcFvConfig &cfg, cudaStream_t s,
             const ChunkHook &before = nullptr, const ChunkHook &after = nullptr,
-            const DevModel<float> *mreal = nullptr) {
+            const DevModel<float> *mreal = nullptr, int ldx = 0) {
   const bool fp32 = (precision == VLB200_PREC_FP32);
   TcPrep tp;
   const int qf = fp32 ? kQImg32 : kQImg16;
@@ -2316,7 +2366,7 @@ void fv_run(const FvLayout &L, Scratch &sc, const float *X, const DevModel<float
   const DevModel<float> &mr = mreal ? *mreal : m;
   const i64 Dr = mr.D;
   const FvConsts fc{&mr, cmu, cis2, cisd, cup, cvp};
-  tc_prepare(m, tp, sc, s, &fc);
+  tc_prepare(m, tp, sc, s, &fc, ldx);
   const int Kq = padQ(tp.Kp);
   int *err = sc.slot[3].get<int>(1);
   void *q = sc.slot[4].p;
@@ -2334,17 +2384,17 @@ void fv_run(const FvLayout &L, Scratch &sc, const float *X, const DevModel<float
       if (precision == VLB200_PREC_BF16_ROUTER) {
         // Router posteriors (row-major) -> fp16 operand image + row counts.
         float *qrows = sc.slot[18].get<float>((size_t)L.maxRows * K);
-        router_default_posteriors(X + c.row0 * D, c.nrows, m, qrows, s);
+        router_default_posteriors(X + c.row0 * tp.ldx, c.nrows, m, qrows, s);
         const i64 rowsPad = ntiles * 128;
         VLB_LAUNCH("tc_rows_to_image", s,
                    k_rows_to_image16<<<(unsigned)((rowsPad + 7) / 8), 256, 0, s>>>(
                        qrows, c.nrows, (int)K, Kq, 1e-6f, (__half *)q, rowcnt, rowsPad, (flags & 4) != 0));
       } else {
-        estep_dispatch(tp.D, qf, X + c.row0 * D, c.nrows, tp, q, (int)K, (flags & 4) != 0, rowcnt, nullptr,
+        estep_dispatch(tp.D, qf, X + c.row0 * tp.ldx, c.nrows, tp, q, (int)K, (flags & 4) != 0, rowcnt, nullptr,
                        err, cfg.estepStages, s);
       }
       SParams sp;
-      sp.X = X; sp.qimg = (const uint8_t *)q; sp.qpart = ntiles * 128 * (i64)Kq * 2; sp.qbase = c.row0;
+      sp.X = X; sp.ldx = tp.ldx; sp.qimg = (const uint8_t *)q; sp.qpart = ntiles * 128 * (i64)Kq * 2; sp.qbase = c.row0;
       sp.K = (int)K; sp.Kp = tp.Kp; sp.Kq = Kq; sp.nst = 0;
       sp.ctr = tp.ctr; sp.scale = tp.scale;
       sp.items = ditems + c.items; sp.order = dorder + c.items; sp.cta_beg = dbeg + c.beg;
@@ -2368,18 +2418,21 @@ void tc_fisher_batch(const float *X, const i64 *h_offsets, i64 numImages, const 
   const int Kp = padK(m.K);
   TcFvConfig cfg;
   FvLayout L;
-  fv_layout(h_offsets, numImages, default_row_budget(Kp, fp32), cfg.itemRows, Kp, tc_pad_dim(m.D), num_sms(), L);
   if (!tc_fv_supported(m.K, m.D)) {
+    // The router reads whole padded rows.
+    const bool router = precision == VLB200_PREC_BF16_ROUTER;
+    const int Dp = router ? (int)route_dim(m.D) : tc_pad_dim(m.D);
     const i64 N = h_offsets[numImages] - h_offsets[0];
-    const Padded P = pad_inputs(X + h_offsets[0] * m.D, N, m, sc, s);
+    const Padded P = pad_inputs(X + h_offsets[0] * m.D, N, m, Dp, router, sc, s);
     std::vector<i64> offs(h_offsets, h_offsets + numImages + 1);
     for (auto &o : offs) o -= h_offsets[0];
-    fv_layout(offs.data(), numImages, default_row_budget(Kp, fp32), cfg.itemRows, Kp, P.m.D, num_sms(), L);
-    fv_upload(L, Kp, padQ(Kp), (int)(2 * P.m.D + 16), fp32, sc, s);
-    fv_run(L, sc, P.X, P.m, enc, nterms, flags, precision, cfg, s, nullptr, nullptr, &m);
+    fv_layout(offs.data(), numImages, default_row_budget(Kp, fp32), cfg.itemRows, Kp, Dp, num_sms(), L);
+    fv_upload(L, Kp, padQ(Kp), 2 * Dp + 16, fp32, sc, s);
+    fv_run(L, sc, P.X, P.m, enc, nterms, flags, precision, cfg, s, nullptr, nullptr, &m, P.ldx);
     check_err((int *)sc.slot[3].p, s);
     return;
   }
+  fv_layout(h_offsets, numImages, default_row_budget(Kp, fp32), cfg.itemRows, Kp, m.D, num_sms(), L);
   fv_upload(L, Kp, padQ(Kp), (int)(2 * m.D + 16), fp32, sc, s);
   fv_run(L, sc, X, m, enc, nterms, flags, precision, cfg, s);
   check_err((int *)sc.slot[3].p, s);
