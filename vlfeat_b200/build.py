@@ -27,7 +27,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hi
           "-I", os.path.join(ROOT, "include"), "-I", CSRC]
 SOURCES = ["runtime.cpp", "gmm_api.cpp", "fisher_api.cpp", "fisher_plan.cpp", "k_exact.cu", "k_tc.cu", "k_noalloc.cu",
            "k_router.cu", "k_mlp.cu", "k_vlad.cu", "k_pca.cu", "k_kmeans.cu"]
-HEADERS = ["common.h", "engine.h", "tc_common.cuh", "exact_math.cuh", "ordered_sum.cuh"]
+HEADERS = ["common.h", "engine.h", "tc_common.cuh", "exact_math.cuh", "ordered_sum.cuh", "seq_sum.cuh"]
 
 
 def _newer(src: str, dst: str, deps) -> bool:

@@ -16,6 +16,7 @@
 #include "engine.h"
 #include "exact_math.cuh"
 #include "ordered_sum.cuh"
+#include "seq_sum.cuh"
 #include "tc_common.cuh"
 
 namespace vlb {
@@ -1882,82 +1883,7 @@ __global__ void __launch_bounds__(kThreads) k_kpp_update(const T *__restrict__ X
   }
 }
 
-// ---- a sequential floating-point sum, formed in parallel ----
-// The sum acc = rn(acc + v_i), in order, of non-negative terms: while acc stays
-// in one binade [2^e, 2^(e+1)) it is an integer A times the binade's ulp u, and
-// an addition adds to A the term rounded to a multiple of u; only an exact tie
-// depends on acc, through A's parity (round half to even).  So a run of terms
-// maps A's parity to an increment, such maps compose associatively, and a
-// block scans them; the term that takes acc past the binade (or is not a
-// finite non-negative number) is added by its thread as it is, and the scan
-// goes on from there with the next binade.  Zero and subnormal acc count as
-// the lowest binade, whose ulp they share.  Every prefix has the bits of the
-// loop's.
-template <typename T>
-struct SeqFloat;
-template <>
-struct SeqFloat<float> {
-  using U = uint32_t;
-  static constexpr int kMant = 23, kExpMax = 255;
-  static __device__ __forceinline__ U bits(float v) { return __float_as_uint(v); }
-  static __device__ __forceinline__ float value(U b) { return __uint_as_float(b); }
-};
-template <>
-struct SeqFloat<double> {
-  using U = unsigned long long;
-  static constexpr int kMant = 52, kExpMax = 2047;
-  static __device__ __forceinline__ U bits(double v) { return (U)__double_as_longlong(v); }
-  static __device__ __forceinline__ double value(U b) { return __longlong_as_double((long long)b); }
-};
-template <typename T>
-struct Seq {
-  using F = SeqFloat<T>;
-  using U = typename F::U;
-  static constexpr U kOne = (U)1 << F::kMant, kLim = kOne * 2, kSat = kOne * 4;
-  // A map is 4 i + (d + 1): i is the increment of an even A (at most kSat), d in
-  // {-1, 0, 1} how much more an odd A gains.  (A tie sends one of the two
-  // starts up and the other down; from then on both have the same parity, so
-  // d stays.)
-  static constexpr U kIdentity = 1;
-  static __device__ __forceinline__ U pack(U i, int d) { return ((i < kSat ? i : kSat) << 2) | (U)(d + 1); }
-  static __device__ __forceinline__ int diff(U m) { return (int)(m & 3) - 1; }
-  static __device__ __forceinline__ U gain(U m, bool odd) { return (m >> 2) + (U)(odd ? diff(m) : 0); }
-  static __device__ __forceinline__ U then(U a, U b) {
-    const bool odd = ((a >> 2) & 1) != 0;
-    const int da = diff(a), db = diff(b);
-    return pack((a >> 2) + gain(b, odd), da ? da : odd ? -db : db);
-  }
-  // Biased exponent (at least 1) and integer of a finite non-negative value.
-  static __device__ __forceinline__ int exponent(U b) { return max(1, (int)(b >> F::kMant)); }
-  static __device__ __forceinline__ U integer(U b) { return (b & (kOne - 1)) | (b >> F::kMant ? kOne : (U)0); }
-  static __device__ __forceinline__ T value(int be, U A) {
-    return F::value(A < kOne ? A : ((U)be << F::kMant) + (A - kOne));  // A < kOne only in the lowest binade
-  }
-  // The map of a run of terms, acc in the binade with biased exponent be: the
-  // run added to the binade's first value (an even A) and to the next (odd).
-  // A sum that leaves the binade, or is not a number, saturates: whatever A it
-  // starts from, its thread adds the terms as they are.
-  template <int EPT>
-  static __device__ __forceinline__ U run(const T (&v)[EPT], int be) {
-    const U b0 = (U)be << F::kMant;
-    T x0 = F::value(b0), x1 = F::value(b0 + 1);
-    const T lim = add_rn(x0, x0);
-#pragma unroll
-    for (int u = 0; u < EPT; ++u) {
-      x0 = add_rn(x0, v[u]);
-      x1 = add_rn(x1, v[u]);
-    }
-    if (!(x0 < lim && x1 < lim && x0 >= F::value(b0))) return pack(kSat, 0);
-    const U i = F::bits(x0) - b0;
-    return pack(i, (int)(F::bits(x1) - b0 - 1 - i));
-  }
-};
-
-constexpr int kKppThreads = 256, kKppStages = 4;
-template <typename T>
-__host__ __device__ constexpr int kpp_ept() { return 128 / (int)sizeof(T); }  // terms per thread and tile
-template <typename T>
-__host__ __device__ constexpr int kpp_tile() { return kKppThreads * kpp_ept<T>(); }
+constexpr int kKppStages = 4;
 
 // The next centre, vl/kmeans.c:631-641: the energy (sum of minDist in order),
 // then the first x whose prefix sum is >= thresh * energy, or N - 1 (a NaN
@@ -1966,37 +1892,33 @@ __host__ __device__ constexpr int kpp_tile() { return kKppThreads * kpp_ept<T>()
 // is scanned again.  One block: 100,000 terms take 28 us, 1 M 138 us; a
 // thread that adds in order takes 290 and 2,900 (7 clocks a term).
 template <typename T>
-__global__ void __launch_bounds__(kKppThreads) k_kpp_select(const T *__restrict__ minDist, i64 N, T thresh,
+__global__ void __launch_bounds__(kSeqThreads) k_kpp_select(const T *__restrict__ minDist, i64 N, T thresh,
                                                             T *__restrict__ ck, i64 *__restrict__ xOut) {
-  using S = Seq<T>;
-  using U = typename S::U;
-  constexpr int NW = kKppThreads / 32, EPT = kpp_ept<T>(), kTile = kpp_tile<T>();
-  __shared__ U s_warp[2][NW];
-  __shared__ T s_acc;
-  __shared__ int s_next, s_tile;
-  __shared__ i64 s_x;
+  constexpr int EPT = seq_ept<T>(), kTile = seq_tile<T>();
+  __shared__ SeqShared<T> sh;
+  __shared__ int s_tile;
   extern __shared__ __align__(16) unsigned char kps_smem[];
   constexpr int VE = 16 / (int)sizeof(T), P = EPT + VE;  // a thread's terms and 16 bytes, so that its reads spread over the banks
   T *ring = (T *)kps_smem;                               // [stage][thread][P]
-  const int tid = threadIdx.x, lane = tid % 32, w = tid / 32;
+  const int tid = threadIdx.x;
   const i64 ntile = (N + kTile - 1) / kTile;
-  int pb = 0;  // warp totals' buffer: a pass writes the one the pass before did not
+  int pb = 0;
   // Terms of a tile to its stage, zeros past the end; and this thread's terms from there.
   auto issue = [&](i64 tile, int stage) {
     if (tile < ntile)
 #pragma unroll
-      for (int u = 0; u < kTile / VE / kKppThreads; ++u) {
-        const int e = (u * kKppThreads + tid) * VE;
+      for (int u = 0; u < kTile / VE / kSeqThreads; ++u) {
+        const int e = (u * kSeqThreads + tid) * VE;
         const i64 i = tile * kTile + e;
         const i64 left = N - i;
         const uint32_t bytes = left >= VE ? 16u : left > 0 ? (uint32_t)(left * (i64)sizeof(T)) : 0u;
-        cp_async16(tc::smem_u32(ring + ((size_t)stage * kKppThreads + e / EPT) * P + e % EPT),
+        cp_async16(tc::smem_u32(ring + ((size_t)stage * kSeqThreads + e / EPT) * P + e % EPT),
                    bytes ? minDist + i : minDist, bytes);
       }
     cp_async_commit();
   };
   auto load = [&](int stage, T(&v)[EPT]) {
-    const T *src = ring + ((size_t)stage * kKppThreads + tid) * P;
+    const T *src = ring + ((size_t)stage * kSeqThreads + tid) * P;
 #pragma unroll
     for (int u = 0; u < EPT; u += VE) {
       using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
@@ -2004,76 +1926,6 @@ __global__ void __launch_bounds__(kKppThreads) k_kpp_select(const T *__restrict_
 #pragma unroll
       for (int e = 0; e < VE; ++e) v[u + e] = ((const T *)&x)[e];
     }
-  };
-  auto scan = [&](U m, int width) {
-    if (!__any_sync(0xffffffffu, S::diff(m) != 0)) {  // no ties: plain saturating sums
-      U i = m >> 2;
-#pragma unroll
-      for (int o = 1; o < width; o <<= 1) {
-        const U p = __shfl_up_sync(0xffffffffu, i, o);
-        if (lane >= o) i = min(i + p, S::kSat);
-      }
-      return S::pack(i, 0);
-    }
-#pragma unroll
-    for (int o = 1; o < width; o <<= 1) {
-      const U p = __shfl_up_sync(0xffffffffu, m, o);
-      if (lane >= o) m = S::then(p, m);
-    }
-    return m;
-  };
-  // Adds the tile's terms to acc; with find, stops at the first prefix >= t and
-  // returns true (its index in s_x).  All threads hold the same acc.
-  auto run = [&](const T(&v)[EPT], T &acc, bool find, T t, i64 base) -> bool {
-    int from = 0;  // first thread whose terms are not in acc
-    while (from < kKppThreads) {
-      if (!(acc < (T)INFINITY)) {
-        // NaN stays; infinity turns into NaN at a NaN or -infinity.
-        bool nan = false;
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) nan |= tid >= from && !(v[u] > -(T)INFINITY);
-        if (__syncthreads_or(nan)) acc = add_rn(acc, (T)NAN);
-        return false;
-      }
-      const U ab = S::F::bits(acc), A = S::integer(ab);
-      const int be = S::exponent(ab);
-      const bool odd = (A & 1) != 0;
-      const U m = scan(tid >= from ? S::run(v, be) : S::kIdentity, 32);
-      if (lane == 31) s_warp[pb][w] = m;
-      __syncthreads();
-      const U x = scan(lane < NW ? s_warp[pb][lane] : S::kIdentity, NW);  // inclusive over the warps, in every warp
-      pb ^= 1;
-      auto stops = [&](U end) { return end >= S::kLim || (find && S::value(be, end) >= t); };
-      const unsigned at = __ballot_sync(0xffffffffu, lane < NW && stops(A + S::gain(x, odd)));
-      if (!at) {
-        acc = S::value(be, A + S::gain(__shfl_sync(0xffffffffu, x, NW - 1), odd));
-        return false;
-      }
-      // The first thread whose terms leave the binade (or reach t) adds them.
-      const U before = __shfl_sync(0xffffffffu, x, max(w - 1, 0));
-      if (w == __ffs(at) - 1) {
-        const U prev = w > 0 ? before : S::kIdentity;
-        const U incl = S::then(prev, m), up = __shfl_up_sync(0xffffffffu, incl, 1);
-        const unsigned in = __ballot_sync(0xffffffffu, stops(A + S::gain(incl, odd)));
-        if (lane == __ffs(in) - 1) {
-          T y = S::value(be, A + S::gain(lane > 0 ? up : prev, odd));
-          i64 hit = -1;
-#pragma unroll
-          for (int u = 0; u < EPT; ++u) {
-            y = add_rn(y, v[u]);
-            if (find && hit < 0 && y >= t) hit = base + tid * EPT + u;
-          }
-          s_acc = y;
-          s_next = tid + 1;
-          s_x = hit;
-        }
-      }
-      __syncthreads();
-      acc = s_acc;
-      from = s_next;
-      if (find && s_x >= 0) return true;
-    }
-    return false;
   };
   T v[EPT];
   T acc = (T)0;
@@ -2083,7 +1935,7 @@ __global__ void __launch_bounds__(kKppThreads) k_kpp_select(const T *__restrict_
     __syncthreads();  // the tile has landed; every thread has read the one before
     load((int)(tile % kKppStages), v);
     issue(tile + kKppStages - 1, (int)((tile + kKppStages - 1) % kKppStages));
-    run(v, acc, false, (T)0, 0);
+    seq_add<T, false>(v, acc, (T)0, 0, sh, pb);
     if (tid == 0) ck[tile] = acc;
   }
   cp_async_wait<0>();
@@ -2091,7 +1943,7 @@ __global__ void __launch_bounds__(kKppThreads) k_kpp_select(const T *__restrict_
   const T t = mul_rn(thresh, acc);
   if (tid == 0) s_tile = 0x7fffffff;
   __syncthreads();
-  for (i64 j = tid; j < ntile; j += kKppThreads)
+  for (i64 j = tid; j < ntile; j += kSeqThreads)
     if (ck[j] >= t) {
       atomicMin(&s_tile, (int)j);
       break;
@@ -2107,8 +1959,8 @@ __global__ void __launch_bounds__(kKppThreads) k_kpp_select(const T *__restrict_
   cp_async_wait<0>();
   __syncthreads();
   load(0, v);
-  const bool found = run(v, acc, true, t, (i64)tile * kTile);
-  if (tid == 0) *xOut = found ? min(s_x, N - 1) : N - 1;
+  const bool found = seq_add<T, true>(v, acc, t, (i64)tile * kTile, sh, pb);
+  if (tid == 0) *xOut = found ? min((i64)sh.x, N - 1) : N - 1;
 }
 
 template <typename T>
@@ -2144,8 +1996,8 @@ void kmeanspp(const T *X, i64 N, i64 D, i64 K, T *centers, i64 x0, const std::ve
   Scratch &sc = thread_scratch(kArenaExact);
   T *minDist = sc.slot[20].get<T>(N);
   i64 *xdev = sc.slot[21].get<i64>(1);
-  T *ck = sc.slot[22].get<T>(N / kpp_tile<T>() + 1);
-  constexpr size_t ssmem = (size_t)kKppStages * kKppThreads * (kpp_ept<T>() * sizeof(T) + 16);
+  T *ck = sc.slot[22].get<T>(N / seq_tile<T>() + 1);
+  constexpr size_t ssmem = (size_t)kKppStages * kSeqThreads * (seq_ept<T>() * sizeof(T) + 16);
   VLB_CUDA(cudaFuncSetAttribute(k_kpp_select<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem));
   for (i64 c = 0; c < K; ++c) {
     const i64 *xp = c == 0 ? nullptr : xdev;
@@ -2159,7 +2011,7 @@ void kmeanspp(const T *X, i64 N, i64 D, i64 K, T *centers, i64 x0, const std::ve
       case 2: launch_kpp_update<T, 2>(X, N, D, xp, x0, centers + c * D, minDist, s); break;
       default: launch_kpp_update<T, 1>(X, N, D, xp, x0, centers + c * D, minDist, s); break;
     }
-    VLB_LAUNCH("kpp_select", s, k_kpp_select<T><<<1, kKppThreads, ssmem, s>>>(minDist, N, thresh[c], ck, xdev));
+    VLB_LAUNCH("kpp_select", s, k_kpp_select<T><<<1, kSeqThreads, ssmem, s>>>(minDist, N, thresh[c], ck, xdev));
   }
 }
 
