@@ -200,19 +200,29 @@ __global__ void __launch_bounds__(16 * NC, 2) k_pca_project(const PcaParams p) {
 //    [2^14, 2^15)), P by 2^g (one g: max |P| into [2^14, 2^15)); the epilogue
 //    undoes both exactly, so fp16's range holds any input and each operand
 //    keeps 22 significant bits;
-//  - roles: warps 0-7 producers (16 rows each; a lane converts 4 dimensions of
+//  - roles: warps 0-15 producers (8 rows each; a lane converts 4 dimensions of
 //    a row: coalesced 512-byte row loads, a warp max for the row's scale, the
-//    hi/lo split, stores into the K-major 64-byte-swizzled A tile), warps 8-11
+//    hi/lo split, stores into the K-major 64-byte-swizzled A tile), warps 16-19
 //    epilogue (one row per thread: TMEM -> scale -> renormalisation -> 'xy'
-//    -> store), warp 12 TMEM allocation and the MMA issue;
+//    -> store), warp 20 TMEM allocation and the MMA issue, warp 21 the frames'
+//    positions;
 //  - two A stages and two TMEM accumulators of np columns; P's image stays in
-//    shared memory for the CTA's life.
-constexpr int kPtThreads = 416;
+//    shared memory for the CTA's life;
+//  - an output tile is one contiguous piece of memory: where shared memory has
+//    room an epilogue warp forms its 32 rows there and one bulk copy writes
+//    them, while the next tile is multiplied.  A thread storing its own row touched a sector per
+//    lane and instruction (2.5 M descriptors, 128 to 80 + xy: 0.80 ms with rows
+//    stored by their threads, 0.58 staged, 0.45 with the producers' loads behind an
+//    L2 prefetch and the frames in a warp of their own; HBM's rate gives 0.32).
+constexpr int kPtEpi = 16;  // first epilogue warp, behind the producers; then the MMA warp and the frames' warp
+constexpr int kPtRows = 128 / kPtEpi;  // rows per producer warp
+constexpr int kPtMma = kPtEpi + 4, kPtXy = kPtMma + 1, kPtThreads = 32 * (kPtXy + 1);
 
 struct PcaTcParams {
   float *out;
   int ldo, din, dout, renorm, nka, np, vec_out;  // vec_out: 4, 2 or 1 floats per store
   int vec_xy;                                    // frames and xy outputs as float2
+  int staged;  // output rows go through shared memory: 32 of a warp at a time (1), 16 (2), or not (0)
   i64 N, nimg, ntiles;
   const float *X, *P, *c, *frames, *sizes;
   const i64 *offs;
@@ -221,11 +231,12 @@ struct PcaTcParams {
 
 // Dynamic shared memory from a 1024-aligned base: A stages (2 x nka x 16 KB:
 // hi atoms then lo atoms), P image (hi nka x np x 64 B, then lo), control
-// block (barriers, flags, row exponents, the image of each stage's first row).
+// block (barriers, flags, row exponents), then the staged output tile.
 __host__ __device__ inline size_t pt_a_bytes(int nka) { return (size_t)2 * nka * 16384; }
 __host__ __device__ inline size_t pt_p_bytes(int nka, int np) { return (size_t)nka * np * 128; }
-constexpr size_t kPtCtl = 128 + 2 * 128 * sizeof(int) + 16;
-__host__ inline size_t pt_smem(int nka, int np) { return 1024 + pt_a_bytes(nka) + pt_p_bytes(nka, np) + kPtCtl; }
+constexpr size_t kPtCtl = 256 + 2 * 128 * (sizeof(int) + sizeof(float2));
+constexpr size_t kPtCtlPad = (kPtCtl + 127) / 128 * 128;
+__host__ inline size_t pt_smem(int nka, int np) { return 1024 + pt_a_bytes(nka) + pt_p_bytes(nka, np) + kPtCtlPad; }
 
 __device__ __forceinline__ float pow2f(int e) {  // 2^e for e in [-126, 127]
   return __int_as_float((e + 127) << 23);
@@ -247,17 +258,23 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
   volatile int *s_abort = (volatile int *)(full + 6);
   uint32_t *s_tmem = (uint32_t *)(full + 7);
   int *s_g = (int *)(full + 8);
-  float *s_red = (float *)(full + 9);     // 13 warp maxima (up to full + 16)
-  int *sexp = (int *)(ctl + 128);         // [2][128] row exponents
-  i64 *timg = (i64 *)(ctl + 128 + 2 * 128 * sizeof(int));  // [2] image of each stage's first row
+  float *s_red = (float *)(full + 9);     // 22 warp maxima (up to full + 20)
+  int *sexp = (int *)(ctl + 256);         // [2][128] row exponents
+  float2 *s_xy = (float2 *)(sexp + 256);  // [2][128] positions of the tiles' frames
+  uint64_t *xyf = full + 22, *xye = full + 24;  // [2] each: written (32 arrivals), read (128)
+  float *s_out = (float *)(ctl + kPtCtlPad);  // staged: the tile's outputs, [128][ldo]
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   if (tid == 0) {
-    mbar_init(&full[0], 256);
-    mbar_init(&full[1], 256);
+    mbar_init(&full[0], 32 * kPtEpi);
+    mbar_init(&full[1], 32 * kPtEpi);
     mbar_init(&accf[0], 1);
     mbar_init(&accf[1], 1);
     mbar_init(&acce[0], 128);
     mbar_init(&acce[1], 128);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&xyf[b], 32);
+      mbar_init(&xye[b], 128);
+    }
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -267,8 +284,8 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
   for (int e = tid; e < nP; e += kPtThreads) mx = fmaxf(mx, fabsf(__ldg(p.P + e)));
   mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
   if (lane == 0) s_red[warp] = mx;
-  if (warp == 12) tmem_alloc(s_tmem, 256);
-  if (warp == 12) tmem_relinquish();
+  if (warp == kPtMma) tmem_alloc(s_tmem, 256);
+  if (warp == kPtMma) tmem_relinquish();
   __syncthreads();
   if (tid == 0) {
     float m = 0.f;
@@ -299,7 +316,7 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  if (warp < 8) {
+  if (warp < kPtEpi) {
     // ------------------------------------------------------- producers
     const int k0 = 4 * lane;
     const bool in = k0 < p.din, pad = k0 < nka * 32;
@@ -309,57 +326,61 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
     const uint32_t chunk = (uint32_t)((lane & 7) >> 1), half8 = (uint32_t)(lane & 1) * 8u;
     int tt = 0;
     // The rows of the next tile are loaded as soon as the current tile's are
-    // converted, before waiting for a free stage, so their latency overlaps
-    // that wait.
-    float4 xv[16];
-    auto load = [&](i64 t) {
-      const i64 r0 = t * 128 + 16 * warp;
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const i64 row = r0 + u;
-        xv[u] = (in && t < p.ntiles && row < p.N) ? __ldg((const float4 *)(p.X + row * p.din + k0))
-                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+    // converted, before waiting for a free stage, and the tile after it is on
+    // its way to L2 by then: the loads wait for L2 and not for HBM.  Rows past
+    // N read as zeros; their outputs are not stored.
+    float4 xv[kPtRows];
+    auto prefetch = [&](i64 t) {
+      if (tid == 0 && t < p.ntiles) {
+        const i64 n = p.N - t * 128 < 128 ? p.N - t * 128 : 128;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.X + t * 128 * p.din), "r"((uint32_t)(n * p.din * 4))
+                     : "memory");
       }
     };
+    auto load = [&](i64 t) {
+      const i64 r0 = t * 128 + kPtRows * warp;
+      const float *src = p.X + r0 * p.din + k0;
+      if (r0 + kPtRows <= p.N) {
+#pragma unroll
+        for (int u = 0; u < kPtRows; ++u) {
+          xv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (in) xv[u] = __ldg((const float4 *)(src + u * p.din));
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < kPtRows; ++u) {
+          xv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (in && r0 + u < p.N) xv[u] = __ldg((const float4 *)(src + u * p.din));
+        }
+      }
+    };
+    prefetch(blockIdx.x + (i64)gridDim.x);
     load(blockIdx.x);
-    i64 pimg = 0;  // image of the previous tile's first row (rows only increase)
     for (i64 t = blockIdx.x; t < p.ntiles; t += gridDim.x, ++tt) {
       const int st = tt & 1;
+      prefetch(t + 2 * (i64)gridDim.x);
       if (tt >= 2 && !mbar_wait(&acce[st], ((tt >> 1) & 1) ^ 1, s_abort, p.err, 11)) break;
-      if (p.frames && tid == 0) {
-        // The last image whose first row is <= the tile's first row: gallop
-        // forward from the previous tile's, then bisect (offs[nimg] = N).
-        const i64 f0 = t * 128;
-        i64 lo = pimg, hi = lo + 1, step = 1;
-        while (hi < p.nimg && __ldg(p.offs + hi) <= f0) {
-          lo = hi;
-          step *= 2;
-          hi = min(p.nimg, lo + step);
-        }
-        while (hi - lo > 1) {
-          const i64 mid = (lo + hi) / 2;
-          if (__ldg(p.offs + mid) <= f0) lo = mid;
-          else hi = mid;
-        }
-        timg[st] = pimg = lo;
-      }
-      const i64 r0 = t * 128 + 16 * warp;
       const uint32_t ahi = a_s + (uint32_t)st * (uint32_t)nka * 16384u, alo = ahi + (uint32_t)nka * 8192u;
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const bool live = in && r0 + u < p.N;
-        const float v0 = live ? __fsub_rn(xv[u].x, cv.x) : 0.f, v1 = live ? __fsub_rn(xv[u].y, cv.y) : 0.f;
-        const float v2 = live ? __fsub_rn(xv[u].z, cv.z) : 0.f, v3 = live ? __fsub_rn(xv[u].w, cv.w) : 0.f;
+      for (int u = 0; u < kPtRows; ++u) {
+        const float v0 = __fsub_rn(xv[u].x, cv.x), v1 = __fsub_rn(xv[u].y, cv.y);
+        const float v2 = __fsub_rn(xv[u].z, cv.z), v3 = __fsub_rn(xv[u].w, cv.w);
         const float m = fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3)));
-        const float rm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-        int e = 0;
-        if (rm > 0.f) frexpf(rm, &e);
-        const int sx = rm > 0.f ? max(-126, min(126, 15 - e)) : 0;
+        // sx = 15 - e with rm = m 2^e, m in [0.5, 1): from the exponent field for
+        // a normal maximum, 0 for zero and NaN, 15 for infinity.
+        const uint32_t rb = __reduce_max_sync(0xffffffffu, __float_as_uint(m)), rx = rb >> 23;
+        int sx = 141 - (int)rx;
+        if (rx == 0u || rx >= 255u) {  // warp-uniform, rare
+          int e = 0;
+          if (rx == 0u && rb) frexpf(__uint_as_float(rb), &e);
+          sx = rb && rb <= 0x7f800000u ? 15 - e : 0;
+        }
+        sx = max(-126, min(126, sx));
         const float f = pow2f(sx);
         uint32_t h0, l0, h1, l1;
         split2<true>(v0 * f, v1 * f, h0, l0);
         split2<true>(v2 * f, v3 * f, h1, l1);
-        const uint32_t rl = (uint32_t)(16 * warp + u);
+        const uint32_t rl = (uint32_t)(kPtRows * warp + u);
         if (pad) {
           const uint32_t off = aoff + kmajor_sw64_off(rl, chunk) + half8;
           st_shared_v2(ahi + off, h0, h1);
@@ -371,19 +392,18 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
       mbar_arrive(&full[st]);
       load(t + gridDim.x);
     }
-  } else if (warp < 12) {
+  } else if (warp < kPtEpi + 4) {
     // -------------------------------------------------------- epilogue
-    const int ew = warp - 8, rl = 32 * ew + lane;
+    const int ew = warp - kPtEpi, rl = 32 * ew + lane;
     const int nch = (np + 31) / 32;
     int tt = 0;
     for (i64 t = blockIdx.x; t < p.ntiles; t += gridDim.x, ++tt) {
       const int buf = tt & 1;
-      if (!mbar_wait(&accf[buf], (tt >> 1) & 1, s_abort, p.err, 12)) break;
-      tc_fence_after();
       const i64 row = t * 128 + rl;
       const bool valid = row < p.N;
+      if (!__all_sync(0xffffffffu, mbar_wait(&accf[buf], (tt >> 1) & 1, s_abort, p.err, 12))) break;
+      tc_fence_after();
       const int sx = sexp[buf * 128 + rl];
-      const i64 img0 = p.frames ? timg[buf] : 0;  // read before the stage is released below
       // acc 2^-(s + g).  The combined exponent e is applied as 2^e1 2^(e - e1)
       // with e1 the part within a float's normal range: the second factor is 1
       // unless |e| > 126, and the first product cannot overflow (or leave the
@@ -392,6 +412,8 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
       const int e = -(sx + g), e1 = e > 126 ? 126 : (e < -126 ? -126 : e);
       const float f1 = pow2f(e1), f2 = pow2f(e - e1);
       const uint32_t taddr = tmem + (uint32_t)(buf * 128) + ((uint32_t)(32 * ew) << 16);
+      const bool one = __all_sync(0xffffffffu, f2 == 1.f);  // f2 leaves every value as it is
+      auto scaled = [&](uint32_t v) { return one ? __uint_as_float(v) * f1 : __uint_as_float(v) * f1 * f2; };
       float inv = 1.f;
       if (p.renorm) {
         float ss = 0.f;
@@ -401,64 +423,150 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
           tmem_wait_ld();
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            const float y = __uint_as_float(v[j]) * f1 * f2;
+            const float y = scaled(v[j]);
             if (ch * 32 + j < p.dout) ss = __fmaf_rn(y, y, ss);
           }
         }
         inv = 1.f / fmaxf(1e-12f, sqrtf(ss));
       }
-      float *o = p.out + row * p.ldo;
-      for (int ch = 0; ch < nch; ++ch) {
-        uint32_t v[32];
-        tmem_ld32(taddr + (uint32_t)(ch * 32), v);
-        tmem_wait_ld();
-        if (!valid) continue;
-        const int j0 = ch * 32;
-        if (p.vec_out == 4) {
+      float2 xy = make_float2(0.f, 0.f);
+      if (p.frames) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&xyf[buf], (tt >> 1) & 1, s_abort, p.err, 15))) break;
+        xy = s_xy[buf * 128 + rl];
+        mbar_arrive(&xye[buf]);
+      }
+      // The warp's 32 rows at once, or in two halves through a staging buffer
+      // of 16.
+      const int parts = p.staged == 2 ? 2 : 1, prow = 32 / parts;
+      float *stg = s_out + ew * prow * p.ldo;
+      for (int h = 0; h < parts; ++h) {
+        const bool mine = valid && lane / prow == h;
+        if (p.staged) {
+          // The warp's last copy has read the staging buffer.
+          if (lane == 0) bulk_wait_read<0>();
+          __syncwarp();
+        }
+        float *o = p.staged ? stg + lane % prow * p.ldo : p.out + row * p.ldo;
+        for (int ch = 0; ch < nch; ++ch) {
+          uint32_t v[32];
+          tmem_ld32(taddr + (uint32_t)(ch * 32), v);
+          tmem_wait_ld();
+          if (!mine) continue;
+          const int j0 = ch * 32;
+          if (p.vec_out == 4) {
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            if (j0 + 4 * q < p.dout) {
-              float4 w;
-              w.x = __uint_as_float(v[4 * q]) * f1 * f2 * inv;
-              w.y = __uint_as_float(v[4 * q + 1]) * f1 * f2 * inv;
-              w.z = __uint_as_float(v[4 * q + 2]) * f1 * f2 * inv;
-              w.w = __uint_as_float(v[4 * q + 3]) * f1 * f2 * inv;
-              *(float4 *)(o + j0 + 4 * q) = w;
+            for (int q = 0; q < 8; ++q) {
+              if (j0 + 4 * q < p.dout) {
+                float4 w;
+                w.x = scaled(v[4 * q]) * inv;
+                w.y = scaled(v[4 * q + 1]) * inv;
+                w.z = scaled(v[4 * q + 2]) * inv;
+                w.w = scaled(v[4 * q + 3]) * inv;
+                *(float4 *)(o + j0 + 4 * q) = w;
+              }
             }
-          }
-        } else if (p.vec_out == 2) {
+          } else if (p.vec_out == 2) {
 #pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            if (j0 + 2 * q < p.dout) {
-              float2 w;
-              w.x = __uint_as_float(v[2 * q]) * f1 * f2 * inv;
-              w.y = __uint_as_float(v[2 * q + 1]) * f1 * f2 * inv;
-              *(float2 *)(o + j0 + 2 * q) = w;
+            for (int q = 0; q < 16; ++q) {
+              if (j0 + 2 * q < p.dout) {
+                float2 w;
+                w.x = scaled(v[2 * q]) * inv;
+                w.y = scaled(v[2 * q + 1]) * inv;
+                *(float2 *)(o + j0 + 2 * q) = w;
+              }
             }
-          }
-        } else {
+          } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j0 + j < p.dout) o[j0 + j] = __uint_as_float(v[j]) * f1 * f2 * inv;
+            for (int j = 0; j < 32; ++j)
+              if (j0 + j < p.dout) o[j0 + j] = scaled(v[j]) * inv;
+          }
+        }
+        if (h == parts - 1) {
+          tc_fence_before();
+          mbar_arrive(&acce[buf]);
+        }
+        if (p.frames && mine) {
+          if (p.vec_xy) {
+            *(float2 *)(o + p.dout) = xy;
+          } else {
+            o[p.dout] = xy.x;
+            o[p.dout + 1] = xy.y;
+          }
+        }
+        if (p.staged) {
+          fence_proxy_async_smem();  // this thread's staging writes, before the copy reads them
+          __syncwarp();
+          const i64 w0 = t * 128 + 32 * ew + h * prow;  // the first row staged
+          const int nr = (int)max((i64)0, min((i64)prow, p.N - w0)), nf = nr * p.ldo;
+          const float *src = stg;
+          float *dst = p.out + w0 * p.ldo;
+          if (lane == 0 && nf >= 4) {
+            bulk_s2g(dst, smem_u32(src), (uint32_t)(nf / 4 * 16));
+            bulk_commit();
+          }
+          if (lane < nf % 4) dst[nf / 4 * 4 + lane] = src[nf / 4 * 4 + lane];  // the last rows' odd end
         }
       }
-      tc_fence_before();
-      mbar_arrive(&acce[buf]);
-      if (p.frames && valid) {
-        // Forward from the image of the tile's first row.
-        i64 img = img0;
-        while (img + 1 < p.nimg && __ldg(p.offs + img + 1) <= row) ++img;
-        if (p.vec_xy) {
-          const float2 fr = __ldg((const float2 *)(p.frames + 2 * row));
-          const float2 sz = __ldg((const float2 *)(p.sizes + 2 * img));
-          *(float2 *)(o + p.dout) = make_float2((fr.x - sz.x * 0.5f) * (1.f / sz.x), (fr.y - sz.y * 0.5f) * (1.f / sz.y));
+    }
+    // The last copy completes before the block exits.
+    if (p.staged && lane == 0) bulk_wait_all();
+  } else if (warp == kPtXy) {
+    // ---------------------------------------------------------- frames
+    // Positions of the tile's frames, up to two tiles ahead of the epilogue (in
+    // its own time the search cost 0.18 ms of 0.59).  The warp keeps the last
+    // image whose first row is <= the tile's first row and probes the next 32
+    // images' first rows at once; those inside the tile tell its rows apart.
+    if (p.frames) {
+      i64 img = 0;
+      int tt = 0;
+      auto probe = [&](i64 stride) {
+        const i64 i = img + (lane + 1) * stride;
+        return i < p.nimg ? __ldg(p.offs + i) : INT64_MAX;
+      };
+      for (i64 t = blockIdx.x; t < p.ntiles; t += gridDim.x, ++tt) {
+        const int buf = tt & 1;
+        const i64 r0 = t * 128;
+        i64 o = probe(1);
+        int c = __popc(__ballot_sync(0xffffffffu, o <= r0));  // first rows do not decrease
+        if (c == 32) {
+          for (i64 stride = 1024; stride >= 1; stride /= 32)
+            do {
+              o = probe(stride);
+              c = __popc(__ballot_sync(0xffffffffu, o <= r0));
+              img += c * stride;
+            } while (c == 32);
+          o = probe(1);
+          c = 0;
         } else {
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const float sz = __ldg(p.sizes + 2 * img + i);
-            o[p.dout + i] = (__ldg(p.frames + 2 * row + i) - sz * 0.5f) * (1.f / sz);
-          }
+          img += c;
         }
+        // Lanes c .. 31 hold the first rows of images img + 1, img + 2, ...
+        const unsigned inside = __ballot_sync(0xffffffffu, o <= r0 + 127) & ~((1u << c) - 1u);
+        i64 im[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const i64 row = r0 + 32 * q + lane;
+          im[q] = img;
+          for (unsigned m = inside; m; m &= m - 1)
+            if (__shfl_sync(0xffffffffu, o, __ffs(m) - 1) <= row) ++im[q];
+          if (inside >> 31)  // the probe may not reach the tile's last image
+            while (im[q] + 1 < p.nimg && __ldg(p.offs + im[q] + 1) <= row) ++im[q];
+        }
+        float fx[4], fy[4], sx[4], sy[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const i64 row = min(r0 + 32 * q + lane, p.N - 1);
+          fx[q] = __ldg(p.frames + 2 * row);
+          fy[q] = __ldg(p.frames + 2 * row + 1);
+          sx[q] = __ldg(p.sizes + 2 * im[q]);
+          sy[q] = __ldg(p.sizes + 2 * im[q] + 1);
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(&xye[buf], ((tt >> 1) & 1) ^ 1, s_abort, p.err, 16))) break;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          s_xy[buf * 128 + 32 * q + lane] =
+              make_float2((fx[q] - sx[q] * 0.5f) * (1.f / sx[q]), (fy[q] - sy[q] * 0.5f) * (1.f / sy[q]));
+        mbar_arrive(&xyf[buf]);
       }
     }
   } else if (lane == 0) {
@@ -490,7 +598,7 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 12) {
+  if (warp == kPtMma) {
     tc_fence_after();
     tmem_dealloc(tmem, 256);
   }
@@ -641,7 +749,12 @@ void pca_project(float *out, i64 ldo, const float *X, i64 din, i64 N, i64 dout, 
     q.vec_xy = (frames && (uintptr_t)frames % 8 == 0 && (uintptr_t)sizes % 8 == 0 && ldo % 2 == 0 &&
                 dout % 2 == 0 && (uintptr_t)out % 8 == 0) ? 1 : 0;
     q.X = X; q.P = P; q.c = c; q.frames = frames; q.sizes = sizes; q.offs = doffs; q.err = derr;
-    const size_t smem = pt_smem(q.nka, q.np);
+    // Output tiles through shared memory where it has room (a bulk copy wants a
+    // 16-byte aligned output; tiles of 128 rows then all start on one).
+    size_t smem = pt_smem(q.nka, q.np);
+    const size_t stage = sizeof(float) * 128 * (size_t)ldo;
+    q.staged = (uintptr_t)out % 16 != 0 ? 0 : smem + stage <= 232448 ? 1 : smem + stage / 2 <= 232448 ? 2 : 0;
+    if (q.staged) smem += stage / q.staged;
     const int grid = (int)std::min<i64>(q.ntiles, (i64)sm_count());
     VLB_CUDA(cudaFuncSetAttribute(k_pca_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     VLB_LAUNCH("pca_project_tc", s, k_pca_tc<<<grid, kPtThreads, smem, s>>>(q));
