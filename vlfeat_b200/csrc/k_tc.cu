@@ -1022,7 +1022,8 @@ struct SParams {
   const uint8_t *qimg;  // q^T operand image written by the E-step
   i64 qpart;            // bytes of one image part
   i64 qbase;            // row of X that the image's first row corresponds to
-  int K, Kp, Kq, nst;
+  int K, Kp, Kq;
+  int nx, nq, no;  // ring depths
   const float *ctr;
   const float *scale;  // per-dimension scale of x' (fp16 operands), or null
   const SItem *items;
@@ -1048,35 +1049,83 @@ struct SLayout {
   static constexpr int A_PART = MT * 4 * 4 * 512;      // [mnblk 4MT][kgroup 4][512 B atom]
   static constexpr int B_PART = NB * 4 * 1024;         // [kgroup 4][nblk NB][1 KB]
   static constexpr int XST = (32 * DIM * 4 + 1023) / 1024 * 1024;  // staged x rows
-  static constexpr int kStage = NPA * A_PART + NPB * B_PART + XST;
+  // Three rings, each freed by the step that reads it: the copied x rows (by
+  // the converters), the x-side operands made from them and the copied q^T (by
+  // the MMA).  Depths are handed out in turn while they fit.
+  static constexpr int kQ = NPA * A_PART, kOp = NPB * B_PART;
   static constexpr size_t fixed = 1024 /*ctr*/ + 1024 /*scale*/ + 1024 /*bars*/ + 1024;
-  static int max_stages() { return (int)((kSmemLimit - fixed) / kStage); }
-  static size_t bytes(int nst) { return fixed + (size_t)nst * kStage; }
+  struct Depth {
+    int x, q, op;
+  };
+  static constexpr Depth depth() {
+    const int room = (int)(kSmemLimit - fixed);
+    if (FS) {  // even rings for the two converter groups
+      Depth r{4, 2, 4};
+      while (r.q < 8 && r.x * XST + (r.q + 1) * kQ + r.op * kOp <= room) ++r.q;
+      return r;
+    }
+    Depth r{2, 2, 2};
+    for (int t = 3; t <= 6; ++t) {
+      if ((r.x + 1) * XST + r.q * kQ + r.op * kOp <= room) ++r.x;
+      if (r.x * XST + (r.q + 1) * kQ + r.op * kOp <= room) ++r.q;
+      if (r.x * XST + r.q * kQ + (r.op + 1) * kOp <= room) ++r.op;
+    }
+    return r;
+  }
+  static constexpr int NX = depth().x, NQ = depth().q, NO = depth().op;
+  static constexpr size_t bytes = fixed + (size_t)NX * XST + (size_t)NQ * kQ + (size_t)NO * kOp;
+  static_assert(NX * XST + NQ * kQ + NO * kOp <= (int)(kSmemLimit - fixed), "operands exceed shared memory");
   static_assert(MT * NF <= 512, "accumulators exceed TMEM");
 };
 
-// Statistics block: converter warps 0-3 and 10-13, epilogue warps 4-7, MMA
-// warp 8, loader warp 9.
-constexpr int kStatsThreads = 448;
-constexpr int kStatsConv = 256;  // converter threads
-// With the features split, the converter warps work in two groups, each on its
-// own stages (stage mod 2, so that a group sees every phase of its stages'
-// barriers): a chunk's conversion is a chain of a wait, shared-memory reads,
-// stores, a proxy fence and an arrival, and the groups run theirs side by side
-// (one item of 3,000 rows, K = 256, D = 80: 75 us with one group, 62 with two).  With all features in one CTA two groups were 3% slower.
-__host__ __device__ constexpr int stats_groups(int fs) { return fs ? 2 : 1; }
+// Statistics block: converter warps 0-3 and 10-15, epilogue warps 4-7, MMA
+// warp 8, loader warps 9 (x rows) and 16 (q^T).
+constexpr int kStatsConv = 320;  // converter threads
+constexpr int kStatsThreads = kStatsConv + 224;
+constexpr int kStatsLastWarp = kStatsThreads / 32 - 1;
+__host__ __device__ constexpr int stats_groups(int fs) { return fs ? 2 : 1; }  // converter groups
+
+// A position in a ring of n buffers, each with a pair of barriers.
+struct Ring {
+  int n, i = 0;
+  uint32_t phase = 0;
+  __device__ explicit Ring(int n_) : n(n_) {}
+  __device__ void next() {
+    if (++i == n) {
+      i = 0;
+      phase ^= 1;
+    }
+  }
+};
+
+// After an abandoned run of copies: waits (with a limit) for the last ones, of
+// which up to n are in flight, `issued` in all.
+__device__ __forceinline__ void drain_copies(uint64_t *full, int n, int issued, int *err, int code) {
+  int never = 0;
+  for (int j = issued - 1; j >= 0 && j >= issued - n; --j)
+    mbar_wait(&full[j % n], (uint32_t)((j / n) & 1), &never, err, code);
+}
 
 // Statistics over work items (runs of rows of one image): for each 32-row
-// chunk, the loader warp bulk-copies the chunk's q^T operand (four 8-row
-// groups of the E-step's image) straight into the operand stage and the
-// chunk's x rows into a staging buffer; converter warps build the x-side
-// operand [x'', x''^2, 1] (zero rows outside the item); one thread issues the
-// MMAs; the epilogue drains the item's accumulators to its partial.
+// chunk, two loader warps copy its x rows and its q^T operand (four 8-row
+// groups of the E-step's image); converter warps build the x-side operand
+// [x'', x''^2, 1] (zero rows outside the item); one thread issues the MMAs; the
+// epilogue drains the item's accumulators to its partial.
+//
+// A chunk is a chain of copy, conversion (a wait, shared-memory reads, stores, a
+// proxy fence, an arrival) and MMAs, so what bounds it is how many chunks are in
+// each step at a time.  With one stage of shared memory held by a chunk from its
+// copy to its MMAs, two or three fitted; with a ring for each step, three or
+// four of each do.  Statistics of 1,024 images, K = 256, ms, before and after:
+// D = 80 FP32 1.31, 1.21; D = 80 BF16 1.01, 0.91; 512 images, D = 128: 1.20,
+// 1.15; 2.5 M rows padded to 96: 0.83, 0.63.  With 256 converter threads
+// 1.21, 0.97, 1.19 and 0.62, with 384 1.22, 0.91, 1.12 and 0.64; in two groups
+// on alternate chunks 1.32, 1.08, 1.29 and 0.68.
 // FS (features per CTA, blockIdx.z the part): with few items, as for one image,
 // the CTAs of an item's row run split the features too.  Each accumulator sees
 // the same products in the same order (the same bits), and a CTA's chunk takes
-// a quarter of the MMA and conversion time, so that the item's chain of chunks
-// runs at the copies' latency over six stages instead of three.
+// a quarter of the MMA and conversion time; here the converters do work in two
+// groups (one item of 3,000 rows, K = 256, D = 80: 75 us with one, 62 with two).
 template <int DIM, int MT, int SPLIT, int FS>
 __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_constant__ SParams p) {
   using L = SLayout<DIM, MT, SPLIT, FS>;
@@ -1087,11 +1136,14 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
   constexpr int NF4 = DIM / 4;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *base = align1024(smem_raw);
-  uint8_t *sS = base;
-  float *s_ctr = (float *)(sS + (size_t)p.nst * L::kStage);
+  uint8_t *sB = base;                   // x-side operands
+  uint8_t *sQ = sB + L::NO * L::kOp;    // copied q^T
+  uint8_t *sX = sQ + L::NQ * L::kQ;     // copied x rows
+  float *s_ctr = (float *)(sX + L::NX * L::XST);
   float *s_scl = s_ctr + 256;
   uint64_t *bars = (uint64_t *)(s_scl + 256);
-  uint64_t *full = bars, *empty = bars + 16, *xfull = bars + 32, *accf = bars + 48, *acce = bars + 49;
+  uint64_t *xfull = bars, *xempty = bars + 8, *qfull = bars + 16, *qempty = bars + 24;
+  uint64_t *full = bars + 32, *empty = bars + 40, *accf = bars + 48, *acce = bars + 49;
   uint32_t *s_tmem = (uint32_t *)(bars + 56);
   volatile int *s_abort = (volatile int *)(s_tmem + 1);
 
@@ -1099,10 +1151,17 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int comp0 = blockIdx.y * MT * 128;  // first component of this CTA's M tiles
   if (tid == 0) {
-    for (int s = 0; s < p.nst; ++s) {
+    for (int s = 0; s < p.nx; ++s) {
+      mbar_init(&xfull[s], 1);
+      mbar_init(&xempty[s], TG);
+    }
+    for (int s = 0; s < p.nq; ++s) {
+      mbar_init(&qfull[s], 1);
+      mbar_init(&qempty[s], 1);
+    }
+    for (int s = 0; s < p.no; ++s) {
       mbar_init(&full[s], TG);
       mbar_init(&empty[s], 1);
-      mbar_init(&xfull[s], 1);
     }
     mbar_init(accf, 1);
     mbar_init(acce, 128);
@@ -1117,12 +1176,8 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
     s_ctr[d] = p.ctr[d];
     s_scl[d] = p.scale ? p.scale[d] : 1.f;
   }
-  // Zero the operand stages once: groups a chunk does not copy keep finite
-  // stale values, and their x-side rows are zero.
-  for (int s = 0; s < p.nst; ++s) {
-    uint4 *st = (uint4 *)(sS + (size_t)s * L::kStage);
-    for (int i = tid; i < (NPA * L::A_PART + L::NPB * L::B_PART) / 16; i += kStatsThreads) st[i] = make_uint4(0, 0, 0, 0);
-  }
+  // Zero the operand slots once: the columns that no chunk writes stay zeros.
+  for (int i = tid; i < L::NO * L::kOp / 16; i += kStatsThreads) ((uint4 *)sB)[i] = make_uint4(0, 0, 0, 0);
   fence_proxy_async_smem();
   __syncthreads();
   tc_fence_after();
@@ -1130,50 +1185,75 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
   const int ib = p.cta_beg[blockIdx.x], ie = p.cta_beg[blockIdx.x + 1];
 
   if (warp == 9) {
-    // ------------------------------------------------------- loader
+    // ------------------------------------------------ loader of x rows
     if (lane == 0) {
+      Ring rx(p.nx);
       int it = 0;
       bool ok = true;
       for (int ii = ib; ii < ie && ok; ++ii) {
         const SItem item = p.items[p.order[ii]];
         for (i64 cb = p.qbase + ((item.row0 - p.qbase) & ~(i64)7); cb < item.row1; cb += 32) {
-          const int stage = it % p.nst;
-          if (!mbar_wait(&empty[stage], ((it / p.nst) & 1) ^ 1, s_abort, p.err, 15)) {
+          if (!mbar_wait(&xempty[rx.i], rx.phase ^ 1, s_abort, p.err, 15)) {
             ok = false;
             break;
           }
-          const uint32_t sa = smem_u32(sS + (size_t)stage * L::kStage);
-          const uint32_t sx = sa + NPA * L::A_PART + L::NPB * L::B_PART;
-          const int nx = (int)min((i64)32, item.row1 - cb);
-          mbar_arrive_expect_tx(&xfull[stage], (uint32_t)(NPA * L::A_PART) + (uint32_t)(nx * p.ldx * 4));
+          const uint32_t nb = (uint32_t)((int)min((i64)32, item.row1 - cb) * p.ldx * 4);
+          mbar_arrive_expect_tx(&xfull[rx.i], nb);
+          bulk_g2s(smem_u32(sX + rx.i * L::XST), p.X + cb * p.ldx, nb, &xfull[rx.i]);
+          rx.next();
+          ++it;
+        }
+      }
+      if (!ok) drain_copies(xfull, p.nx, it, p.err, 15);
+    }
+  } else if (warp == kStatsLastWarp) {
+    // ----------------------------------------------------- loader of q^T
+    if (lane == 0) {
+      Ring rq(p.nq);
+      int it = 0;
+      bool ok = true;
+      for (int ii = ib; ii < ie && ok; ++ii) {
+        const SItem item = p.items[p.order[ii]];
+        for (i64 cb = p.qbase + ((item.row0 - p.qbase) & ~(i64)7); cb < item.row1; cb += 32) {
+          if (!mbar_wait(&qempty[rq.i], rq.phase ^ 1, s_abort, p.err, 18)) {
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(&qfull[rq.i], (uint32_t)L::kQ);
           // q^T for the chunk: groups (cb - qbase) / 8 .. +3 of this CTA's
           // 4 MT blocks, all parts, as one box laid out [part][block][group]
           // (groups past the image read as zero; groups past the item are
           // finite and meet zero x-side rows).
-          tma_load_4d(sa, &p.qmap, 0, (int)((cb - p.qbase) >> 3), comp0 / 32, 0, &xfull[stage]);
-          bulk_g2s(sx, p.X + cb * p.ldx, (uint32_t)(nx * p.ldx * 4), &xfull[stage]);
+          tma_load_4d(smem_u32(sQ + rq.i * L::kQ), &p.qmap, 0, (int)((cb - p.qbase) >> 3), comp0 / 32, 0, &qfull[rq.i]);
+          rq.next();
           ++it;
         }
       }
+      if (!ok) drain_copies(qfull, p.nq, it, p.err, 18);
     }
-  } else if (warp < 4 || warp >= 10) {
+  } else if (warp < 4 || (warp >= 10 && warp < kStatsLastWarp)) {
     // ---------------------------------------------------- converters
     const int cw = warp < 4 ? warp : warp - 6;  // converter warp
-    const int ctid = (cw % (8 / G)) * 32 + lane, group = cw / (8 / G);
+    constexpr int WG = kStatsConv / 32 / G;  // warps of a group
+    const int ctid = (cw % WG) * 32 + lane, group = cw / WG;
+    Ring rx(p.nx), ro(p.no);
     int it = -1;
     bool ok = true;
     for (int ii = ib; ii < ie && ok; ++ii) {
       const SItem item = p.items[p.order[ii]];
       for (i64 cb = p.qbase + ((item.row0 - p.qbase) & ~(i64)7); cb < item.row1; cb += 32) {
-        const int stage = ++it % p.nst;
-        if (G > 1 && stage % G != group) continue;
-        if (!mbar_wait(&xfull[stage], (it / p.nst) & 1, s_abort, p.err, 11)) {
+        if (it >= 0) {
+          rx.next();
+          ro.next();
+        }
+        if (++it % G != group) continue;  // rings are multiples of G: a group sees every phase of its barriers
+        if (!mbar_wait(&empty[ro.i], ro.phase ^ 1, s_abort, p.err, 17) ||
+            !mbar_wait(&xfull[rx.i], rx.phase, s_abort, p.err, 11)) {
           ok = false;
           break;
         }
-        const uint32_t sa = smem_u32(sS + (size_t)stage * L::kStage);
-        const uint32_t sb = sa + NPA * L::A_PART;
-        const float *xs = (const float *)(sS + (size_t)stage * L::kStage + NPA * L::A_PART + L::NPB * L::B_PART);
+        const uint32_t sb = smem_u32(sB + ro.i * L::kOp);
+        const float *xs = (const float *)(sX + rx.i * L::XST);
         if constexpr (FS == 0) {
 #pragma unroll
           for (int j = 0; j < (32 * NF4 + TG - 1) / TG; ++j) {
@@ -1254,7 +1334,8 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
           }
         }
         fence_proxy_async_smem();
-        mbar_arrive(&full[stage]);
+        mbar_arrive(&xempty[rx.i]);
+        mbar_arrive(&full[ro.i]);
       }
     }
   } else if (warp < 8) {
@@ -1294,7 +1375,8 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
     }
   } else if (warp == 8 && lane == 0) {
     // ---------------------------------------------------------- MMA
-    int it = 0, n = 0;
+    Ring rq(p.nq), ro(p.no);
+    int n = 0;
     bool ok = true;
     for (int ii = ib; ii < ie && ok; ++ii, ++n) {
       const SItem item = p.items[p.order[ii]];
@@ -1302,15 +1384,14 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
       tc_fence_after();
       int chunk = 0;
       for (i64 cb = p.qbase + ((item.row0 - p.qbase) & ~(i64)7); cb < item.row1; cb += 32, ++chunk) {
-        const int stage = it % p.nst;
-        if (!mbar_wait(&full[stage], (it / p.nst) & 1, s_abort, p.err, 14) ||
-            !mbar_wait(&xfull[stage], (it / p.nst) & 1, s_abort, p.err, 16)) {
+        if (!mbar_wait(&full[ro.i], ro.phase, s_abort, p.err, 14) ||
+            !mbar_wait(&qfull[rq.i], rq.phase, s_abort, p.err, 16)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t sa = smem_u32(sS + (size_t)stage * L::kStage);
-        const uint32_t sb = sa + NPA * L::A_PART;
+        const uint32_t sa = smem_u32(sQ + rq.i * L::kQ);
+        const uint32_t sb = smem_u32(sB + ro.i * L::kOp);
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
 #pragma unroll
@@ -1333,8 +1414,10 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
             }
           }
         }
-        mma_commit(&empty[stage]);
-        ++it;
+        mma_commit(&empty[ro.i]);
+        mma_commit(&qempty[rq.i]);
+        rq.next();
+        ro.next();
       }
       if (ok) mma_commit(accf);
     }
@@ -1837,10 +1920,13 @@ template <int DIM, int MT, int SPLIT, int FS = 0>
 void launch_stats(const SParams &p0, int grid_x, int grid_y, int nst_req, cudaStream_t s) {
   using L = SLayout<DIM, MT, SPLIT, FS>;
   SParams p = p0;
-  p.nst = std::min(nst_req > 0 ? nst_req : 8, L::max_stages());
-  p.nst -= p.nst % stats_groups(FS);
-  VLB_CHECK(p.nst >= 2, VL_ERR_BAD_ARG, "tensor-core statistics: operands exceed shared memory");
-  const size_t smem = L::bytes(p.nst);
+  const int G = stats_groups(FS);
+  auto ring = [&](int n) { return (nst_req > 0 ? std::min(nst_req, n) : n) / G * G; };
+  p.nx = ring(L::NX);
+  p.nq = nst_req > 0 ? std::min(nst_req, L::NQ) : L::NQ;
+  p.no = ring(L::NO);
+  VLB_CHECK(p.nx >= 2 && p.nq >= 2 && p.no >= 2, VL_ERR_BAD_ARG, "tensor-core statistics: operands exceed shared memory");
+  const size_t smem = L::bytes;
   auto kern = k_tc_stats<DIM, MT, SPLIT, FS>;
   VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   {
@@ -2176,7 +2262,7 @@ void tc_em_stats(const float *X, i64 row0, i64 n, i64 K, i64 D, int split, float
   VLB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   SParams sp;
   sp.X = X; sp.ldx = (int)D; sp.qimg = (const uint8_t *)sc.slot[4].p; sp.qpart = ntiles * 128 * (i64)Kq * 2; sp.qbase = row0;
-  sp.K = (int)K; sp.Kp = Kp; sp.Kq = Kq; sp.nst = 0;
+  sp.K = (int)K; sp.Kp = Kp; sp.Kq = Kq;
   sp.ctr = (const float *)sc.slot[0].p; sp.scale = (const float *)sc.slot[12].p;
   sp.items = ditems; sp.order = dorder; sp.cta_beg = dbeg; sp.partial = partial; sp.err = err;
   stats_dispatch((int)D, split, sp, gx, 0, 0, s);
@@ -2395,7 +2481,7 @@ void fv_run(const FvLayout &L, Scratch &sc, const float *X, const DevModel<float
       }
       SParams sp;
       sp.X = X; sp.ldx = tp.ldx; sp.qimg = (const uint8_t *)q; sp.qpart = ntiles * 128 * (i64)Kq * 2; sp.qbase = c.row0;
-      sp.K = (int)K; sp.Kp = tp.Kp; sp.Kq = Kq; sp.nst = 0;
+      sp.K = (int)K; sp.Kp = tp.Kp; sp.Kq = Kq;
       sp.ctr = tp.ctr; sp.scale = tp.scale;
       sp.items = ditems + c.items; sp.order = dorder + c.items; sp.cta_beg = dbeg + c.beg;
       sp.partial = partial; sp.err = err;
