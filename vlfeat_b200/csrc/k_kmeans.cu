@@ -173,6 +173,7 @@ struct KdBuilder {
 struct KdDev {
   const double *thr, *lb, *ub;
   const int *lower, *upper, *dim, *ent;
+  const int *parent, *leaf;  // of each node (the root's: -1); the leaf that holds each centre
   int numNodes;
 };
 
@@ -417,10 +418,16 @@ __device__ __forceinline__ T warp_row_dist(const T *q, const T *__restrict__ c, 
 // follow vl/heap-def.h: push sifts towards the root while strictly smaller,
 // pop moves the last entry to the root and sifts it towards the smaller
 // child (the right one on ties) while strictly larger.
-template <typename T, int L>
+// KNOWN: the tree is in shared memory and pd holds the row's distance to every
+// centre.
+template <typename T, int L, bool KNOWN = false>
 __device__ int kd_query_warp(const T *q, const T *__restrict__ C, int D, const KdDev &tr, i64 maxComp,
                              double *__restrict__ hk, int *__restrict__ hn, int cap, double &bestOut,
-                             int *__restrict__ err, int lane) {
+                             int *__restrict__ err, int lane, const T *pd = nullptr) {
+  auto ld = [](const auto *p) {
+    if constexpr (KNOWN) return *p;
+    else return __ldg(p);
+  };
   const bool exact = maxComp == 0;
   i64 comps = 0;
   int nh = 1;
@@ -469,12 +476,14 @@ __device__ int kd_query_warp(const T *q, const T *__restrict__ C, int D, const K
     const double dist = pk;
     int n = pn;
     while (true) {
-      const int lc = __ldg(tr.lower + n);
+      const int lc = ld(tr.lower + n);
       if (lc < 0) {  // leaf
-        const int b = -lc - 1, e = -__ldg(tr.upper + n) - 1;
+        const int b = -lc - 1, e = -ld(tr.upper + n) - 1;
         for (int it = b; it < e && (exact || comps < maxComp); ++it) {
-          const int di = __ldg(tr.ent + it);
-          const double dd = (double)warp_row_dist<T, L>(q, C + (i64)di * D, D, lane);
+          const int di = ld(tr.ent + it);
+          double dd;
+          if constexpr (KNOWN) dd = (double)pd[di];
+          else dd = (double)warp_row_dist<T, L>(q, C + (i64)di * D, D, lane);
           ++comps;
           if (!have) {
             have = true;
@@ -487,9 +496,9 @@ __device__ int kd_query_warp(const T *q, const T *__restrict__ C, int D, const K
         }
         break;
       }
-      const int up = __ldg(tr.upper + n);
-      const double xv = (double)q[__ldg(tr.dim + n)];
-      const double x1 = __ldg(tr.lb + n), x2 = __ldg(tr.thr + n), x3 = __ldg(tr.ub + n);
+      const int up = ld(tr.upper + n);
+      const double xv = (double)q[ld(tr.dim + n)];
+      const double x1 = ld(tr.lb + n), x2 = ld(tr.thr + n), x3 = ld(tr.ub + n);
       double delta = __dsub_rn(xv, x2);
       double save = __dadd_rn(dist, __dmul_rn(delta, delta));
       int next, sv;
@@ -585,6 +594,181 @@ __global__ void k_km_ann(const T *__restrict__ X, i64 N, int D, const T *__restr
         if (prev > ndt) {
           dist[x] = ndt;
           assign[x] = (uint32_t)ni;
+        } else {
+          dist[x] = prev;
+        }
+      }
+    }
+  }
+}
+
+// One step of the search from node n towards its children: sv is the child that
+// the search keeps for later, under the returned key, when n's own key is dist.
+__device__ __forceinline__ double kd_far_key(const KdDev &tr, int n, double xv, double dist, int &sv) {
+  const double x1 = tr.lb[n], x2 = tr.thr[n], x3 = tr.ub[n];
+  double delta = __dsub_rn(xv, x2);
+  double save = __dadd_rn(dist, __dmul_rn(delta, delta));
+  if (xv <= x2) {
+    sv = tr.upper[n];
+    if (xv <= x1) {
+      delta = __dsub_rn(xv, x1);
+      save = __dsub_rn(save, __dmul_rn(delta, delta));
+    }
+  } else {
+    sv = tr.lower[n];
+    if (xv > x3) {
+      delta = __dsub_rn(xv, x3);
+      save = __dsub_rn(save, __dmul_rn(delta, delta));
+    }
+  }
+  return save;
+}
+
+// The same assignment for the rows of a list when the budget covers every
+// centre: the near ties that the screen leaves.  A search is a chain of some 500
+// node visits, 250 heap pops and 250 distances by one warp, 0.7 ms at K = 256,
+// D = 80, and a pass over the rows waits for its few listed rows alone.  Here the
+// warp's lanes first compute all K distances of the row side by side.  If one
+// centre is strictly nearest, and on the way from the root to its leaf the key
+// of every branch that the search would put off is below its distance m, then
+// the search visits it for certain: no distance found so far is below m, so
+// none of those branches is pruned, nor does the search stop before it has
+// taken them off the heap.  The nearest of the visited centres is then that one.
+// Otherwise (equal distances, whose order of visits decides; NaN or infinite
+// distances; a key rounded up to m) the search itself runs, on the distances
+// and a copy of the tree in shared memory.
+// 60,001 rows, K = 256, D = 80: 0.70 ms a pass with the search alone, 0.06 here;
+// 12,007 rows of integers 0 to 2, with many equal distances: 0.71 and 0.10.
+template <typename T, int L, bool VEC>
+__global__ void k_km_ties(const T *__restrict__ X, int D, const T *__restrict__ C, int K, KdDev gt, i64 maxComp,
+                          int update, uint32_t *__restrict__ assign, T *__restrict__ dist, int cap,
+                          int *__restrict__ err, const uint32_t *__restrict__ list, i64 count) {
+  extern __shared__ __align__(16) unsigned char km_smem[];
+  const int WPB = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32, nn = gt.numNodes;
+  double *td = (double *)km_smem;
+  int *ti = (int *)(td + 3 * nn);
+  // The tree's arrays are packed as the host lays them out: three of doubles,
+  // then lower, upper, dim, parent (nodes) and ent, leaf (centres).
+  for (int i = threadIdx.x; i < 3 * nn; i += blockDim.x) td[i] = __ldg(gt.thr + i);
+  for (int i = threadIdx.x; i < 4 * nn + 2 * K; i += blockDim.x) ti[i] = __ldg(gt.lower + i);
+  KdDev tr;
+  tr.thr = td;
+  tr.lb = td + nn;
+  tr.ub = td + 2 * nn;
+  tr.lower = ti;
+  tr.upper = ti + nn;
+  tr.dim = ti + 2 * nn;
+  tr.parent = ti + 3 * nn;
+  tr.ent = ti + 4 * nn;
+  tr.leaf = tr.ent + K;
+  tr.numNodes = nn;
+  __syncthreads();
+  const size_t rowB = align16(sizeof(T) * (size_t)D), distB = align16(sizeof(T) * (size_t)K);
+  const size_t per = align16(rowB + distB + (size_t)cap * (sizeof(double) + sizeof(int)));
+  unsigned char *mine = km_smem + align16(sizeof(double) * 3 * nn + sizeof(int) * (4 * nn + 2 * K)) + per * warp;
+  T *q = (T *)mine, *pd = (T *)(mine + rowB);
+  double *hk = (double *)(mine + rowB + distB);
+  int *hn = (int *)(hk + cap);
+  for (i64 pidx = (i64)blockIdx.x * WPB + warp; pidx < count; pidx += (i64)gridDim.x * WPB) {
+    const i64 x = (i64)list[pidx];
+    __syncwarp();
+    for (int d = lane; d < D; d += 32) q[d] = X[x * D + d];
+    __syncwarp();
+    T m = (T)INFINITY;
+    int mi = -1, ties = 0, odd = 0;  // least distance, its centre, how many have it; NaN or infinite ones
+    for (int c = lane; c < K; c += 32) {
+      const T *cr = C + (i64)c * D;
+      T acc[L];
+#pragma unroll
+      for (int l = 0; l < L; ++l) acc[l] = (T)0;
+      int i = 0;
+#pragma unroll 4
+      for (; i + L <= D; i += L) {
+        T cg[L];
+        if constexpr (VEC) {
+          constexpr int V = 16 / sizeof(T);
+#pragma unroll
+          for (int u = 0; u < L / V; ++u) {
+            const float4 w = __ldg(reinterpret_cast<const float4 *>(cr + i) + u);
+            const T *wp = reinterpret_cast<const T *>(&w);
+#pragma unroll
+            for (int e = 0; e < V; ++e) cg[u * V + e] = wp[e];
+          }
+        } else {
+#pragma unroll
+          for (int l = 0; l < L; ++l) cg[l] = __ldg(cr + i + l);
+        }
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+          const T dl = sub_rn(q[i + l], cg[l]);
+          acc[l] = add_rn(acc[l], mul_rn(dl, dl));
+        }
+      }
+      T d = lane_sum<T, L>(acc);
+      for (; i < D; ++i) {
+        const T dl = sub_rn(q[i], __ldg(cr + i));
+        d = add_rn(d, mul_rn(dl, dl));
+      }
+      pd[c] = d;
+      odd |= !(d < (T)INFINITY);
+      if (d < m) {
+        m = d;
+        mi = c;
+        ties = 1;
+      } else if (d == m) {
+        ++ties;
+      }
+    }
+    odd = __any_sync(0xffffffffu, odd);
+    T least = m;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const T v = __shfl_xor_sync(0xffffffffu, least, o);
+      least = v < least ? v : least;
+    }
+    const int mine_ties = (mi >= 0 && m == least) ? ties : 0;
+    ties = __reduce_add_sync(0xffffffffu, mine_ties);
+    mi = __reduce_max_sync(0xffffffffu, mine_ties ? mi : -1);
+    __syncwarp();
+    bool sure = !odd && ties == 1;
+    if (sure) {
+      int depth = 0;
+      for (int n = tr.leaf[mi]; n > 0; n = tr.parent[n]) {
+        if (lane == 0) hn[depth] = n;
+        ++depth;
+      }
+      __syncwarp();
+      double key = 0.0;
+      for (int n = 0; depth > 0;) {
+        const int child = hn[--depth];
+        int sv;
+        const double save = kd_far_key(tr, n, (double)q[tr.dim[n]], key, sv);
+        if (child == sv) {
+          if (!(save < (double)least)) {
+            sure = false;
+            break;
+          }
+          key = save;
+        }
+        n = child;
+      }
+      __syncwarp();
+    }
+    T ndt = least;
+    if (!sure) {
+      double nd;
+      mi = kd_query_warp<T, L, true>(q, C, D, tr, maxComp, hk, hn, cap, nd, err, lane, pd);
+      ndt = (T)nd;  // exact: the distance was computed in T
+    }
+    if (lane == 0) {
+      if (!update) {
+        dist[x] = ndt;
+        assign[x] = (uint32_t)mi;
+      } else {
+        const T prev = pd[assign[x]];
+        if (prev > ndt) {
+          dist[x] = ndt;
+          assign[x] = (uint32_t)mi;
         } else {
           dist[x] = prev;
         }
@@ -869,12 +1053,15 @@ struct KMeansRun {
     }
   }
 
-  // Builds the tree over the current centres (reading them back), uploads
-  // it and returns its device view.
-  KdDev tree(const T *centers) {
+  std::vector<T> read_centres(const T *centers) {
     std::vector<T> hc((size_t)(K * D));
     VLB_CUDA(cudaMemcpyAsync(hc.data(), centers, sizeof(T) * K * D, cudaMemcpyDeviceToHost, s));
     VLB_CUDA(cudaStreamSynchronize(s));
+    return hc;
+  }
+
+  // Builds the tree over the centres hc, uploads it and returns its device view.
+  KdDev tree(const std::vector<T> &hc) {
     KdBuilder<T> b{hc.data(), D, rand, {}, {}};
     b.nodes.reserve((size_t)(2 * K));
     b.entries.resize((size_t)K);
@@ -888,7 +1075,7 @@ struct KMeansRun {
     b.bounds(0, sb);
     const i64 nn = (i64)b.nodes.size();
     const size_t dbytes = sizeof(double) * 3 * nn;
-    const size_t ibytes = sizeof(int) * (3 * nn + K);
+    const size_t ibytes = sizeof(int) * (4 * nn + 2 * K);
     std::vector<unsigned char> pack(dbytes + ibytes);
     double *pd = (double *)pack.data();
     int *pi = (int *)(pack.data() + dbytes);
@@ -900,13 +1087,24 @@ struct KMeansRun {
       pi[nn + n] = (int)b.nodes[(size_t)n].upperChild;
       pi[2 * nn + n] = (int)b.nodes[(size_t)n].splitDimension;
     }
-    for (i64 k = 0; k < K; ++k) pi[3 * nn + k] = (int)b.entries[(size_t)k].index;
+    int *parent = pi + 3 * nn, *ent = pi + 4 * nn, *leaf = ent + K;
+    parent[0] = -1;
+    for (i64 k = 0; k < K; ++k) ent[k] = (int)b.entries[(size_t)k].index;
+    for (i64 n = 0; n < nn; ++n) {
+      const KdNode &nd = b.nodes[(size_t)n];
+      if (nd.lowerChild < 0) {
+        for (i64 i = -nd.lowerChild - 1; i < -nd.upperChild - 1; ++i) leaf[ent[i]] = (int)n;
+      } else {
+        parent[nd.lowerChild] = parent[nd.upperChild] = (int)n;
+      }
+    }
     unsigned char *dev = sc.slot[4].get<unsigned char>(pack.size());
     VLB_CUDA(cudaMemcpyAsync(dev, pack.data(), pack.size(), cudaMemcpyHostToDevice, s));
     VLB_CUDA(cudaStreamSynchronize(s));  // pack is a local
     const double *dd = (const double *)dev;
     const int *di = (const int *)(dev + dbytes);
-    return KdDev{dd, dd + nn, dd + 2 * nn, di, di + nn, di + 2 * nn, di + 3 * nn, (int)nn};
+    return KdDev{dd,     dd + nn,     dd + 2 * nn,     di,     di + nn, di + 2 * nn,
+                 di + 4 * nn, di + 3 * nn, di + 4 * nn + K, (int)nn};
   }
 
   double energy(const T *dist) {
@@ -954,6 +1152,41 @@ struct KMeansRun {
       VLB_LAUNCH("km_ann", r.s, (kern<<<(int)blocks, 32 * wpb, smem, r.s>>>(r.X, r.N, (int)r.D, centers, tr, maxComp,
                                                                              update, assign, dist, hk, hn, cap, err,
                                                                              list, count)));
+    }
+  };
+
+  // The screen's near ties: k_km_ties when the tree and one warp's row,
+  // distances and heap fit 200 KB (K up to about 1,700), else the general search.
+  template <typename TT, int L>
+  struct TiesLaunch {
+    static void run(KMeansRun &r, const TT *centers, const KdDev &tr, i64 maxComp, int update, uint32_t *assign,
+                    TT *dist, int *err, const uint32_t *list, i64 count) {
+      const int cap = tr.numNodes;
+      const size_t treeB = align16(sizeof(double) * 3 * cap + sizeof(int) * (4 * (size_t)cap + 2 * (size_t)r.K));
+      const size_t perW = align16(align16(sizeof(TT) * (size_t)r.D) + align16(sizeof(TT) * (size_t)r.K) +
+                                  (size_t)cap * (sizeof(double) + sizeof(int)));
+      const size_t budget = (size_t)200 * 1024;
+      if (treeB + perW > budget) {
+        AnnLaunch<TT, L>::run(r, centers, tr, maxComp, update, assign, dist, err, list, count);
+        return;
+      }
+      const int sms = num_sms();
+      const int wpb = (int)std::min<i64>({(i64)8, (i64)((budget - treeB) / perW), (count + sms - 1) / sms});
+      const i64 blocks = std::min<i64>((count + wpb - 1) / wpb, (i64)sms * 8);
+      const size_t smem = treeB + perW * wpb;
+      auto launch = [&](auto kern) {
+        VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        VLB_LAUNCH("km_ties", r.s, (kern<<<(int)blocks, 32 * wpb, smem, r.s>>>(
+                                       r.X, (int)r.D, centers, (int)r.K, tr, maxComp, update, assign, dist, cap, err,
+                                       list, count)));
+      };
+      if constexpr ((L * sizeof(TT)) % 16 == 0) {
+        if (r.vec(L)) {
+          launch(k_km_ties<TT, L, true>);
+          return;
+        }
+      }
+      launch(k_km_ties<TT, L, false>);
     }
   };
 
@@ -1031,17 +1264,20 @@ struct KMeansRun {
     VLB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
     double energy = INFINITY, prev = INFINITY, initial = INFINITY;
     for (i64 it = 0;; ++it) {
-      const KdDev tr = tree(centers);
+      const std::vector<T> hc = read_centres(centers);
       const int update = it > 0 ? 1 : 0;
-      if (screen) {
+      if (screen) {  // on the device while the host builds the tree
         VLB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s));
         by_lanes<NearestLaunch>(*this, (const T *)centers, (int)kNearestScreen, update, assign, dist, list, cnt);
-        unsigned long long hc = 0;
-        VLB_CUDA(cudaMemcpyAsync(&hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, s));
+      }
+      const KdDev tr = tree(hc);
+      if (screen) {
+        unsigned long long listed = 0;
+        VLB_CUDA(cudaMemcpyAsync(&listed, cnt, sizeof(listed), cudaMemcpyDeviceToHost, s));
         VLB_CUDA(cudaStreamSynchronize(s));
-        if (hc > 0)
-          by_lanes<AnnLaunch>(*this, (const T *)centers, tr, (i64)cfg.maxNumComparisons, update, assign, dist, err,
-                              (const uint32_t *)list, (i64)hc);
+        if (listed > 0)
+          by_lanes<TiesLaunch>(*this, (const T *)centers, tr, (i64)cfg.maxNumComparisons, update, assign, dist, err,
+                               (const uint32_t *)list, (i64)listed);
       } else {
         by_lanes<AnnLaunch>(*this, (const T *)centers, tr, (i64)cfg.maxNumComparisons, update, assign, dist, err,
                             (const uint32_t *)nullptr, (i64)0);
