@@ -1078,11 +1078,10 @@ struct SLayout {
   static_assert(MT * NF <= 512, "accumulators exceed TMEM");
 };
 
-// Statistics block: converter warps 0-3 and 10-15, epilogue warps 4-7, MMA
-// warp 8, loader warps 9 (x rows) and 16 (q^T).
-constexpr int kStatsConv = 320;  // converter threads
-constexpr int kStatsThreads = kStatsConv + 224;
-constexpr int kStatsLastWarp = kStatsThreads / 32 - 1;
+// Statistics block: converter warps 0-3 and from 10 on, epilogue warps 4-7, MMA
+// warp 8, loader warps 9 (x rows) and the last (q^T).
+__host__ __device__ constexpr int stats_conv(int dim) { return dim == 64 ? 512 : 4 * dim; }  // converter threads
+__host__ __device__ constexpr int stats_threads(int dim) { return stats_conv(dim) + 224; }
 __host__ __device__ constexpr int stats_groups(int fs) { return fs ? 2 : 1; }  // converter groups
 
 // A position in a ring of n buffers, each with a pair of barriers.
@@ -1116,18 +1115,21 @@ __device__ __forceinline__ void drain_copies(uint64_t *full, int n, int issued, 
 // proxy fence, an arrival) and MMAs, so what bounds it is how many chunks are in
 // each step at a time.  With one stage of shared memory held by a chunk from its
 // copy to its MMAs, two or three fitted; with a ring for each step, three or
-// four of each do.  Statistics of 1,024 images, K = 256, ms, before and after:
-// D = 80 FP32 1.31, 1.21; D = 80 BF16 1.01, 0.91; 512 images, D = 128: 1.20,
-// 1.15; 2.5 M rows padded to 96: 0.83, 0.63.  With 256 converter threads
-// 1.21, 0.97, 1.19 and 0.62, with 384 1.22, 0.91, 1.12 and 0.64; in two groups
-// on alternate chunks 1.32, 1.08, 1.29 and 0.68.
+// four of each do.  The converter threads are as many as make whole rounds of 16
+// or 32 rows, so that a thread keeps its four dimensions' centre and scale in
+// registers.  Statistics of 1,024 images, K = 256, D = 80, ms, with one ring and
+// 256 converters, and now: FP32 1.31, 1.21 (0.98 is its HBM time); BF16 1.01,
+// 0.89; 512 images, D = 128: FP32 1.20, 1.13; BF16 1.17, 0.97; K = 64, D = 64:
+// 0.38, 0.36; 2.5 M rows padded to 96: 0.83, 0.63.  At D = 64 256 converters
+// (16 rows a round) took 0.38.  In two groups on alternate chunks the converters
+// were slower: 1.32, 1.08, 1.29 at D = 80 FP32, BF16 and D = 128.
 // FS (features per CTA, blockIdx.z the part): with few items, as for one image,
 // the CTAs of an item's row run split the features too.  Each accumulator sees
 // the same products in the same order (the same bits), and a CTA's chunk takes
 // a quarter of the MMA and conversion time; here the converters do work in two
 // groups (one item of 3,000 rows, K = 256, D = 80: 75 us with one, 62 with two).
 template <int DIM, int MT, int SPLIT, int FS>
-__global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_constant__ SParams p) {
+__global__ void __launch_bounds__(stats_threads(DIM), 1) k_tc_stats(const __grid_constant__ SParams p) {
   using L = SLayout<DIM, MT, SPLIT, FS>;
   constexpr int NST = L::NST, NB = L::NB, NPA = L::NPA;
   const int f0 = FS ? (int)blockIdx.z * FS : 0;     // this CTA's features: [f0, f0 + nf)
@@ -1147,7 +1149,8 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
   uint32_t *s_tmem = (uint32_t *)(bars + 56);
   volatile int *s_abort = (volatile int *)(s_tmem + 1);
 
-  constexpr int G = stats_groups(FS), TG = kStatsConv / G;  // converter groups, threads of one
+  constexpr int kStatsThreads = stats_threads(DIM), kLastWarp = kStatsThreads / 32 - 1;
+  constexpr int G = stats_groups(FS), TG = stats_conv(DIM) / G;  // converter groups, threads of one
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int comp0 = blockIdx.y * MT * 128;  // first component of this CTA's M tiles
   if (tid == 0) {
@@ -1206,7 +1209,7 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
       }
       if (!ok) drain_copies(xfull, p.nx, it, p.err, 15);
     }
-  } else if (warp == kStatsLastWarp) {
+  } else if (warp == kLastWarp) {
     // ----------------------------------------------------- loader of q^T
     if (lane == 0) {
       Ring rq(p.nq);
@@ -1231,11 +1234,13 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
       }
       if (!ok) drain_copies(qfull, p.nq, it, p.err, 18);
     }
-  } else if (warp < 4 || (warp >= 10 && warp < kStatsLastWarp)) {
+  } else if (warp < 4 || (warp >= 10 && warp < kLastWarp)) {
     // ---------------------------------------------------- converters
     const int cw = warp < 4 ? warp : warp - 6;  // converter warp
-    constexpr int WG = kStatsConv / 32 / G;  // warps of a group
+    constexpr int WG = TG / 32;  // warps of a group
     const int ctid = (cw % WG) * 32 + lane, group = cw / WG;
+    const int pp = ctid % NF4, r0 = ctid / NF4, d0 = 4 * pp;  // the quad and first row of FS == 0
+    const float4 c4 = *(const float4 *)(s_ctr + d0), s4 = *(const float4 *)(s_scl + d0);
     Ring rx(p.nx), ro(p.no);
     int it = -1;
     bool ok = true;
@@ -1255,21 +1260,21 @@ __global__ void __launch_bounds__(kStatsThreads, 1) k_tc_stats(const __grid_cons
         const uint32_t sb = smem_u32(sB + ro.i * L::kOp);
         const float *xs = (const float *)(sX + rx.i * L::XST);
         if constexpr (FS == 0) {
+          // A thread has the same four dimensions of one row in RR.
+          constexpr int RR = stats_conv(DIM) / NF4;  // 16 or 32
+          static_assert(32 % RR == 0 && stats_conv(DIM) % NF4 == 0, "whole rounds of rows");
 #pragma unroll
-          for (int j = 0; j < (32 * NF4 + TG - 1) / TG; ++j) {
-            const int i = ctid + TG * j;
-            if (i >= 32 * NF4) break;
-            const int rs = i / NF4, pp = i % NF4;
+          for (int j = 0; j < 32 / RR; ++j) {
+            const int rs = r0 + RR * j;
             const i64 row = cb + rs;
             const bool in = row >= item.row0 && row < item.row1;
-            const int d0 = 4 * pp;
             float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
             if (in && d0 < p.ldx) {
               const float4 x = *(const float4 *)(xs + rs * p.ldx + d0);
-              v0 = (x.x - s_ctr[d0]) * s_scl[d0];
-              v1 = (x.y - s_ctr[d0 + 1]) * s_scl[d0 + 1];
-              v2 = (x.z - s_ctr[d0 + 2]) * s_scl[d0 + 2];
-              v3 = (x.w - s_ctr[d0 + 3]) * s_scl[d0 + 3];
+              v0 = (x.x - c4.x) * s4.x;
+              v1 = (x.y - c4.y) * s4.y;
+              v2 = (x.z - c4.z) * s4.z;
+              v3 = (x.w - c4.w) * s4.w;
             }
             const int kr = rs & 7, kg = rs >> 3;
             uint32_t h0, l0, h1, l1;
@@ -1941,7 +1946,7 @@ void launch_stats(const SParams &p0, int grid_x, int grid_y, int nst_req, cudaSt
     tc::tma_map(&p.qmap, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, p.qimg, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
   }
   VLB_LAUNCH(SPLIT == 2 ? "tc_stats_f16x3" : "tc_stats_f16x2", s,
-             kern<<<dim3(grid_x, grid_y, L::NSPLIT), kStatsThreads, smem, s>>>(p));
+             kern<<<dim3(grid_x, grid_y, L::NSPLIT), stats_threads(DIM), smem, s>>>(p));
 }
 
 constexpr int kStatsFeat = 48;  // features per CTA when they are split
