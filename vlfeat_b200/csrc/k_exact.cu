@@ -73,8 +73,12 @@ __device__ __forceinline__ void cp_async_piece(uint32_t dst, const T *src, bool 
 // in chunks of es_dc dimensions.  The image holds them in the order its lanes
 // read: components in blocks of 32 NJ (component 32 j + l of a block belongs
 // to lane l), per block, dimension, pair of components (j, j + 1) and lane
-// [-mu_j, -mu_j+1, 1/s2_j, 1/s2_j+1].  Padded components and dimensions are
-// zeros, which add nothing to a distance.
+// [-mu_j, -mu_j+1, 1/s2_j, 1/s2_j+1].  Padding has mean 0 and variance 1: the
+// rows' padded dimensions are zeros, so those add nothing to a distance, and a
+// padded component's distance stays a number (or infinity, where a row's squares
+// overflow), so that with its constant -inf its logit is -inf.  An inverse
+// variance of 0 there turned infinity into NaN, which the row's sum of
+// exponentials kept.
 template <typename T>
 __host__ __device__ constexpr int es_dc() { return 64 / (int)sizeof(T); }  // dimensions per chunk
 // Pairs of components per lane (NJ / 2) for K components: the smallest block
@@ -121,7 +125,7 @@ __global__ void k_prepare(const T *__restrict__ priors, const T *__restrict__ me
     for (int d = lane; d < Dp; d += 32) {
       const bool in = k < K && d < D;
       o[(i64)d * h * 128] = in ? -means[(i64)k * D + d] : (T)0;
-      o[(i64)d * h * 128 + 2] = in ? (T)1 / covs[(i64)k * D + d] : (T)0;
+      o[(i64)d * h * 128 + 2] = in ? (T)1 / covs[(i64)k * D + d] : (T)1;
     }
   }
   if (k >= K) return;
