@@ -1256,6 +1256,11 @@ bool launch_stats_sparse(SparseStatsArgs<T> a, i64 nblk, cudaStream_t s) {
 constexpr int kFvCluster = 8;
 // Elements of each half (u and v) per block.
 __host__ __device__ inline i64 fv_part(i64 KD) { return (KD + kFvCluster - 1) / kFvCluster; }
+// Components that a part of E elements of dimension D touches, at most.  Their
+// factors are tabulated in shared memory up to kFvTable of them (64 KB); above
+// that, from 32,752 components on, each element forms its own.
+__host__ __device__ inline i64 fv_part_comps(i64 E, i64 D) { return E / D + 2; }
+constexpr i64 kFvTable = 4096;
 
 // cached: the block's part fits in shared memory; else it is formed in place
 // in the output and scaled there.
@@ -1279,15 +1284,21 @@ __global__ void __launch_bounds__(kThreads) k_fisher_finalize(
   // Per-component factors 1 / (n sqrt(pi_k)) and 1 / (n sqrt(2 pi_k)) of this
   // part's components (-1: the component is skipped, its entries are 0).
   const int ka = (int)(lo / D), nk = hi > lo ? (int)((hi - 1) / D) - ka + 1 : 0;
-  double *sfu = (double *)fin_smem, *sfv = sfu + (E / D + 2);
-  T *zu = (T *)(sfv + (E / D + 2)), *zv = zu + E;
-  for (int k = tid; k < nk; k += kThreads) {
-    const double pk = (double)priors[ka + k];
-    const bool ok = pk >= 1e-6 && n > 0;
-    sfu[k] = ok ? 1.0 / ((double)n * sqrt(pk)) : -1.0;
-    sfv[k] = ok ? 1.0 / ((double)n * sqrt(2.0 * pk)) : -1.0;
+  const i64 ncomp = fv_part_comps(E, D);
+  const bool table = ncomp <= kFvTable;
+  double *sfu = (double *)fin_smem, *sfv = sfu + (table ? ncomp : 0);
+  T *zu = (T *)(sfv + (table ? ncomp : 0)), *zv = zu + E;
+  auto factor = [&](int k, double c) -> double {  // 1 / (n sqrt(c pi_k))
+    const double pk = (double)priors[k];
+    return pk >= 1e-6 && n > 0 ? 1.0 / ((double)n * sqrt(c * pk)) : -1.0;
+  };
+  if (table) {
+    for (int k = tid; k < nk; k += kThreads) {
+      sfu[k] = factor(ka + k, 1.0);
+      sfv[k] = factor(ka + k, 2.0);
+    }
+    __syncthreads();
   }
-  __syncthreads();
   double sq = 0;
   // For float, sqrtf is the float rounding of the double square root (double
   // rounding is innocuous for sqrt with 53 >= 2 x 24 + 2 bits).
@@ -1308,7 +1319,8 @@ __global__ void __launch_bounds__(kThreads) k_fisher_finalize(
       au += pu[(i64)s * KD + e];
       av += pv[(i64)s * KD + e];
     }
-    const T u = finish(au, sfu[k]), v = finish(av, sfv[k]);
+    const T u = finish(au, table ? sfu[k] : factor(ka + k, 1.0));
+    const T v = finish(av, table ? sfv[k] : factor(ka + k, 2.0));
     if (cached) {
       zu[e - lo] = u;
       zv[e - lo] = v;
@@ -1372,7 +1384,8 @@ void launch_fisher_finalize(i64 nimg, i64 K, i64 D, const int *imgSegBegin, cons
                             const double *pv, const unsigned long long *pnt, const T *priors, int flags, i64 imgBase,
                             T *enc, unsigned long long *nterms, cudaStream_t s) {
   const i64 E = fv_part(K * D);
-  size_t smem = sizeof(double) * 2 * (size_t)(E / D + 2);
+  const i64 ncomp = fv_part_comps(E, D);
+  size_t smem = ncomp <= kFvTable ? sizeof(double) * 2 * (size_t)ncomp : 0;
   const int cached = smem + 2 * sizeof(T) * (size_t)E <= 200 * 1024;
   if (cached) smem += 2 * sizeof(T) * (size_t)E;
   auto kern = k_fisher_finalize<T>;
