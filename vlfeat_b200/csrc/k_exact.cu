@@ -991,7 +991,8 @@ __global__ void __launch_bounds__(kFsThreads, 1) k_stats_sparse(const SparseStat
   constexpr int U = 4;         // rows of a list in flight
   Entry *list = (Entry *)(sq + 2 * R * QP) + w * R;  // this warp's passing rows of one component
   const unsigned below = (1u << lane) - 1u;
-  const int sidx = blockIdx.x, k0 = blockIdx.y * KB;
+  const int sidx = blockIdx.x, k0 = (blockIdx.z * gridDim.y + blockIdx.y) * KB;
+  if (k0 >= K) return;
   i64 row0, row1;
   if constexpr (MODE == kSpFisher) {
     const Segment sg = a.segs[sidx];
@@ -1202,7 +1203,8 @@ void launch_stats_sparse_as(const SparseStatsArgs<T> &a, i64 nblk, cudaStream_t 
   const size_t smem = sparse_stats_smem<T, CPW>(a.D);
   VLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int kb = kFsThreads / 32 * CPW;
-  kern<<<dim3((unsigned)nblk, (unsigned)((a.K + kb - 1) / kb)), kFsThreads, smem, s>>>(a);
+  const unsigned nb = (unsigned)((a.K + kb - 1) / kb), nz = (nb + 65534) / 65535;  // a grid has 65,535 rows at most
+  kern<<<dim3((unsigned)nblk, (nb + nz - 1) / nz, nz), kFsThreads, smem, s>>>(a);
 }
 
 // Launches k_stats_sparse over nblk segments (or slabs); false when the shape
