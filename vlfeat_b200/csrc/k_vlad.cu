@@ -146,12 +146,82 @@ __global__ void __launch_bounds__(kVladThreads) k_vlad_accum(
   }
 }
 
-// Global L2 of each image (vl/vlad.c:226-240), one block per image: the squares
-// are added in element order with the bits of the loop (seq_add, tiles through
-// shared memory so that a thread gets neighbouring terms, the next tile's loads
-// in flight), then the block divides the image by the floored norm.  Bound by
-// the scans' latency, about 0.7 us per tile of 8192 terms or binade crossing:
-// 256 images of 20,480 values, 33 us (a warp per image adding in order: 158).
+// Global L2 of each image (vl/vlad.c:226-240): the squares added in element
+// order, the image divided by the floored norm.  Two kernels with the same bits.
+//
+// One warp per image: per chunk of 256 values (8 loads per lane, issued while
+// lane 0 sums the previous chunk) the lanes square their values into shared
+// memory and lane 0 adds the squares.  Bound by the chain, 7 ns a value in float
+// and 10 in double, for as many images as the chip holds warps.
+constexpr int kGnChunk = 256;
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_vlad_global_norm_warp(T *__restrict__ enc, i64 KD, i64 nimg) {
+  __shared__ __align__(16) T sq[8][kGnChunk];
+  __shared__ T s_n[8];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const i64 img = (i64)blockIdx.x * 8 + w;
+  if (img >= nimg) return;
+  T *e = enc + img * KD;
+  T n = (T)0;
+  T z[kGnChunk / 32];
+  auto load = [&](i64 i0) {
+#pragma unroll
+    for (int q = 0; q < kGnChunk / 32; ++q) {
+      const i64 i = i0 + q * 32 + lane;
+      z[q] = i < KD ? e[i] : (T)0;
+    }
+  };
+  load(0);
+  for (i64 i0 = 0; i0 < KD; i0 += kGnChunk) {
+#pragma unroll
+    for (int q = 0; q < kGnChunk / 32; ++q) sq[w][q * 32 + lane] = mul_t(z[q], z[q]);
+    __syncwarp();
+    if (i0 + kGnChunk < KD) load(i0 + kGnChunk);  // next chunk in flight during the sum
+    if (lane == 0) {
+      const int lim = KD - i0 < kGnChunk ? (int)(KD - i0) : kGnChunk;
+      if (lim == kGnChunk) {
+        if constexpr (sizeof(T) == 4) {
+          const float4 *v4 = (const float4 *)sq[w];
+#pragma unroll 16
+          for (int l = 0; l < kGnChunk / 4; ++l) {
+            const float4 v = v4[l];
+            n = add_t(add_t(add_t(add_t(n, v.x), v.y), v.z), v.w);
+          }
+        } else {
+#pragma unroll 32
+          for (int l = 0; l < kGnChunk; ++l) n = add_t(n, sq[w][l]);
+        }
+      } else {
+        for (int l = 0; l < lim; ++l) n = add_t(n, sq[w][l]);
+      }
+    }
+    __syncwarp();
+  }
+  if (lane == 0) s_n[w] = (T)fmax((double)sqrt_t(n), 1e-12);
+  __syncwarp();
+  n = s_n[w];
+  // Eight loads in flight before their divisions and stores.
+  for (i64 i0 = lane; i0 < KD; i0 += 32 * 8) {
+    T v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const i64 i = i0 + 32 * u;
+      v[u] = i < KD ? e[i] : (T)0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const i64 i = i0 + 32 * u;
+      if (i < KD) e[i] = div_t(v[u], n);
+    }
+  }
+}
+
+// One block per image: the squares are added with the bits of the loop (seq_add,
+// tiles through shared memory so that a thread gets neighbouring terms, the next
+// tile's loads in flight).  Bound by the scans' latency, about 0.7 us per tile
+// of 8192 terms or binade crossing, and eight warps an image: 256 images of
+// 20,480 values, 37 us (a warp per image: 148).
 template <typename T>
 __global__ void __launch_bounds__(kSeqThreads) k_vlad_global_norm(T *__restrict__ enc, i64 KD) {
   constexpr int EPT = seq_ept<T>(), kTile = seq_tile<T>(), P = EPT + 16 / (int)sizeof(T);
@@ -611,24 +681,21 @@ struct VgParams {
   int D, K, flags;
 };
 
-// One warp per block: components differ in length, and a block's slot frees
-// when its longest is done (256 images, K = 256, D = 80: 154 us; 8 warps 178).
-constexpr int kVgWarps = 1;
 constexpr int kVgPrefetch = 8;  // rows whose descriptors are loaded together
 
 // One warp per (image, component): the component's rows in order (lane l
 // holds dimensions l + 32 j), the chain step and the mass as in the
 // reference's loop, then the mass step, the signed square root and the
 // component norm (a sum of squares in dimension order), and the coalesced store.  Images with a multi-weight row
-// are left to the streaming kernel.
-template <typename T, int JD>
-__global__ void __launch_bounds__(kVgWarps * 32) k_vlad_group(const VgParams p) {
+// are left to the streaming kernel.  W: warps per block (launch_group).
+template <typename T, int JD, int W>
+__global__ void __launch_bounds__(W * 32) k_vlad_group(const VgParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const i64 img = p.img0 + blockIdx.y;
   if (p.soft[img]) return;
-  const int K = p.K, D = p.D, k = blockIdx.x * kVgWarps + warp;
+  const int K = p.K, D = p.D, k = blockIdx.x * W + warp;
   if (k >= K) return;
-  const T *X = (const T *)p.X, *W = (const T *)p.wgt;
+  const T *X = (const T *)p.X, *A = (const T *)p.wgt;
   const i64 r0 = p.offs[img];
   const int b = p.cstart[img * (K + 1) + k], e = p.cstart[img * (K + 1) + k + 1];
   const int *rows = p.sorted + r0;
@@ -641,7 +708,7 @@ __global__ void __launch_bounds__(kVgWarps * 32) k_vlad_group(const VgParams p) 
   for (int t = b; t < e; t += 32) {
     const int cnt = min(32, e - t);
     const int myrow = lane < cnt ? rows[t + lane] : 0;
-    const T mya = lane < cnt ? W[r0 + myrow] : (T)0;
+    const T mya = lane < cnt ? A[r0 + myrow] : (T)0;
     for (int u0 = 0; u0 < cnt; u0 += kVgPrefetch) {
       T av[kVgPrefetch], xv[kVgPrefetch][JD];
 #pragma unroll
@@ -754,14 +821,31 @@ void launch_stream(T *enc, const T *means, int D, int K, const T *X, const T *A,
   launch_stream_cpw<T, JD, kVsCpw>(p, nimg, s);
 }
 
-template <typename T, int JD>
-void launch_group(const VgParams &p0, i64 nimg, cudaStream_t s) {
+template <typename T, int JD, int W>
+void launch_group_as(const VgParams &p0, i64 nimg, cudaStream_t s) {
   VgParams p = p0;
   for (i64 img0 = 0; img0 < nimg; img0 += 65535) {
     p.img0 = img0;
-    dim3 grid((unsigned)((p.K + kVgWarps - 1) / kVgWarps), (unsigned)std::min<i64>(65535, nimg - img0));
-    VLB_LAUNCH("vlad_group", s, (k_vlad_group<T, JD><<<grid, kVgWarps * 32, 0, s>>>(p)));
+    dim3 grid((unsigned)((p.K + W - 1) / W), (unsigned)std::min<i64>(65535, nimg - img0));
+    VLB_LAUNCH("vlad_group", s, (k_vlad_group<T, JD, W><<<grid, W * 32, 0, s>>>(p)));
   }
+}
+
+// One warp per block: components differ in length, and a block's slot frees
+// when its longest is done (256 images, K = 256, D = 80: 154 us; 8 warps 178).
+// But an SM takes 32 blocks, and float rows of up to 32 dimensions leave room
+// for 48 warps: when the chip cannot hold all blocks at once those take two (20,000
+// images, K = 16, D = 32, half a row a component: 109 us, with one 172, eight
+// 119; 256 such images of 40 rows a component: 17 us, with one 15).
+template <typename T, int JD>
+void launch_group(const VgParams &p, i64 nimg, cudaStream_t s) {
+  if constexpr (sizeof(T) == 4 && JD == 1) {
+    if (p.K * nimg > 32 * 148) {
+      launch_group_as<T, JD, 2>(p, nimg, s);
+      return;
+    }
+  }
+  launch_group_as<T, JD, 1>(p, nimg, s);
 }
 
 // The grouped path's pre-passes: per row its one positive weight, then per
@@ -859,8 +943,19 @@ void vlad_batch(T *enc, const T *means, i64 D, i64 K, const T *X, const T *A, co
   } else {
     vlad_tiles<T>(enc, means, D, K, X, A, doffs, nimg, flags, s);
   }
-  if (!(flags & VL_VLAD_FLAG_UNNORMALIZED))
-    VLB_LAUNCH("vlad_global_norm", s, k_vlad_global_norm<T><<<(unsigned)nimg, kSeqThreads, 0, s>>>(enc, K * D));
+  if (!(flags & VL_VLAD_FLAG_UNNORMALIZED)) {
+    // A block per image costs the scans' 4 us and more whatever the image's
+    // length, and holds eight times the warps; a warp per image its chain.  So
+    // the block for long images, while there are not too many of them.  us, warp
+    // and block, float: 2,048 values, 256 images 22 and 20, 512 images 22 and 30;
+    // 8,192 values, 512 images 62 and 39, 1,024 images 64 and 68, 4,096 images 146
+    // and 231; 32,768 values, 2,048 images 364 and 273; 128 values, 20,000 images
+    // 20 and 324.  Double crosses at the same sizes.
+    const bool block = K * D >= 2048 && nimg * 8 <= K * D;
+    VLB_LAUNCH("vlad_global_norm", s,
+               (block ? k_vlad_global_norm<T><<<(unsigned)nimg, kSeqThreads, 0, s>>>(enc, K * D)
+                      : k_vlad_global_norm_warp<T><<<(unsigned)((nimg + 7) / 8), 256, 0, s>>>(enc, K * D, nimg)));
+  }
   // The scratch above is reused by the next call on this thread, which may
   // use another stream: finish before returning.
   VLB_CUDA(cudaStreamSynchronize(s));
