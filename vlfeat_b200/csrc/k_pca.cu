@@ -451,35 +451,37 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
           uint32_t v[32];
           tmem_ld32(taddr + (uint32_t)(ch * 32), v);
           tmem_wait_ld();
-          if (!mine) continue;
-          const int j0 = ch * 32;
-          if (p.vec_out == 4) {
+          if (mine) {
+            const int j0 = ch * 32;
+            if (p.vec_out == 4) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              if (j0 + 4 * q < p.dout) {
-                float4 w;
-                w.x = scaled(v[4 * q]) * inv;
-                w.y = scaled(v[4 * q + 1]) * inv;
-                w.z = scaled(v[4 * q + 2]) * inv;
-                w.w = scaled(v[4 * q + 3]) * inv;
-                *(float4 *)(o + j0 + 4 * q) = w;
+              for (int q = 0; q < 8; ++q) {
+                if (j0 + 4 * q < p.dout) {
+                  float4 w;
+                  w.x = scaled(v[4 * q]) * inv;
+                  w.y = scaled(v[4 * q + 1]) * inv;
+                  w.z = scaled(v[4 * q + 2]) * inv;
+                  w.w = scaled(v[4 * q + 3]) * inv;
+                  *(float4 *)(o + j0 + 4 * q) = w;
+                }
               }
-            }
-          } else if (p.vec_out == 2) {
+            } else if (p.vec_out == 2) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
-              if (j0 + 2 * q < p.dout) {
-                float2 w;
-                w.x = scaled(v[2 * q]) * inv;
-                w.y = scaled(v[2 * q + 1]) * inv;
-                *(float2 *)(o + j0 + 2 * q) = w;
+              for (int q = 0; q < 16; ++q) {
+                if (j0 + 2 * q < p.dout) {
+                  float2 w;
+                  w.x = scaled(v[2 * q]) * inv;
+                  w.y = scaled(v[2 * q + 1]) * inv;
+                  *(float2 *)(o + j0 + 2 * q) = w;
+                }
               }
-            }
-          } else {
+            } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (j0 + j < p.dout) o[j0 + j] = scaled(v[j]) * inv;
+              for (int j = 0; j < 32; ++j)
+                if (j0 + j < p.dout) o[j0 + j] = scaled(v[j]) * inv;
+            }
           }
+          __syncwarp();  // the next load is the whole warp's
         }
         if (h == parts - 1) {
           tc_fence_before();
