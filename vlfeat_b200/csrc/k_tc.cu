@@ -1097,8 +1097,10 @@ struct Ring {
   }
 };
 
-// After an abandoned run of copies: waits (with a limit) for the last ones, of
-// which up to n are in flight, `issued` in all.
+// After a run of copies, `issued` in all, of which up to n are in flight: waits
+// (with a limit) for the last ones.  A loader does so however it left its loop:
+// one that has issued its last copies cannot know whether another role gives up
+// before they land, and no copy may land in a block that has exited.
 __device__ __forceinline__ void drain_copies(uint64_t *full, int n, int issued, int *err, int code) {
   int never = 0;
   for (int j = issued - 1; j >= 0 && j >= issued - n; --j)
@@ -1207,7 +1209,7 @@ __global__ void __launch_bounds__(stats_threads(DIM), 1) k_tc_stats(const __grid
           ++it;
         }
       }
-      if (!ok) drain_copies(xfull, p.nx, it, p.err, 15);
+      drain_copies(xfull, p.nx, it, p.err, 15);
     }
   } else if (warp == kLastWarp) {
     // ----------------------------------------------------- loader of q^T
@@ -1232,7 +1234,7 @@ __global__ void __launch_bounds__(stats_threads(DIM), 1) k_tc_stats(const __grid
           ++it;
         }
       }
-      if (!ok) drain_copies(qfull, p.nq, it, p.err, 18);
+      drain_copies(qfull, p.nq, it, p.err, 18);
     }
   } else if (warp < 4 || (warp >= 10 && warp < kLastWarp)) {
     // ---------------------------------------------------- converters
