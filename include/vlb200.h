@@ -231,8 +231,10 @@ VL_EXPORT int vlb200_pca_learn_device(float *projection, float *center, vl_size 
  * recorded as the last error); vlb200_fisher_plan_new returns NULL on error.
  *
  * Tile configuration (vlb200_fisher_plan_get/set_config), five int64:
- *   [0] rows per statistics work item (multiple of 128, default 8192; batches
- *       of up to 4,096 rows use shorter ones when those all run at once)
+ *   [0] rows per statistics work item (a multiple of 128).  The default, 8192,
+ *       stands for the built-in choice: at most that many, and fewer for batches
+ *       of up to 4,096 rows when those all run at once.  Any other value is used
+ *       as it is.
  *   [1] 128-component M tiles per statistics CTA (0: two when they fit; 1; 2)
  *   [2] operand stages of the statistics kernel (0: as many as fit)
  *   [3] operand stages of the E-step (0: as many as fit)

@@ -235,7 +235,7 @@ void tc_fisher_batch(const float *X, const i64 *h_offsets, i64 numImages,
 
 // Tunable shapes of the batched Fisher encoder (0: the built-in choice).
 struct TcFvConfig {
-  i64 itemRows = 8192;  // rows per statistics work item (multiple of 128), at most
+  i64 itemRows = 8192;  // rows per statistics work item (multiple of 128); this default: at most that many
   int statsMT = 0;      // 128-component M tiles per statistics CTA: 0 (two when they fit), 1, 2
   int statsStages = 0;  // operand stages of the statistics kernel (0: as many as fit)
   int estepStages = 0;  // operand stages of the E-step (0: as many as fit, at most 8)

@@ -2332,29 +2332,30 @@ i64 default_row_budget(int Kp, bool fp32) {
   return std::max<i64>(1 << 16, (i64)(4ull << 30) / (Kp * qsz));
 }
 
-// Rows per work item: itemRows, except that a batch of up to kSmallRows rows
-// (one image, or a few small ones) is cut into the shortest items (multiples
-// of 128 rows) whose CTAs (M tiles times feature parts) all run at once: an
-// item is one chain of dependent MMAs, about 0.6 us per 32 rows however few
-// features and components a CTA has (3,000 rows in 12 items: 12 us, in one: 62).  Shorter fp32 chains are also closer to
-// FP64 (one image of 3,000 rows, D = 80, K = 256, plain vector: 6.6e-6 with
-// one item, 1.6e-6 with 12; longer images keep their items, so that their
-// vectors stay within a few 1e-6 of what they were).
+// Rows per work item.  A value other than the default is the caller's and is
+// used as it is.  The default stands for at most 8,192 rows; a batch of up to
+// kSmallRows rows (one image, or a few small ones) is cut into the shortest
+// items (256 rows and its doubles) whose CTAs (M tiles times feature parts) all
+// run at once: an item is one chain of dependent MMAs, about 0.6 us per 32 rows
+// however few features and components a CTA has (3,000 rows in 12 items: 12 us, in
+// one: 62).  Shorter fp32 chains are also closer to FP64 (one image of 3,000 rows,
+// D = 80, K = 256, plain vector: 6.6e-6 with one item, 1.6e-6 with 12).
 constexpr i64 kSmallRows = 4096;
-i64 fv_item_rows(const i64 *off, i64 numImages, i64 itemRows, int Kp, i64 D, int nsm) {
-  if (off[numImages] - off[0] > kSmallRows) return itemRows;
+i64 fv_item_rows(const i64 *off, i64 numImages, const TcFvConfig &cfg, int Kp, i64 D, int nsm) {
+  if (cfg.itemRows != TcFvConfig().itemRows || off[numImages] - off[0] > kSmallRows) return cfg.itemRows;
   const i64 per = (i64)(padQ(Kp) / 128) * ((2 * D + 16 + kStatsFeat - 1) / kStatsFeat);
-  for (i64 r = 256; r < itemRows; r *= 2) {
+  for (i64 r = 256; r < cfg.itemRows; r *= 2) {
     i64 items = 0;
     for (i64 j = 0; j < numImages; ++j) items += (off[j + 1] - off[j] + r - 1) / r;
     if (items * per <= nsm) return r;
   }
-  return itemRows;
+  return cfg.itemRows;
 }
 
-void fv_layout(const i64 *off, i64 numImages, i64 rowBudget, i64 itemRows, int Kp, i64 D, int nsm, FvLayout &L) {
+void fv_layout(const i64 *off, i64 numImages, i64 rowBudget, const TcFvConfig &cfg, int Kp, i64 D, int nsm,
+               FvLayout &L) {
   L = FvLayout();
-  itemRows = fv_item_rows(off, numImages, itemRows, Kp, D, nsm);
+  const i64 itemRows = fv_item_rows(off, numImages, cfg, Kp, D, nsm);
   i64 img = 0;
   while (img < numImages) {
     FvChunk c;
@@ -2519,13 +2520,13 @@ void tc_fisher_batch(const float *X, const i64 *h_offsets, i64 numImages, const 
     const Padded P = pad_inputs(X + h_offsets[0] * m.D, N, m, Dp, router, sc, s);
     std::vector<i64> offs(h_offsets, h_offsets + numImages + 1);
     for (auto &o : offs) o -= h_offsets[0];
-    fv_layout(offs.data(), numImages, default_row_budget(Kp, fp32), cfg.itemRows, Kp, Dp, num_sms(), L);
+    fv_layout(offs.data(), numImages, default_row_budget(Kp, fp32), cfg, Kp, Dp, num_sms(), L);
     fv_upload(L, Kp, padQ(Kp), 2 * Dp + 16, fp32, sc, s);
     fv_run(L, sc, P.X, P.m, enc, nterms, flags, precision, cfg, s, nullptr, nullptr, &m, P.ldx);
     check_err((int *)sc.slot[3].p, s);
     return;
   }
-  fv_layout(h_offsets, numImages, default_row_budget(Kp, fp32), cfg.itemRows, Kp, m.D, num_sms(), L);
+  fv_layout(h_offsets, numImages, default_row_budget(Kp, fp32), cfg, Kp, m.D, num_sms(), L);
   fv_upload(L, Kp, padQ(Kp), (int)(2 * m.D + 16), fp32, sc, s);
   fv_run(L, sc, X, m, enc, nterms, flags, precision, cfg, s);
   check_err((int *)sc.slot[3].p, s);
@@ -2572,7 +2573,7 @@ namespace {
 void plan_build(TcFvPlan &p, cudaStream_t s) {
   const bool fp32 = (p.precision == VLB200_PREC_FP32);
   const i64 budget = p.cfg.rowBudget > 0 ? p.cfg.rowBudget : default_row_budget(p.Kp, fp32);
-  fv_layout(p.offsets.data(), p.numImages, budget, p.cfg.itemRows, p.Kp, p.D, num_sms(), p.layout);
+  fv_layout(p.offsets.data(), p.numImages, budget, p.cfg, p.Kp, p.D, num_sms(), p.layout);
   fv_upload(p.layout, p.Kp, padQ(p.Kp), (int)(2 * p.D + 16), fp32, p.sc, s);
   VLB_CUDA(cudaStreamSynchronize(s));
 }
@@ -2628,7 +2629,7 @@ void tc_fv_plan_run_host(TcFvPlan *p, const DevModel<float> &m, const float *Xh,
   const i64 D = p->D, FV = 2 * p->K * p->D;
   if (!p->pipeBuilt) {
     const i64 budget = std::max<i64>(1, (total + TcFvPlan::kPipeChunks - 1) / TcFvPlan::kPipeChunks);
-    fv_layout(p->offsets.data(), p->numImages, budget, p->cfg.itemRows, p->Kp, p->D, num_sms(), p->pipe);
+    fv_layout(p->offsets.data(), p->numImages, budget, p->cfg, p->Kp, p->D, num_sms(), p->pipe);
     fv_upload(p->pipe, p->Kp, padQ(p->Kp), (int)(2 * p->D + 16), fp32, p->scPipe, s);
     if (!p->h2d) VLB_CUDA(cudaStreamCreateWithFlags(&p->h2d, cudaStreamNonBlocking));
     if (!p->d2h) VLB_CUDA(cudaStreamCreateWithFlags(&p->d2h, cudaStreamNonBlocking));
@@ -2698,7 +2699,10 @@ TcFvConfig tc_fv_plan_autotune(TcFvPlan *p, const DevModel<float> &m, const floa
   const i64 qsz = fp32 ? 4 : 2;
   // A single chunk when its q image fits in 16 GB; else the default budget.
   const i64 big = std::min<i64>(whole, (i64)(16ull << 30) / (p->Kp * qsz));
-  for (int itemRows : {4096, 8192, 16384})
+  i64 longest = 0;
+  for (i64 j = 0; j < p->numImages; ++j) longest = std::max(longest, p->offsets[j + 1] - p->offsets[j]);
+  for (int itemRows : {4096, 8192, 16384}) {
+    if (itemRows > 8192 && longest <= 4096) continue;  // one item an image, as with 4,096
     for (int mt : {0, 1})
       for (int est : {0, 2})
         for (i64 budget : {(i64)0, big}) {
@@ -2706,6 +2710,7 @@ TcFvConfig tc_fv_plan_autotune(TcFvPlan *p, const DevModel<float> &m, const floa
           c.itemRows = itemRows; c.statsMT = mt; c.estepStages = est; c.rowBudget = budget;
           cands.push_back(c);
         }
+  }
   cudaEvent_t e0, e1;
   VLB_CUDA(cudaEventCreate(&e0));
   VLB_CUDA(cudaEventCreate(&e1));
