@@ -232,9 +232,10 @@ VL_EXPORT int vlb200_pca_learn_device(float *projection, float *center, vl_size 
  *
  * Tile configuration (vlb200_fisher_plan_get/set_config), five int64:
  *   [0] rows per statistics work item (a multiple of 128).  The default, 8192,
- *       stands for the built-in choice: at most that many, and fewer for batches
- *       of up to 4,096 rows when those all run at once.  Any other value is used
- *       as it is.
+ *       stands for the built-in choice: at most that many, and fewer where a
+ *       batch's items are so few that shorter ones still all run at once (the
+ *       rounding of an image's vector then depends on the rest of its batch).
+ *       Any other value is used as it is.
  *   [1] 128-component M tiles per statistics CTA (0: two when they fit; 1; 2)
  *   [2] operand stages of the statistics kernel (0: as many as fit)
  *   [3] operand stages of the E-step (0: as many as fit)

@@ -1,7 +1,8 @@
 """The statistics' work items of small batches.  An explicit item_rows of a plan is
 used as it is: an image's plain vector then has the same bits alone and among other
 images (at a row offset that is a multiple of 8, the posterior image's row group),
-and whatever larger value is given."""
+and whatever larger value is given.  The default shortens items while they all run at
+once, so the statistics' time has no step at any one row count."""
 import numpy as np
 import pytest
 
@@ -49,3 +50,27 @@ def test_config_round_trip_keeps_the_default(vl):
     saved = p.get_config()
     assert saved["item_rows"] == 8192
     assert torch.equal(_plan(vl, 80, 256, offs, 3, "fp32", x, **saved)[1], enc)
+
+
+def test_no_step_in_time(vl):
+    """Device time of the statistics of one image, K=256, D=80: 17 us up to 4,096
+    rows and 84 at 4,097 when short items ended there.  Below twice per 500 rows."""
+    import torch
+    from vlfeat_b200 import workloads as W
+    pr, mu, cv = (torch.from_numpy(v).cuda() for v in W.fv_gmm(256, 80, seed=3))
+    x = torch.from_numpy(W.pca_like(9000, 80, seed=4)).cuda()
+    enc = torch.zeros((1, 2 * 256 * 80), device="cuda")
+    t = []
+    for n in range(1000, 9001, 500):
+        best = np.inf
+        for i in range(6):
+            vl.profile_reset()
+            vl.profile_enable(True)
+            vl.fisher_encode_batch_device(enc, mu, cv, pr, x[:n], np.array([0, n], np.int64), 3, "fp32")
+            torch.cuda.synchronize()
+            if i:
+                best = min(best, vl.profile_read()["tc_stats_f16x3"][1])
+            vl.profile_enable(False)
+        t.append(best)
+    vl.profile_reset()
+    assert max(b / a for a, b in zip(t, t[1:])) < 2, t

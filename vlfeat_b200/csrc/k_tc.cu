@@ -2332,24 +2332,39 @@ i64 default_row_budget(int Kp, bool fp32) {
   return std::max<i64>(1 << 16, (i64)(4ull << 30) / (Kp * qsz));
 }
 
+// CTAs of the statistics kernel that work on one item, as Tc::stats launches it
+// when items are few: M tiles times feature parts, or with an explicit statsMT
+// the M tiles alone.
+i64 fv_item_ctas(int Kp, i64 D, int mt) {
+  const i64 mtiles = padQ(Kp) / 128;
+  if (mt == 0) return mtiles * ((2 * D + 16 + kStatsFeat - 1) / kStatsFeat);
+  const bool two = mt == 2 && 2 * (2 * D + 16) <= 512 && mtiles % 2 == 0;
+  return two ? mtiles / 2 : mtiles;
+}
+
 // Rows per work item.  A value other than the default is the caller's and is
-// used as it is.  The default stands for at most 8,192 rows; a batch of up to
-// kSmallRows rows (one image, or a few small ones) is cut into the shortest
-// items (256 rows and its doubles) whose CTAs (M tiles times feature parts) all
-// run at once: an item is one chain of dependent MMAs, about 0.6 us per 32 rows
-// however few features and components a CTA has (3,000 rows in 12 items: 12 us, in
-// one: 62).  Shorter fp32 chains are also closer to FP64 (one image of 3,000 rows,
-// D = 80, K = 256, plain vector: 6.6e-6 with one item, 1.6e-6 with 12).
-constexpr i64 kSmallRows = 4096;
+// used as it is.  The default stands for at most 8,192 rows, and fewer where a
+// batch's items are so few that the chip could run more at once: then the
+// shortest (a multiple of 128, from 256) whose CTAs all run at once.  An item is
+// one chain of dependent MMAs, about 0.6 us per 32 rows however few features and
+// components a CTA has (3,000 rows in 12 items: 12 us, in one: 62).  Above the
+// size where 8,192-row items fill the chip (147,000 rows of one image at K = 256,
+// D = 80) nothing is shorter.  Shorter fp32 chains are also closer to FP64 (one
+// image of 3,000 rows, D = 80, K = 256, plain vector: 6.6e-6 with one item, 1.6e-6
+// with 12).  An image's items, and with them its rounding, so depend on the other
+// images of its batch; with an explicit itemRows only on the image's own rows.
 i64 fv_item_rows(const i64 *off, i64 numImages, const TcFvConfig &cfg, int Kp, i64 D, int nsm) {
-  if (cfg.itemRows != TcFvConfig().itemRows || off[numImages] - off[0] > kSmallRows) return cfg.itemRows;
-  const i64 per = (i64)(padQ(Kp) / 128) * ((2 * D + 16 + kStatsFeat - 1) / kStatsFeat);
-  for (i64 r = 256; r < cfg.itemRows; r *= 2) {
-    i64 items = 0;
-    for (i64 j = 0; j < numImages; ++j) items += (off[j + 1] - off[j] + r - 1) / r;
-    if (items * per <= nsm) return r;
-  }
-  return cfg.itemRows;
+  if (cfg.itemRows != TcFvConfig().itemRows) return cfg.itemRows;
+  const i64 most = nsm / fv_item_ctas(Kp, D, cfg.statsMT);  // items that run at once
+  auto items = [&](i64 r) {
+    i64 n = 0;
+    for (i64 j = 0; j < numImages && n <= most; ++j) n += (off[j + 1] - off[j] + r - 1) / r;
+    return n;
+  };
+  if (items(cfg.itemRows) > most) return cfg.itemRows;
+  i64 r = 256;
+  while (r < cfg.itemRows && items(r) > most) r += 128;
+  return r;
 }
 
 void fv_layout(const i64 *off, i64 numImages, i64 rowBudget, const TcFvConfig &cfg, int Kp, i64 D, int nsm,
