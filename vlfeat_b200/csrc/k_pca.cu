@@ -539,20 +539,34 @@ __global__ void __launch_bounds__(kPtThreads, 1) k_pca_tc(const PcaTcParams p) {
             } while (c == 32);
           o = probe(1);
           c = 0;
-        } else {
-          img += c;
         }
-        // Lanes c .. 31 hold the first rows of images img + 1, img + 2, ...
-        const unsigned inside = __ballot_sync(0xffffffffu, o <= r0 + 127) & ~((1u << c) - 1u);
-        i64 im[4];
+        // A row's image is as many past img as there are first rows up to it: counted
+        // 32 images at a time, one by one where few start inside the tile, else
+        // by bisection over the lanes.
+        i64 im[4] = {img, img, img, img};
+        i64 w = img;
+        img += c;
+        while (true) {
+          const int rel = (int)max((i64)-1, min((i64)128, o - r0));
+          const int n0 = __popc(__ballot_sync(0xffffffffu, rel <= 0)), n = __popc(__ballot_sync(0xffffffffu, rel <= 127));
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const i64 row = r0 + 32 * q + lane;
-          im[q] = img;
-          for (unsigned m = inside; m; m &= m - 1)
-            if (__shfl_sync(0xffffffffu, o, __ffs(m) - 1) <= row) ++im[q];
-          if (inside >> 31)  // the probe may not reach the tile's last image
-            while (im[q] + 1 < p.nimg && __ldg(p.offs + im[q] + 1) <= row) ++im[q];
+          for (int q = 0; q < 4; ++q) {
+            const int row = 32 * q + lane;
+            int k = n0;
+            if (n - n0 <= 6) {
+              for (int l = n0; l < n; ++l) k += __shfl_sync(0xffffffffu, rel, l) <= row;
+            } else {
+              k = 0;
+#pragma unroll
+              for (int d = 16; d >= 1; d /= 2)
+                if (__shfl_sync(0xffffffffu, rel, k + d - 1) <= row) k += d;
+              if (__shfl_sync(0xffffffffu, rel, k) <= row) ++k;
+            }
+            im[q] += k;
+          }
+          if (n < 32) break;  // the tile's last image is among them
+          w += 32;
+          o = w + lane + 1 < p.nimg ? __ldg(p.offs + w + lane + 1) : INT64_MAX;
         }
         float fx[4], fy[4], sx[4], sy[4];
 #pragma unroll
