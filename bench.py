@@ -21,6 +21,8 @@ FP64 GPU encodings of all images are reported beside it, with the BF16+router
 to FP32 ratio the metric compares.  `e2e` times the same metric through the public API with
 host buffers (pinned host -> device copy of the step's descriptors, encode,
 device -> host copy of the encodings, all inside the timed region).
+Rank 0 writes the whole report (every path, kernel and secondary workload) to
+standard error and the result as one short JSON line to standard output.
 Under torchrun every rank encodes its own image set (replicas, weak scaling);
 the step time is the max over ranks.
 """
@@ -43,6 +45,7 @@ METRIC = "FV-encoded descriptors/s, K=256 D=80: plain FP32 vs BF16+router @ rel 
 K, D = 256, 80
 NUM_IMAGES = 4096
 FLAGS = 3  # VL_FISHER_FLAG_IMPROVED
+LINE_DICTS = ("config", "clocks", "e2e", "roofline", "path_roofline", "cpu_baseline")
 PATHS = ["exact", "fp32", "bf16", "bf16_router"]
 
 
@@ -957,6 +960,18 @@ def router_config3(capi, n_train=2_000_000, n_eval=10_000_000, ms=(4, 8, 16), th
     return out
 
 
+def result_line(report):
+    """The result as one short line: the report's plain values and those of its
+    main entries.  (The whole report, 20 KB with every path's kernels and errors
+    per iteration, is no line that a reader of the output's end gets whole.)"""
+    plain = lambda v: not isinstance(v, (dict, list))
+    line = {k: v for k, v in report.items() if plain(v)}
+    for k in LINE_DICTS:
+        if k in report:
+            line[k] = {n: v for n, v in report[k].items() if plain(v) or (k, n) == ("clocks", "reasons")}
+    return json.dumps({k: line[k] for k in report if k in line})
+
+
 def run_reference(args, rank, world):
     """The reference arm: VLFeat's own CPU code on the host cores."""
     if rank != 0:
@@ -1134,7 +1149,8 @@ def main():
                 capi.lib().vlb200_router_set_default(None, 8, 0.99)
                 del router
             out["router_config3"] = router_config3(capi, n_train=args.router_train, n_eval=args.router_eval)
-        print(json.dumps(out), flush=True)
+        print(json.dumps(out), file=sys.stderr, flush=True)
+        print(result_line(out), flush=True)
     if dist:
         dist.barrier()
         dist.destroy_process_group()
