@@ -677,8 +677,8 @@ struct VgParams {
   const void *means, *X, *wgt;
   const i64 *offs;
   const int *sorted, *cstart, *soft;
-  i64 img0;
-  int D, K, flags;
+  i64 N, img0, img1;
+  int D, K, flags, per;  // per: images per block (launch_group_as)
 };
 
 constexpr int kVgPrefetch = 8;  // rows whose descriptors are loaded together
@@ -691,89 +691,91 @@ constexpr int kVgPrefetch = 8;  // rows whose descriptors are loaded together
 template <typename T, int JD, int W>
 __global__ void __launch_bounds__(W * 32) k_vlad_group(const VgParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const i64 img = p.img0 + blockIdx.y;
-  if (p.soft[img]) return;
   const int K = p.K, D = p.D, k = blockIdx.x * W + warp;
   if (k >= K) return;
   const T *X = (const T *)p.X, *A = (const T *)p.wgt;
-  const i64 r0 = p.offs[img];
-  const int b = p.cstart[img * (K + 1) + k], e = p.cstart[img * (K + 1) + k + 1];
-  const int *rows = p.sorted + r0;
-  T acc[JD];
+  const i64 first = p.img0 + (i64)blockIdx.y * p.per, last = min(p.img1, first + p.per);
+  for (i64 img = first; img < last; ++img) {
+    if (p.soft[img]) continue;
+    const i64 r0 = p.offs[img];
+    const int b = p.cstart[img * (K + 1) + k], e = p.cstart[img * (K + 1) + k + 1];
+    const int *rows = p.sorted + r0;
+    T acc[JD];
 #pragma unroll
-  for (int j = 0; j < JD; ++j) acc[j] = (T)0;
-  double mass = 0.0;
-  // 32 of the component's rows at a time: lane j loads the j-th row index and
-  // weight; the rows' descriptors are loaded kVgPrefetch rows ahead.
-  for (int t = b; t < e; t += 32) {
-    const int cnt = min(32, e - t);
-    const int myrow = lane < cnt ? rows[t + lane] : 0;
-    const T mya = lane < cnt ? A[r0 + myrow] : (T)0;
-    for (int u0 = 0; u0 < cnt; u0 += kVgPrefetch) {
-      T av[kVgPrefetch], xv[kVgPrefetch][JD];
+    for (int j = 0; j < JD; ++j) acc[j] = (T)0;
+    double mass = 0.0;
+    // 32 of the component's rows at a time: lane j loads the j-th row index and
+    // weight; the rows' descriptors are loaded kVgPrefetch rows ahead.
+    for (int t = b; t < e; t += 32) {
+      const int cnt = min(32, e - t);
+      const int myrow = lane < cnt ? rows[t + lane] : 0;
+      const T mya = lane < cnt ? A[r0 + myrow] : (T)0;
+      for (int u0 = 0; u0 < cnt; u0 += kVgPrefetch) {
+        T av[kVgPrefetch], xv[kVgPrefetch][JD];
 #pragma unroll
-      for (int u = 0; u < kVgPrefetch; ++u) {
-        const int rr = __shfl_sync(0xffffffffu, myrow, (u0 + u) & 31);
-        av[u] = __shfl_sync(0xffffffffu, mya, (u0 + u) & 31);
-        if (u0 + u < cnt) {
-          const i64 row = r0 + rr;
+        for (int u = 0; u < kVgPrefetch; ++u) {
+          const int rr = __shfl_sync(0xffffffffu, myrow, (u0 + u) & 31);
+          av[u] = __shfl_sync(0xffffffffu, mya, (u0 + u) & 31);
+          if (u0 + u < cnt) {
+            const i64 row = r0 + rr;
 #pragma unroll
-          for (int j = 0; j < JD; ++j) {
-            const int d = lane + 32 * j;
-            xv[u][j] = d < D ? X[row * D + d] : (T)0;
+            for (int j = 0; j < JD; ++j) {
+              const int d = lane + 32 * j;
+              xv[u][j] = d < D ? X[row * D + d] : (T)0;
+            }
           }
         }
-      }
 #pragma unroll
-      for (int u = 0; u < kVgPrefetch; ++u) {
-        if (u0 + u < cnt) {
-          mass += (double)av[u];
-          if (sizeof(T) == 4 && av[u] == (T)1) {
+        for (int u = 0; u < kVgPrefetch; ++u) {
+          if (u0 + u < cnt) {
+            mass += (double)av[u];
+            if (sizeof(T) == 4 && av[u] == (T)1) {
 #pragma unroll
-            for (int j = 0; j < JD; ++j) acc[j] = add_t(acc[j], xv[u][j]);
-          } else {
+              for (int j = 0; j < JD; ++j) acc[j] = add_t(acc[j], xv[u][j]);
+            } else {
 #pragma unroll
-            for (int j = 0; j < JD; ++j) acc[j] = acc_step(acc[j], av[u], xv[u][j]);
+              for (int j = 0; j < JD; ++j) acc[j] = acc_step(acc[j], av[u], xv[u][j]);
+            }
           }
         }
       }
     }
-  }
-  const T *mu = (const T *)p.means + (i64)k * D;
-  T z[JD];
-#pragma unroll
-  for (int j = 0; j < JD; ++j) {
-    const int d = lane + 32 * j;
-    z[j] = (T)0;
-    if (d < D) {
-      T v = vlad_mass_step<T>(acc[j], mu[d], mass, p.flags);
-      if (p.flags & VL_VLAD_FLAG_SQUARE_ROOT) v = v >= (T)0 ? sqrt_t(v) : -sqrt_t(-v);
-      z[j] = v;
-    }
-  }
-  if (p.flags & VL_VLAD_FLAG_NORMALIZE_COMPONENTS) {
-    // In dimension order: every lane adds the shuffled squares, so that the
-    // chain is the additions alone.
-    T nrm = (T)0;
+    const T *mu = (const T *)p.means + (i64)k * D;
+    T z[JD];
 #pragma unroll
     for (int j = 0; j < JD; ++j) {
-      const T sq = mul_t(z[j], z[j]);
-      if (32 * j + 32 <= D) {
-#pragma unroll
-        for (int l = 0; l < 32; ++l) nrm = add_t(nrm, __shfl_sync(0xffffffffu, sq, l));
-      } else {
-        for (int l = 0; l < D - 32 * j; ++l) nrm = add_t(nrm, __shfl_sync(0xffffffffu, sq, l));
+      const int d = lane + 32 * j;
+      z[j] = (T)0;
+      if (d < D) {
+        T v = vlad_mass_step<T>(acc[j], mu[d], mass, p.flags);
+        if (p.flags & VL_VLAD_FLAG_SQUARE_ROOT) v = v >= (T)0 ? sqrt_t(v) : -sqrt_t(-v);
+        z[j] = v;
       }
     }
-    nrm = (T)fmax((double)sqrt_t(nrm), 1e-12);
+    if (p.flags & VL_VLAD_FLAG_NORMALIZE_COMPONENTS) {
+      // In dimension order: every lane adds the shuffled squares, so that the
+      // chain is the additions alone.
+      T nrm = (T)0;
 #pragma unroll
-    for (int j = 0; j < JD; ++j) z[j] = div_t(z[j], nrm);
-  }
-  T *out = (T *)p.enc + img * (i64)K * D + (i64)k * D;
+      for (int j = 0; j < JD; ++j) {
+        const T sq = mul_t(z[j], z[j]);
+        if (32 * j + 32 <= D) {
 #pragma unroll
-  for (int j = 0; j < JD; ++j) {
-    const int d = lane + 32 * j;
-    if (d < D) out[d] = z[j];
+          for (int l = 0; l < 32; ++l) nrm = add_t(nrm, __shfl_sync(0xffffffffu, sq, l));
+        } else {
+          for (int l = 0; l < D - 32 * j; ++l) nrm = add_t(nrm, __shfl_sync(0xffffffffu, sq, l));
+        }
+      }
+      nrm = (T)fmax((double)sqrt_t(nrm), 1e-12);
+#pragma unroll
+      for (int j = 0; j < JD; ++j) z[j] = div_t(z[j], nrm);
+    }
+    T *out = (T *)p.enc + img * (i64)K * D + (i64)k * D;
+#pragma unroll
+    for (int j = 0; j < JD; ++j) {
+      const int d = lane + 32 * j;
+      if (d < D) out[d] = z[j];
+    }
   }
 }
 
@@ -821,12 +823,25 @@ void launch_stream(T *enc, const T *means, int D, int K, const T *X, const T *A,
   launch_stream_cpw<T, JD, kVsCpw>(p, nimg, s);
 }
 
+// Images per block: as many, up to eight, as leave four blocks for each that the
+// chip holds, or ten where components have more than four rows on average and
+// blocks so differ more in length.  A block takes 0.55 ns to start and end even
+// when its image is left to the streaming kernel.  us, one image a block and this
+// rule, float: 3,000 images of 100 rows, K = 64, D = 64, 125 and 117, all of them
+// soft 105 and 19 (eight warps a block: 21); 20,000 of 20 rows 691 and 506, soft 662
+// and 88; 4,000 of 300 rows, K = 32, D = 48, 148 and 144.  256 images of 4,000 rows,
+// K = 256, D = 80 stay at one (150; with two 181), as do 600 of 2,000 rows,
+// K = 128, D = 64 (130; 148).
 template <typename T, int JD, int W>
 void launch_group_as(const VgParams &p0, i64 nimg, cudaStream_t s) {
   VgParams p = p0;
-  for (i64 img0 = 0; img0 < nimg; img0 += 65535) {
+  const i64 blocks = (p.K + W - 1) / W * nimg, chip = 32 * 148;
+  p.per = (int)std::max<i64>(1, std::min<i64>(8, blocks / (p.N <= 4 * p.K * nimg ? 4 * chip : 10 * chip)));
+  const i64 step = (i64)65535 * p.per;
+  for (i64 img0 = 0; img0 < nimg; img0 += step) {
     p.img0 = img0;
-    dim3 grid((unsigned)((p.K + W - 1) / W), (unsigned)std::min<i64>(65535, nimg - img0));
+    p.img1 = std::min(nimg, img0 + step);
+    dim3 grid((unsigned)((p.K + W - 1) / W), (unsigned)((p.img1 - img0 + p.per - 1) / p.per));
     VLB_LAUNCH("vlad_group", s, (k_vlad_group<T, JD, W><<<grid, W * 32, 0, s>>>(p)));
   }
 }
@@ -928,7 +943,7 @@ void vlad_batch(T *enc, const T *means, i64 D, i64 K, const T *X, const T *A, co
     const int *only = nullptr;
     if (K <= 1024 && N < (i64)INT32_MAX) {
       VgParams g;
-      g.enc = enc; g.means = means; g.X = X; g.offs = doffs; g.D = (int)D; g.K = (int)K; g.flags = flags;
+      g.enc = enc; g.means = means; g.X = X; g.offs = doffs; g.N = N; g.D = (int)D; g.K = (int)K; g.flags = flags;
       only = group_rows<T>(sc, A, N, (int)K, doffs, nimg, g, s);
       if (jd <= 1) launch_group<T, 1>(g, nimg, s);
       else if (jd == 2) launch_group<T, 2>(g, nimg, s);
