@@ -965,7 +965,7 @@ def result_line(report):
     main entries.  (The whole report, 20 KB with every path's kernels and errors
     per iteration, is no line that a reader of the output's end gets whole.)"""
     plain = lambda v: not isinstance(v, (dict, list))
-    line = {k: v for k, v in report.items() if plain(v)}
+    line = {k: v for k, v in report.items() if plain(v) and k != "precision_note"}
     for k in LINE_DICTS:
         if k in report:
             line[k] = {n: v for n, v in report[k].items() if plain(v) or (k, n) == ("clocks", "reasons")}
