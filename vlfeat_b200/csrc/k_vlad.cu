@@ -687,14 +687,16 @@ constexpr int kVgPrefetch = 8;  // rows whose descriptors are loaded together
 // holds dimensions l + 32 j), the chain step and the mass as in the
 // reference's loop, then the mass step, the signed square root and the
 // component norm (a sum of squares in dimension order), and the coalesced store.  Images with a multi-weight row
-// are left to the streaming kernel.  W: warps per block (launch_group).
-template <typename T, int JD, int W>
+// are left to the streaming kernel.  W: warps per block (launch_group); MANY: per
+// images a block, else one.
+template <typename T, int JD, int W, bool MANY>
 __global__ void __launch_bounds__(W * 32) k_vlad_group(const VgParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int K = p.K, D = p.D, k = blockIdx.x * W + warp;
   if (k >= K) return;
   const T *X = (const T *)p.X, *A = (const T *)p.wgt;
-  const i64 first = p.img0 + (i64)blockIdx.y * p.per, last = min(p.img1, first + p.per);
+  const i64 first = p.img0 + (i64)blockIdx.y * (MANY ? p.per : 1);
+  const i64 last = MANY ? min(p.img1, first + p.per) : first + 1;
   for (i64 img = first; img < last; ++img) {
     if (p.soft[img]) continue;
     const i64 r0 = p.offs[img];
@@ -824,25 +826,25 @@ void launch_stream(T *enc, const T *means, int D, int K, const T *X, const T *A,
 }
 
 // Images per block: as many, up to eight, as leave four blocks for each that the
-// chip holds, or ten where components have more than four rows on average and
+// chip holds, or twenty where components have more than four rows on average and
 // blocks so differ more in length.  A block takes 0.55 ns to start and end even
 // when its image is left to the streaming kernel.  us, one image a block and this
-// rule, float: 3,000 images of 100 rows, K = 64, D = 64, 125 and 117, all of them
-// soft 105 and 19 (eight warps a block: 21); 20,000 of 20 rows 691 and 506, soft 662
-// and 88; 4,000 of 300 rows, K = 32, D = 48, 148 and 144.  256 images of 4,000 rows,
-// K = 256, D = 80 stay at one (150; with two 181), as do 600 of 2,000 rows,
-// K = 128, D = 64 (130; 148).
+// rule, float: 3,000 images of 100 rows, K = 64, D = 64, 119 and 117, all of them
+// soft 105 and 19 (eight warps a block: 21); 20,000 of 20 rows 668 and 506, soft 666
+// and 88.  256 images of 4,000 rows, K = 256, D = 80, stay at one (142; with two
+// 181), as do 4,000 of 300 rows, K = 32, D = 48 (140; 142).
 template <typename T, int JD, int W>
 void launch_group_as(const VgParams &p0, i64 nimg, cudaStream_t s) {
   VgParams p = p0;
   const i64 blocks = (p.K + W - 1) / W * nimg, chip = 32 * 148;
-  p.per = (int)std::max<i64>(1, std::min<i64>(8, blocks / (p.N <= 4 * p.K * nimg ? 4 * chip : 10 * chip)));
+  p.per = (int)std::max<i64>(1, std::min<i64>(8, blocks / (p.N <= 4 * p.K * nimg ? 4 * chip : 20 * chip)));
   const i64 step = (i64)65535 * p.per;
   for (i64 img0 = 0; img0 < nimg; img0 += step) {
     p.img0 = img0;
     p.img1 = std::min(nimg, img0 + step);
     dim3 grid((unsigned)((p.K + W - 1) / W), (unsigned)((p.img1 - img0 + p.per - 1) / p.per));
-    VLB_LAUNCH("vlad_group", s, (k_vlad_group<T, JD, W><<<grid, W * 32, 0, s>>>(p)));
+    if (p.per > 1) VLB_LAUNCH("vlad_group", s, (k_vlad_group<T, JD, W, true><<<grid, W * 32, 0, s>>>(p)));
+    else VLB_LAUNCH("vlad_group", s, (k_vlad_group<T, JD, W, false><<<grid, W * 32, 0, s>>>(p)));
   }
 }
 
@@ -850,8 +852,8 @@ void launch_group_as(const VgParams &p0, i64 nimg, cudaStream_t s) {
 // when its longest is done (256 images, K = 256, D = 80: 154 us; 8 warps 178).
 // But an SM takes 32 blocks, and float rows of up to 32 dimensions leave room
 // for 48 warps: when the chip cannot hold all blocks at once those take two (20,000
-// images, K = 16, D = 32, half a row a component: 109 us, with one 172, eight
-// 119; 256 such images of 40 rows a component: 17 us, with one 15).
+// images, K = 16, D = 32, half a row a component, an image a block: 109 us, with one
+// 172, eight 119; 256 such images of 40 rows a component: 17 us, with one 15).
 template <typename T, int JD>
 void launch_group(const VgParams &p, i64 nimg, cudaStream_t s) {
   if constexpr (sizeof(T) == 4 && JD == 1) {
