@@ -686,98 +686,107 @@ constexpr int kVgPrefetch = 8;  // rows whose descriptors are loaded together
 // One warp per (image, component): the component's rows in order (lane l
 // holds dimensions l + 32 j), the chain step and the mass as in the
 // reference's loop, then the mass step, the signed square root and the
-// component norm (a sum of squares in dimension order), and the coalesced store.  Images with a multi-weight row
-// are left to the streaming kernel.  W: warps per block (launch_group); MANY: per
-// images a block, else one.
+// component norm (a sum of squares in dimension order), and the coalesced store.
+template <typename T, int JD>
+__device__ __forceinline__ void vlad_group_one(const VgParams &p, i64 img, int k, int lane) {
+  const int K = p.K, D = p.D;
+  const T *X = (const T *)p.X, *A = (const T *)p.wgt;
+  const i64 r0 = p.offs[img];
+  const int b = p.cstart[img * (K + 1) + k], e = p.cstart[img * (K + 1) + k + 1];
+  const int *rows = p.sorted + r0;
+  T acc[JD];
+#pragma unroll
+  for (int j = 0; j < JD; ++j) acc[j] = (T)0;
+  double mass = 0.0;
+  // 32 of the component's rows at a time: lane j loads the j-th row index and
+  // weight; the rows' descriptors are loaded kVgPrefetch rows ahead.
+  for (int t = b; t < e; t += 32) {
+    const int cnt = min(32, e - t);
+    const int myrow = lane < cnt ? rows[t + lane] : 0;
+    const T mya = lane < cnt ? A[r0 + myrow] : (T)0;
+    for (int u0 = 0; u0 < cnt; u0 += kVgPrefetch) {
+      T av[kVgPrefetch], xv[kVgPrefetch][JD];
+#pragma unroll
+      for (int u = 0; u < kVgPrefetch; ++u) {
+        const int rr = __shfl_sync(0xffffffffu, myrow, (u0 + u) & 31);
+        av[u] = __shfl_sync(0xffffffffu, mya, (u0 + u) & 31);
+        if (u0 + u < cnt) {
+          const i64 row = r0 + rr;
+#pragma unroll
+          for (int j = 0; j < JD; ++j) {
+            const int d = lane + 32 * j;
+            xv[u][j] = d < D ? X[row * D + d] : (T)0;
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kVgPrefetch; ++u) {
+        if (u0 + u < cnt) {
+          mass += (double)av[u];
+          if (sizeof(T) == 4 && av[u] == (T)1) {
+#pragma unroll
+            for (int j = 0; j < JD; ++j) acc[j] = add_t(acc[j], xv[u][j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < JD; ++j) acc[j] = acc_step(acc[j], av[u], xv[u][j]);
+          }
+        }
+      }
+    }
+  }
+  const T *mu = (const T *)p.means + (i64)k * D;
+  T z[JD];
+#pragma unroll
+  for (int j = 0; j < JD; ++j) {
+    const int d = lane + 32 * j;
+    z[j] = (T)0;
+    if (d < D) {
+      T v = vlad_mass_step<T>(acc[j], mu[d], mass, p.flags);
+      if (p.flags & VL_VLAD_FLAG_SQUARE_ROOT) v = v >= (T)0 ? sqrt_t(v) : -sqrt_t(-v);
+      z[j] = v;
+    }
+  }
+  if (p.flags & VL_VLAD_FLAG_NORMALIZE_COMPONENTS) {
+    // In dimension order: every lane adds the shuffled squares, so that the
+    // chain is the additions alone.
+    T nrm = (T)0;
+#pragma unroll
+    for (int j = 0; j < JD; ++j) {
+      const T sq = mul_t(z[j], z[j]);
+      if (32 * j + 32 <= D) {
+#pragma unroll
+        for (int l = 0; l < 32; ++l) nrm = add_t(nrm, __shfl_sync(0xffffffffu, sq, l));
+      } else {
+        for (int l = 0; l < D - 32 * j; ++l) nrm = add_t(nrm, __shfl_sync(0xffffffffu, sq, l));
+      }
+    }
+    nrm = (T)fmax((double)sqrt_t(nrm), 1e-12);
+#pragma unroll
+    for (int j = 0; j < JD; ++j) z[j] = div_t(z[j], nrm);
+  }
+  T *out = (T *)p.enc + img * (i64)K * D + (i64)k * D;
+#pragma unroll
+  for (int j = 0; j < JD; ++j) {
+    const int d = lane + 32 * j;
+    if (d < D) out[d] = z[j];
+  }
+}
+
+// Images with a multi-weight row are left to the streaming kernel.  W: warps per
+// block (launch_group); MANY: per images a block, else one.
 template <typename T, int JD, int W, bool MANY>
 __global__ void __launch_bounds__(W * 32) k_vlad_group(const VgParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int K = p.K, D = p.D, k = blockIdx.x * W + warp;
-  if (k >= K) return;
-  const T *X = (const T *)p.X, *A = (const T *)p.wgt;
-  const i64 first = p.img0 + (i64)blockIdx.y * (MANY ? p.per : 1);
-  const i64 last = MANY ? min(p.img1, first + p.per) : first + 1;
-  for (i64 img = first; img < last; ++img) {
-    if (p.soft[img]) continue;
-    const i64 r0 = p.offs[img];
-    const int b = p.cstart[img * (K + 1) + k], e = p.cstart[img * (K + 1) + k + 1];
-    const int *rows = p.sorted + r0;
-    T acc[JD];
-#pragma unroll
-    for (int j = 0; j < JD; ++j) acc[j] = (T)0;
-    double mass = 0.0;
-    // 32 of the component's rows at a time: lane j loads the j-th row index and
-    // weight; the rows' descriptors are loaded kVgPrefetch rows ahead.
-    for (int t = b; t < e; t += 32) {
-      const int cnt = min(32, e - t);
-      const int myrow = lane < cnt ? rows[t + lane] : 0;
-      const T mya = lane < cnt ? A[r0 + myrow] : (T)0;
-      for (int u0 = 0; u0 < cnt; u0 += kVgPrefetch) {
-        T av[kVgPrefetch], xv[kVgPrefetch][JD];
-#pragma unroll
-        for (int u = 0; u < kVgPrefetch; ++u) {
-          const int rr = __shfl_sync(0xffffffffu, myrow, (u0 + u) & 31);
-          av[u] = __shfl_sync(0xffffffffu, mya, (u0 + u) & 31);
-          if (u0 + u < cnt) {
-            const i64 row = r0 + rr;
-#pragma unroll
-            for (int j = 0; j < JD; ++j) {
-              const int d = lane + 32 * j;
-              xv[u][j] = d < D ? X[row * D + d] : (T)0;
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kVgPrefetch; ++u) {
-          if (u0 + u < cnt) {
-            mass += (double)av[u];
-            if (sizeof(T) == 4 && av[u] == (T)1) {
-#pragma unroll
-              for (int j = 0; j < JD; ++j) acc[j] = add_t(acc[j], xv[u][j]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < JD; ++j) acc[j] = acc_step(acc[j], av[u], xv[u][j]);
-            }
-          }
-        }
-      }
-    }
-    const T *mu = (const T *)p.means + (i64)k * D;
-    T z[JD];
-#pragma unroll
-    for (int j = 0; j < JD; ++j) {
-      const int d = lane + 32 * j;
-      z[j] = (T)0;
-      if (d < D) {
-        T v = vlad_mass_step<T>(acc[j], mu[d], mass, p.flags);
-        if (p.flags & VL_VLAD_FLAG_SQUARE_ROOT) v = v >= (T)0 ? sqrt_t(v) : -sqrt_t(-v);
-        z[j] = v;
-      }
-    }
-    if (p.flags & VL_VLAD_FLAG_NORMALIZE_COMPONENTS) {
-      // In dimension order: every lane adds the shuffled squares, so that the
-      // chain is the additions alone.
-      T nrm = (T)0;
-#pragma unroll
-      for (int j = 0; j < JD; ++j) {
-        const T sq = mul_t(z[j], z[j]);
-        if (32 * j + 32 <= D) {
-#pragma unroll
-          for (int l = 0; l < 32; ++l) nrm = add_t(nrm, __shfl_sync(0xffffffffu, sq, l));
-        } else {
-          for (int l = 0; l < D - 32 * j; ++l) nrm = add_t(nrm, __shfl_sync(0xffffffffu, sq, l));
-        }
-      }
-      nrm = (T)fmax((double)sqrt_t(nrm), 1e-12);
-#pragma unroll
-      for (int j = 0; j < JD; ++j) z[j] = div_t(z[j], nrm);
-    }
-    T *out = (T *)p.enc + img * (i64)K * D + (i64)k * D;
-#pragma unroll
-    for (int j = 0; j < JD; ++j) {
-      const int d = lane + 32 * j;
-      if (d < D) out[d] = z[j];
-    }
+  const int k = blockIdx.x * W + warp;
+  if constexpr (!MANY) {
+    const i64 img = p.img0 + blockIdx.y;
+    if (p.soft[img] || k >= p.K) return;
+    vlad_group_one<T, JD>(p, img, k, lane);
+  } else {
+    if (k >= p.K) return;
+    const i64 first = p.img0 + (i64)blockIdx.y * p.per, last = min(p.img1, first + p.per);
+    for (i64 img = first; img < last; ++img)
+      if (!p.soft[img]) vlad_group_one<T, JD>(p, img, k, lane);
   }
 }
 
