@@ -834,19 +834,20 @@ void launch_stream(T *enc, const T *means, int D, int K, const T *X, const T *A,
   launch_stream_cpw<T, JD, kVsCpw>(p, nimg, s);
 }
 
-// Images per block: as many, up to eight, as leave four blocks for each that the
-// chip holds, or twenty where components have more than four rows on average and
-// blocks so differ more in length.  A block takes 0.55 ns to start and end even
-// when its image is left to the streaming kernel.  us, one image a block and this
-// rule, float: 3,000 images of 100 rows, K = 64, D = 64, 119 and 117, all of them
-// soft 105 and 19 (eight warps a block: 21); 20,000 of 20 rows 668 and 506, soft 666
-// and 88.  256 images of 4,000 rows, K = 256, D = 80, stay at one (142; with two
-// 181), as do 4,000 of 300 rows, K = 32, D = 48 (140; 142).
+// Images per block.  A block takes 0.55 ns to start and end, also where its image
+// is soft and left to the streaming kernel, so where components have four rows or
+// fewer on average a block takes as many images, up to eight, as leave four
+// blocks for each that the chip holds.  us, one image a block and this rule,
+// float: 3,000 images of 100 rows, K = 64, D = 64, 119 and 117, all of them soft 105 and
+// 19 (eight warps a block: 21); 20,000 of 20 rows 668 and 506, soft 666 and 88; 4,096
+// of 620 rows, K = 256, D = 80, 865 and 754, soft 545 and 74.  With more rows one image
+// a block is faster: 18 rows a component, 4,096 images, K = 256, 1,730, two images
+// 1,826, eight 1,841 (soft 545, 277, 74, beside 15,100 of the streaming kernel).
 template <typename T, int JD, int W>
 void launch_group_as(const VgParams &p0, i64 nimg, cudaStream_t s) {
   VgParams p = p0;
   const i64 blocks = (p.K + W - 1) / W * nimg, chip = 32 * 148;
-  p.per = (int)std::max<i64>(1, std::min<i64>(8, blocks / (p.N <= 4 * p.K * nimg ? 4 * chip : 20 * chip)));
+  p.per = p.N <= 4 * p.K * nimg ? (int)std::max<i64>(1, std::min<i64>(8, blocks / (4 * chip))) : 1;
   const i64 step = (i64)65535 * p.per;
   for (i64 img0 = 0; img0 < nimg; img0 += step) {
     p.img0 = img0;
