@@ -165,7 +165,7 @@ __global__ void k_prepare(const T *__restrict__ priors, const T *__restrict__ me
 // (measured: 123), so R x NJ = 64 accumulators per lane keep the operand loads
 // (NJ / 2 16-byte loads per dimension, R broadcast 8-byte loads per two) at
 // under half of the shared-memory bandwidth.  Model and row chunks are copied
-// asynchronously, three stages ahead; two blocks of 64 rows share an SM, so
+// asynchronously, two chunks ahead in three stages; two blocks of 64 rows share an SM, so
 // that one block's exponentials and divisions run beside the other's sums.
 // A packed instruction holds the issue port for two clocks, so the sum of all
 // instructions' issue clocks bounds the kernel: 3 x 80 of about 117 a row and
